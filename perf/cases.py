@@ -35,7 +35,16 @@ from pylorenzmie_b200.theory import AberratedLorenzMie, LayeredSphere, autograd
 
 WAVELENGTH, MAGNIFICATION, N_M, NOISE = 0.447, 0.048, 1.340, 0.003
 KEYS = ('x_p', 'y_p', 'z_p', 'a_p', 'n_p', 'k_p')
-FITTED = KEYS[:5]
+
+
+def _fitted(case):
+    '''The free parameters: of core-shell particles the material is known.'''
+    return KEYS[:4] if case.get('layers', 1) > 1 else KEYS[:5]
+
+
+def _table(case):
+    return [k for v in _fitted(case) for k in (v, 'd' + v)] + [
+        'success', 'npix', 'redchi']
 
 
 def listed():
@@ -188,7 +197,7 @@ def _scene(case, seed):
             s['frac'] = inner + rng.uniform(-0.05, 0.05, (n, L - 1))
             s['core'] = rng.uniform(1.40, 1.45, (n, L - 1)).astype(complex)
             start[:, 3] *= 1.005
-            start[:, 4] = p[:, 4] + 0.002
+            start[:, 4] = p[:, 4]
             start[:, 2] = p[:, 2] + 1.
         s['p'], s['start'], s['sides'] = p, start, sides
     return s
@@ -298,7 +307,7 @@ def prepare(case, seed):
         else:
             model = LorenzMie(instrument=_instrument())
         opt = Optimizer(model=model)
-        opt.variables = list(FITTED)
+        opt.variables = list(_fitted(case))
         state['optimizer'] = opt
     else:
         start, data, boxes = _frame(case, s, seed, dev)
@@ -319,10 +328,6 @@ def _columns(table, names):
         v = np.asarray(table[name])
         out[name] = v.astype(np.float32) if v.dtype.kind == 'f' else v
     return out
-
-
-_TABLE = [k for v in FITTED for k in (v, 'd' + v)] + ['success', 'npix',
-                                                      'redchi']
 
 
 def run(state):
@@ -346,7 +351,7 @@ def run(state):
             opt.model.particle = _sphere(s['start'][0])
             result = opt.optimize(state['holograms'][0])
             return {k: (np.float32(result[k]) if isinstance(
-                result[k], float) else int(result[k])) for k in _TABLE}
+                result[k], float) else int(result[k])) for k in _table(case)}
         if case['layers'] > 1:
             particles = []
             for row, f, c in zip(s['start'], s['frac'], s['core']):
@@ -357,14 +362,14 @@ def run(state):
             table = opt.optimize_batch(state['holograms'], particles)
         else:
             table = opt.optimize_batch(state['holograms'], starts=s['start'])
-        return _columns(table, _TABLE)
+        return _columns(table, _table(case))
     frame = state['frame']
     np.random.seed(state['seed'] % (1 << 31))   # the random pixel subsets
     if kind == 'frame_fit':
         for f, row in zip(frame.features, state['start']):
             f.particle.r_p = row[:3]
             f.particle.a_p, f.particle.n_p = row[3], row[4]
-        return _columns(frame.optimize(), _TABLE)
+        return _columns(frame.optimize(), _table(case))
     frame.estimate()
     return np.array([[f.particle.z_p, f.particle.a_p, f.particle.n_p]
                      for f in frame.features])
@@ -555,10 +560,10 @@ class _Model:
         return torch.stack(out)
 
 
-def _exact_fit(m, data, start):
+def _exact_fit(m, data, start, fitted):
     '''The least-squares minimum from ``start`` and its statistics.'''
     p = start.copy()
-    n, nv = p.shape[0], len(FITTED)
+    n, nv = p.shape[0], len(fitted)
     own = m.owner
     npix = torch.bincount(own, minlength=n).double()
 
@@ -578,7 +583,7 @@ def _exact_fit(m, data, start):
     err = (redchi[:, None] * torch.linalg.inv(A).diagonal(
         dim1=-2, dim2=-1)).sqrt()
     out = {}
-    for j, v in enumerate(FITTED):
+    for j, v in enumerate(fitted):
         out[v], out['d' + v] = p[:, j].copy(), err[:, j].cpu().numpy()
     out['success'] = out['npix'] = None
     out['redchi'] = redchi.cpu().numpy()
@@ -616,7 +621,7 @@ def exact(case, seed):
         return {'hologram': h, 'grad': grad}
     if kind == 'fit' and case['features'] * case['hi'] ** 2 <= 3_000_000:
         m, data = _crops(case, s, seed, dev)
-        out = _exact_fit(m, data, s['start'])
+        out = _exact_fit(m, data, s['start'], _fitted(case))
         if case['features'] == 1 and case['layers'] == 1:
             out = {k: None if v is None else float(v[0])
                    for k, v in out.items()}
