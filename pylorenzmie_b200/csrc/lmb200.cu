@@ -12,59 +12,15 @@
 
 #include "lmb200.h"
 #include "lmb_kernels.cuh"
+#include "lmb_launch.cuh"
 
 using namespace lmb;
 
 namespace {
 
-#define LMB_CK(x)                                    \
-  do {                                               \
-    cudaError_t e_ = (x);                            \
-    if (e_ != cudaSuccess) return LMB_ERR_CUDA;      \
-  } while (0)
-
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
-
-// Opt a kernel in to more than 48 KB of dynamic shared memory when needed.
-// Per-call host work kept off the path between fits: the shared-memory
-// attribute of a kernel is raised once per device to the largest size asked
-// for, and persistent grid sizes are looked up once per (device, kernel,
-// block, shared memory).
-std::mutex g_launch_cache_lock;
-struct AttrEntry {
-  int device;
-  const void* fn;
-  size_t value;
-  int tpb;
-  size_t smem;
-};
-std::vector<AttrEntry> g_smem_set;    // value: bytes set
-std::vector<AttrEntry> g_grid_sizes;  // value: grid
-
-inline int current_device() {
-  int dev = -1;
-  return cudaGetDevice(&dev) == cudaSuccess ? dev : -1;
-}
-
-inline cudaError_t smem_attr(const void* fn, size_t bytes) {
-  if (bytes <= 48 * 1024) return cudaSuccess;
-  const int dev = current_device();
-  std::lock_guard<std::mutex> hold(g_launch_cache_lock);
-  for (const AttrEntry& e : g_smem_set)
-    if (e.device == dev && e.fn == fn && e.value >= bytes) return cudaSuccess;
-  const cudaError_t r = cudaFuncSetAttribute(
-      fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
-  if (r != cudaSuccess || dev < 0) return r;
-  for (AttrEntry& e : g_smem_set)
-    if (e.device == dev && e.fn == fn) {
-      e.value = bytes;
-      return r;
-    }
-  g_smem_set.push_back({dev, fn, bytes, 0, 0});
-  return r;
-}
 
 inline bool bad_cap(int nmax_cap) { return nmax_cap < 1 || nmax_cap > LMB_NMAX_LIMIT; }
 
