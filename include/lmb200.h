@@ -135,6 +135,62 @@ int lmb_hologram_aberrated(const double *coords, long long npts,
                            double aberration, void *out, void *stream);
 
 /*
+ * Fields and holograms on a unit-step pixel grid in one plane, from radial
+ * tables: in a plane the sums over the orders depend on the distance from a
+ * sphere's axis alone, so they are formed in FP64 at equidistant distances
+ * and interpolated at the pixels (FP32 outputs, within the FP32 rounding of
+ * the direct sums; holograms within 2e-5 of FP64 as lmb_hologram).  Pixel
+ * (column, row) lies at (x0 + column, y0 + row, z), row-major outputs.
+ *
+ * With ``points`` (device, [3][npts], all in the plane z) the pixels are
+ * those instead, and the grid is a box around them.
+ *
+ * lmb_grid_probe       of a coordinate list [3][npts], 7 values out
+ *                      (device): the row length; the pixels that are not on
+ *                      the grid of that row length (a grid if 0 and the row
+ *                      length divides npts); the pixels that are not finite
+ *                      or not in the first one's plane; then, as doubles,
+ *                      the bounds min x, min y, max x, max y.
+ * lmb_radial_intervals host only: the table intervals a particle that
+ *                      these n spheres (host records, a_p the outer radius)
+ *                      need for npts pixels, or 0 where the tables do not
+ *                      apply and the coordinate entry points are to be used:
+ *                      a plane closer than k d = 1.8 to a sphere or cutting
+ *                      it, distances above 8000 px, spherical components,
+ *                      FP64, an aberration phase steeper than a fifth of k,
+ *                      or too few pixels to pay for the tables.
+ * lmb_field_grid / lmb_hologram_grid: as lmb_field_aberrated /
+ *                      lmb_hologram_aberrated (aberration 0: ideal optics);
+ *                      nparticles = item_start[nitems], intervals from
+ *                      lmb_radial_intervals, workspace of
+ *                      lmb_radial_workspace_bytes(nparticles, intervals).
+ */
+typedef struct lmb_grid {
+  double x0, y0, z;
+  long long nx, ny;
+} lmb_grid;
+int lmb_grid_probe(const double *coords, long long npts,
+                   unsigned long long *out, void *stream);
+int lmb_radial_intervals(const lmb_grid *grid, long long npts,
+                         const lmb_sphere *spheres, int n, double k, double magnification, int flags,
+                         double aberration);
+size_t lmb_radial_workspace_bytes(int nparticles, int intervals);
+int lmb_field_grid(const lmb_grid *grid, const double *points,
+                   long long npts, const lmb_sphere *spheres,
+                   const int *item_start, int nitems, int nparticles,
+                   int intervals, const double *ab, const int *nmax,
+                   int nmax_cap, double k, int flags, double aberration,
+                   void *out, void *workspace, size_t workspace_bytes,
+                   void *stream);
+int lmb_hologram_grid(const lmb_grid *grid, const double *points,
+                      long long npts, const lmb_sphere *spheres,
+                      const int *item_start, int nitems, int nparticles,
+                      int intervals, const double *ab, const int *nmax,
+                      int nmax_cap, double k, int flags, double aberration,
+                      void *out, void *workspace, size_t workspace_bytes,
+                      void *stream);
+
+/*
  * chi^2 = sum over pixels of ((hologram - data) / noise)^2 for each of
  * nitems particle lists at shared coordinates: the objective of one
  * differential-evolution generation in one launch.  Replaces the

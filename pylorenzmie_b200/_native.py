@@ -54,6 +54,12 @@ class FitStats(ctypes.Structure):
                 ('iterations', ctypes.c_int), ('pad', ctypes.c_int)]
 
 
+class Grid(ctypes.Structure):
+    _fields_ = [('x0', ctypes.c_double), ('y0', ctypes.c_double),
+                ('z', ctypes.c_double), ('nx', ctypes.c_longlong),
+                ('ny', ctypes.c_longlong)]
+
+
 class LMBError(RuntimeError):
     '''A non-zero status from the CUDA library.'''
 
@@ -82,6 +88,16 @@ _SIGNATURES = {
                                  _i, _d, _vp, _vp]),
     'lmb_hologram_aberrated': (_i, [_vp, _ll, _vp, _vp, _i, _vp, _vp, _i,
                                     _d, _i, _d, _vp, _vp]),
+    'lmb_grid_probe': (_i, [_vp, _ll, _vp, _vp]),
+    'lmb_radial_intervals': (_i, [ctypes.POINTER(Grid), _ll, _vp, _i, _d, _d,
+                                  _i, _d]),
+    'lmb_radial_workspace_bytes': (_sz, [_i, _i]),
+    'lmb_field_grid': (_i, [ctypes.POINTER(Grid), _vp, _ll, _vp, _vp, _i, _i,
+                            _i, _vp, _vp, _i, _d, _i, _d, _vp, _vp, _sz,
+                            _vp]),
+    'lmb_hologram_grid': (_i, [ctypes.POINTER(Grid), _vp, _ll, _vp, _vp, _i,
+                               _i, _i, _vp, _vp, _i, _d, _i, _d, _vp, _vp,
+                               _sz, _vp]),
     'lmb_jacobian': (_i, [_vp, _ll, _vp, _i, _vp, _vp, _vp, _i, _d, _i, _vp,
                           _vp, _vp]),
     'lmb_de_trial': (_i, [_i, _i, _vp, _i, _i, _vp, _vp, _vp, _i, _d, _d,

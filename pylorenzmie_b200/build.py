@@ -20,7 +20,7 @@ CSRC = PKG / 'csrc'
 INCLUDE = ROOT / 'include'
 LIBDIR = PKG / '_lib'
 LIBRARY = LIBDIR / 'liblmb200.so'
-SOURCES = ['lmb200.cu', 'lmb_host.cpp']
+SOURCES = ['lmb200.cu', 'lmb_radial.cu', 'lmb_host.cpp']
 GENCODE = ['-gencode', 'arch=compute_100a,code=sm_100a']
 
 
@@ -48,6 +48,7 @@ def up_to_date():
 
 def command(output=LIBRARY, extra=()):
     return [nvcc_path(), *GENCODE, '-lineinfo', '-O3', '-std=c++17',
+            '--threads', '0',
             '-shared', '-Xcompiler', '-fPIC', '-Xcompiler', '-O3',
             f'-I{INCLUDE}', f'-I{CSRC}', *extra,
             *[str(CSRC / s) for s in SOURCES], '-o', str(output)]

@@ -1,0 +1,683 @@
+// Fields and holograms on a pixel grid from radial tables (lmb_radial.cuh):
+// lmb_grid_probe, lmb_radial_intervals, lmb_radial_workspace_bytes,
+// lmb_field_grid, lmb_hologram_grid.  Declarations: include/lmb200.h.
+#include <cuda_pipeline.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <math.h>
+
+#include "lmb200.h"
+#include "lmb_launch.cuh"
+#include "lmb_radial.cuh"
+
+using namespace lmb;
+
+namespace {
+
+// ---------------------------------------------------------------------------
+// Is a coordinate list a unit-step pixel grid, or at least in one plane?
+
+enum { PROBE_ROW, PROBE_OFF_GRID, PROBE_OFF_PLANE, PROBE_LO_X, PROBE_LO_Y, PROBE_HI_X,
+       PROBE_HI_Y };
+
+// Doubles as unsigned integers in the same order, and back.
+__device__ inline unsigned long long ordered(double v) {
+  const unsigned long long u = (unsigned long long)__double_as_longlong(v);
+  return u ^ ((u >> 63) ? ~0ull : 1ull << 63);
+}
+__device__ inline double unordered(unsigned long long u) {
+  return __longlong_as_double((long long)(u ^ ((u >> 63) ? 1ull << 63 : ~0ull)));
+}
+
+__global__ void k_probe_init(long long npts, unsigned long long* out) {
+  out[PROBE_ROW] = (unsigned long long)npts;
+  out[PROBE_OFF_GRID] = out[PROBE_OFF_PLANE] = 0ull;
+  out[PROBE_LO_X] = out[PROBE_LO_Y] = ~0ull;
+  out[PROBE_HI_X] = out[PROBE_HI_Y] = 0ull;
+}
+
+// The first index whose y differs from the first pixel's (npts if none),
+// i.e. the row length of a grid.
+__global__ void k_probe_row(const double* __restrict__ coords, long long npts,
+                            unsigned long long* out) {
+  const double y0 = coords[npts];
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < npts;
+       i += (long long)gridDim.x * blockDim.x)
+    if (coords[npts + i] != y0) {
+      atomicMin(out + PROBE_ROW, (unsigned long long)i);
+      break;
+    }
+}
+
+// How many pixels are not (x0 + column, y0 + row, z0), how many are not
+// finite or not in the plane z0, and the bounds of x and y.
+__global__ void k_probe_check(const double* __restrict__ coords, long long npts,
+                              unsigned long long* out) {
+  const long long nx = (long long)out[PROBE_ROW];
+  const double x0 = coords[0], y0 = coords[npts], z0 = coords[2 * npts];
+  unsigned long long off = 0, plane = 0, b[4] = {~0ull, ~0ull, 0ull, 0ull};
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < npts;
+       i += (long long)gridDim.x * blockDim.x) {
+    const double x = coords[i], y = coords[npts + i], z = coords[2 * npts + i];
+    const long long row = i / nx;
+    if (!(x == x0 + double(i - row * nx)) || !(y == y0 + double(row)) || !(z == z0)) ++off;
+    if (!isfinite(x) || !isfinite(y) || !isfinite(z) || z != z0) ++plane;
+    b[0] = min(b[0], ordered(x));
+    b[1] = min(b[1], ordered(y));
+    b[2] = max(b[2], ordered(x));
+    b[3] = max(b[3], ordered(y));
+  }
+  for (int o = 16; o > 0; o >>= 1)
+    for (int j = 0; j < 4; ++j) {
+      const unsigned long long v = __shfl_xor_sync(0xffffffffu, b[j], o);
+      b[j] = j < 2 ? min(b[j], v) : max(b[j], v);
+    }
+  if (off) atomicAdd(out + PROBE_OFF_GRID, off);
+  if (plane) atomicAdd(out + PROBE_OFF_PLANE, plane);
+  if ((threadIdx.x & 31) == 0)
+    for (int j = 0; j < 4; ++j)
+      if (j < 2) atomicMin(out + PROBE_LO_X + j, b[j]);
+      else atomicMax(out + PROBE_LO_X + j, b[j]);
+}
+
+__global__ void k_probe_bounds(unsigned long long* out) {
+  for (int j = PROBE_LO_X; j <= PROBE_HI_Y; ++j)
+    out[j] = (unsigned long long)__double_as_longlong(unordered(out[j]));
+}
+
+// ---------------------------------------------------------------------------
+// The plan of one call, from lmb_radial_intervals' rule.
+
+struct RadialPlan {
+  double x0, y0, z;     // first pixel, plane
+  long long nx, ny;
+  double k, aberr;
+  double spacing;       // node spacing = interval width (px), a multiple of 1/64
+  float inv_half;       // 2 / spacing (1/px)
+  int intervals;        // capacity per particle
+  int flags;
+};
+
+// Interval width in pixels, a multiple of 1/64 so that i * width is exact
+// in FP32; 0 if k is out of range.
+inline double radial_spacing(double k) {
+  const double w = std::min(floor(64. * RADIAL_SPACING / k) / 64., 64.);
+  return w >= 0.0625 ? w : 0.;
+}
+
+// Largest distance of a particle from the grid's pixels.
+__host__ __device__ inline double radial_reach(double x0, double y0, long long nx,
+                                               long long ny, double xp, double yp) {
+  const double dx = fmax(fabs(x0 - xp), fabs(x0 + double(nx - 1) - xp));
+  const double dy = fmax(fabs(y0 - yp), fabs(y0 + double(ny - 1) - yp));
+  return sqrt(fma(dx, dx, dy * dy));  // the same value wherever it is compiled
+}
+
+// Intervals a particle uses: indices 0 .. count - 1 cover its pixels.
+__host__ __device__ inline int radial_count(double reach, double spacing) {
+  return int(reach / spacing) + 2;
+}
+
+// ---------------------------------------------------------------------------
+// Nodes and polynomials: one block per (chunk of intervals, particle).
+//
+// One thread sums the orders of one node in FP64 (serial recurrences, bound
+// by FP64 issue: ~40 FP64 instructions an order), so a block of 128 threads
+// covers 112 intervals and the 8 nodes that their polynomials reach on
+// either side.  Then every thread forms the polynomials of (interval,
+// function) pairs, 2 x 6 x 17 FP64 FMAs each with the matrix in the constant
+// bank.  The FP64 nodes are kept for the pixels that k_field_radial sums
+// again in FP64.
+constexpr int kNodeThreads = 128;
+constexpr int kChunk = kNodeThreads - 2 * RADIAL_SIDE;
+
+__global__ void __launch_bounds__(kNodeThreads)
+k_radial_table(RadialPlan pl, RadialMatrix A, const lmb_sphere* __restrict__ spheres,
+               const zd* __restrict__ ab, const int* __restrict__ nmax, int nmaxp,
+               float* __restrict__ table, double* __restrict__ nodes) {
+  extern __shared__ __align__(16) char smem[];
+  double* val = reinterpret_cast<double*>(smem);  // [RADIAL_FUNCS][kNodeThreads]
+  Quad<double>* rec = reinterpret_cast<Quad<double>*>(
+      smem + sizeof(double) * RADIAL_FUNCS * kNodeThreads);
+  const int p = blockIdx.y, i0 = blockIdx.x * kChunk;
+  const lmb_sphere sp = spheres[p];
+  const int count = min(pl.intervals,
+                        radial_count(radial_reach(pl.x0, pl.y0, pl.nx, pl.ny,
+                                                  sp.x_p, sp.y_p), pl.spacing));
+  if (i0 >= count) return;  // the whole block
+  const int nm = min(max(nmax[p], 0), nmaxp - 1);
+  for (int n = threadIdx.x; n <= nm; n += kNodeThreads) {
+    Quad<double> q[2];
+    order_record<double>(ab + (size_t(p) * nmaxp + n) * 2, (const zd*)0, n, 2, q);
+    rec[2 * n] = q[0];
+    rec[2 * n + 1] = q[1];
+  }
+  __syncthreads();
+  const int j = i0 - RADIAL_SIDE + int(threadIdx.x);  // node of this thread
+  const int ncap = pl.intervals + 2 * RADIAL_SIDE;
+  if (j < count + RADIAL_SIDE) {
+    double v[RADIAL_FUNCS];
+    radial_field(pl.k, j ? pl.spacing * double(abs(j)) : RADIAL_AXIS, pl.z - sp.z_p, pl.z,
+                 sp.z_p, pl.flags & LMB_BOHREN, pl.aberr, rec, nm, v);
+    const int t = threadIdx.x;
+    for (int f = 0; f < RADIAL_FUNCS; ++f) val[f * kNodeThreads + t] = v[f];
+    // each node is written by the chunk it lies in (the ends by the outer ones)
+    if ((t >= RADIAL_SIDE || i0 == 0) &&
+        (t < kNodeThreads - RADIAL_SIDE || i0 + kChunk >= count)) {
+      double* out = nodes + (size_t(p) * ncap + (j + RADIAL_SIDE)) * RADIAL_FUNCS;
+      for (int f = 0; f < RADIAL_FUNCS; ++f) out[f] = v[f];
+    }
+  }
+  __syncthreads();
+  const int n = min(kChunk, count - i0);
+  for (int w = threadIdx.x; w < n * (RADIAL_FUNCS / 2); w += kNodeThreads) {
+    const int f = w / n, i = w - f * n;
+    const double* s = val + 2 * f * kNodeThreads + i;
+    double cr[RADIAL_COEFS], ci[RADIAL_COEFS];
+#pragma unroll
+    for (int q = 0; q < RADIAL_COEFS; ++q) cr[q] = ci[q] = 0.;
+#pragma unroll
+    for (int l = 0; l < RADIAL_TAPS; ++l) {
+      const double x = s[l], y = s[kNodeThreads + l];
+#pragma unroll
+      for (int q = 0; q < RADIAL_COEFS; ++q) {
+        cr[q] = fma(A.m[q][l], x, cr[q]);
+        ci[q] = fma(A.m[q][l], y, ci[q]);
+      }
+    }
+    // re and im of a coefficient side by side
+    float4* out = reinterpret_cast<float4*>(
+        table + (size_t(p) * pl.intervals + i0 + i) * RADIAL_REC + f * 2 * RADIAL_COEFS);
+#pragma unroll
+    for (int q = 0; q < RADIAL_COEFS; q += 2)
+      out[q / 2] = make_float4(float(cr[q]), float(ci[q]), float(cr[q + 1]), float(ci[q + 1]));
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Pixels.
+
+// FP64 values of the marked pixels of a tile, interpolated straight from
+// the FP64 nodes (17 points, error ~1e-12): for the pixels whose FP32 value
+// may be off by more than HOLO_TOL, a few per thousand.  A tile's marked
+// pixels sit together, so the particles of a pixel are spread over lanes: a
+// group of lanes (the next power of two from the particle count, up to the
+// warp) per pixel, combined by a fixed shuffle tree.  where(entry, x, y)
+// gives a list entry's position and returns its index in out.
+template <typename Where>
+__device__ void radial_resum64(const RadialPlan& pl, const int* list, int F, Where where,
+                               const lmb_sphere* __restrict__ spheres, int pb, int pe,
+                               const double* __restrict__ nodes, float* out) {
+  const int ncap = pl.intervals + 2 * RADIAL_SIDE;
+  const int lane = threadIdx.x & 31;
+  int group = 1;
+  while (group < 32 && group < pe - pb) group <<= 1;
+  const int per = 32 / group, sub = lane & (group - 1);
+  const int step = int(blockDim.x >> 5) * per;
+  // the same trip count for every lane of a warp
+  for (int f0 = int(threadIdx.x >> 5) * per; f0 < F; f0 += step) {
+    const int f = f0 + lane / group;
+    const bool live = f < F;
+    double x, y;
+    const long long pix = where(list[live ? f : F - 1], &x, &y);
+    double e[6] = {0., 0., 0., 0., 0., 0.};
+    for (int p = pb + sub; live && p < pe; p += group) {
+      const double dx = x - spheres[p].x_p, dy = y - spheres[p].y_p;
+      const double rho = sqrt(dx * dx + dy * dy);
+      const double u = rho / pl.spacing;
+      const int j = min(int(u + 0.5), pl.intervals - 1);
+      double w[RADIAL_TAPS], v[RADIAL_FUNCS];
+      radial_weights(u - double(j), w);
+      for (int c = 0; c < RADIAL_FUNCS; ++c) v[c] = 0.;
+      const double2* s =
+          reinterpret_cast<const double2*>(nodes + (size_t(p) * ncap + j) * RADIAL_FUNCS);
+#pragma unroll
+      for (int l = 0; l < RADIAL_TAPS; ++l)
+        for (int c = 0; c < RADIAL_FUNCS / 2; ++c) {
+          const double2 n = s[l * (RADIAL_FUNCS / 2) + c];
+          v[2 * c] = fma(w[l], n.x, v[2 * c]);
+          v[2 * c + 1] = fma(w[l], n.y, v[2 * c + 1]);
+        }
+      const double c2 = dx * dx - dy * dy, s2 = 2. * dx * dy;
+      for (int c = 0; c < 2; ++c) {
+        e[c] += v[c] + c2 * v[2 + c];
+        e[2 + c] += s2 * v[2 + c];
+        e[4 + c] += dx * v[4 + c];
+      }
+    }
+    for (int o = group >> 1; o > 0; o >>= 1)
+      for (int c = 0; c < 6; ++c) e[c] += __shfl_xor_sync(0xffffffffu, e[c], o);
+    const zd t[3] = {mk(e[0], e[1]), mk(e[2], e[3]), mk(e[4], e[5])};
+    if (live && sub == 0) out[pix] = float(intensity<double>(t));
+  }
+}
+
+// The bound on an FP32 pixel's error from the tables: the field of a
+// particle is off by at most RADIAL_FIELD_REL |E_p| (coefficients and
+// Horner's rule in FP32), with |E_p| <= 1.8 max(|Re U|, |Im U|) wherever it
+// is large; |H - H64| <= 2 sqrt(H) sum_p of that.
+#define RADIAL_FIELD_REL 4e-7f
+
+__device__ inline bool radial_needs_fp64(float h, float m1) {
+  return 2.f * sqrtf(fmaxf(h, 0.f)) * (1.8f * RADIAL_FIELD_REL) * m1 > HOLO_TOL;
+}
+
+struct TileParticle {
+  float ax, rx, ay, ry;  // first pixel minus particle: 2^-10 px part, rest
+  int lo, count;         // intervals that the tile's pixels use
+};
+
+constexpr int kTile = 32;          // tiles of 32 x 32 pixels
+constexpr int kPixThreads = 256;   // a 2x2 group each
+constexpr int kTileGroup = 32;     // particles whose TileParticle is staged at once
+
+// One complex function (re, im) at t: degree RADIAL_COEFS - 1.
+__device__ inline f2 radial_eval(const float4* r, float t) {
+  const float4 a = r[0], b = r[1], c = r[2];
+  const f2 tt = pk(t, t);
+  f2 v = pfma(pk(c.z, c.w), tt, pk(c.x, c.y));
+  v = pfma(v, tt, pk(b.z, b.w));
+  v = pfma(v, tt, pk(b.x, b.y));
+  v = pfma(v, tt, pk(a.z, a.w));
+  return pfma(v, tt, pk(a.x, a.y));
+}
+
+// One block per 32x32-pixel tile and item, 4 pixels per thread.  For each
+// particle the intervals that the tile needs (its distances span at most
+// 43.9 px, ~70 intervals of 144 bytes) are copied to shared memory, kStages
+// - 1 copies ahead, and every pixel reads its interval's coefficients (9
+// LDS.128) and evaluates the three complex polynomials with (re, im) in the
+// two lanes of packed FP32, so that the coefficients come paired from memory
+// and only t is duplicated.  A pixel's value depends on its position alone,
+// not on its neighbours (groups of pixels that share an interval would read
+// less, but differ from the same pixel in a list by their rounding).
+constexpr int kStages = 3;
+constexpr int kStepX = 8, kStepY = 4;
+template <bool kHolo>
+__global__ void __launch_bounds__(kPixThreads, 2)
+k_field_radial(RadialPlan pl, const lmb_sphere* __restrict__ spheres,
+               const int* __restrict__ item_start, const float* __restrict__ table,
+               const double* __restrict__ nodes, int buffer, void* out) {
+  extern __shared__ __align__(16) float4 buf[];  // [kStages][buffer]
+  __shared__ TileParticle s_tp[kTileGroup];
+  __shared__ int s_marked;
+  const int item = blockIdx.z;
+  const int pb = item_start[item], pe = item_start[item + 1];
+  const long long tx = (long long)blockIdx.x * kTile, ty = (long long)blockIdx.y * kTile;
+  // A warp takes 16x8 pixels as four patches of 8x4, a pixel of each per
+  // lane: columns cx and cx + kStepX, rows cy and cy + kStepY.  The eight
+  // lanes of a quarter warp, whose LDS.128 go together, sit on 4x2 pixels,
+  // whose distances span less than eight intervals: no bank conflicts.
+  const int lane_id = threadIdx.x & 31, warp_id = threadIdx.x >> 5;
+  const int cx = 16 * (warp_id & 1) + 4 * ((lane_id >> 3) & 1) + (lane_id & 3);
+  const int cy = 8 * (warp_id >> 1) + 2 * (lane_id >> 4) + ((lane_id >> 2) & 1);
+  const float inv_spacing = float(1. / pl.spacing), spacing = float(pl.spacing);
+  constexpr int RQ = RADIAL_REC / 4;  // float4 per interval
+  // field sums (re, im) and error bounds of the pixels (2 row + column)
+  f2 ex[4], ey[4], ez[4];
+  float m1[4];
+  for (int q = 0; q < 4; ++q) {
+    ex[q] = ey[q] = ez[q] = pk(0.f, 0.f);
+    m1[q] = 0.f;
+  }
+  for (int g0 = pb; g0 < pe; g0 += kTileGroup) {
+    const int G = min(kTileGroup, pe - g0);
+    __syncthreads();  // the previous group's data is no longer read
+    if (threadIdx.x < G) {
+      const lmb_sphere sp = spheres[g0 + threadIdx.x];
+      const double dx = pl.x0 + double(tx) - sp.x_p, dy = pl.y0 + double(ty) - sp.y_p;
+      TileParticle t;
+      const double ax = rint(dx * 1024.) * (1. / 1024.), ay = rint(dy * 1024.) * (1. / 1024.);
+      t.ax = float(ax);
+      t.rx = float(dx - ax);
+      t.ay = float(ay);
+      t.ry = float(dy - ay);
+      // nearest and farthest distances of the tile's pixels
+      const double e = double(kTile - 1);
+      const double nx = dx > 0. ? dx : (dx + e < 0. ? -(dx + e) : 0.);
+      const double ny = dy > 0. ? dy : (dy + e < 0. ? -(dy + e) : 0.);
+      const double fx = fmax(fabs(dx), fabs(dx + e)), fy = fmax(fabs(dy), fabs(dy + e));
+      const int all = min(pl.intervals,
+                          radial_count(radial_reach(pl.x0, pl.y0, pl.nx, pl.ny, sp.x_p,
+                                                    sp.y_p), pl.spacing));
+      t.lo = max(0, min(all - 1, int(sqrt(nx * nx + ny * ny) / pl.spacing) - 1));
+      const int hi = min(all, int(sqrt(fx * fx + fy * fy) / pl.spacing) + 3);
+      t.count = max(1, min(hi - t.lo, buffer / RQ));
+      s_tp[threadIdx.x] = t;
+    }
+    __syncthreads();
+    // a commit per particle, empty past the last, so that the wait below
+    // always leaves the kStages - 2 newest copies in flight
+    auto fetch = [&](int g) {
+      if (g < G) {
+        const TileParticle t = s_tp[g];
+        const float4* src = reinterpret_cast<const float4*>(table) +
+                            (size_t(g0 + g) * pl.intervals + t.lo) * RQ;
+        float4* dst = buf + (g % kStages) * buffer;
+        for (int i = threadIdx.x; i < t.count * RQ; i += kPixThreads)
+          __pipeline_memcpy_async(dst + i, src + i, 16);
+      }
+      __pipeline_commit();
+    };
+    for (int g = 0; g < kStages - 1; ++g) fetch(g);
+    for (int g = 0; g < G; ++g) {
+      __pipeline_wait_prior(kStages - 2);
+      // copy g has landed, and everyone is done with the buffer that the
+      // next fetch refills (that of particle g - 1)
+      __syncthreads();
+      fetch(g + kStages - 1);
+      const TileParticle t = s_tp[g];
+      const float4* rec = buf + (g % kStages) * buffer;
+      // column and row terms
+      const f2 X = padd(pk(t.ax, t.ax), pk(float(cx), float(cx + kStepX)));
+      const f2 px = pmul(X, X);
+      const f2 lx = pfma(pk(2.f * t.rx, 2.f * t.rx), padd(X, pk(0.5f * t.rx, 0.5f * t.rx)),
+                         pfma(X, X, pneg(px)));
+      const f2 Xr = padd(X, pk(t.rx, t.rx)), X2 = padd(Xr, Xr);
+      const f2 Y = padd(pk(t.ay, t.ay), pk(float(cy), float(cy + kStepY)));
+      const f2 qy = pmul(Y, Y);
+      const f2 ly = pfma(pk(2.f * t.ry, 2.f * t.ry), padd(Y, pk(0.5f * t.ry, 0.5f * t.ry)),
+                         pfma(Y, Y, pneg(qy)));
+      const f2 Yr = padd(Y, pk(t.ry, t.ry));
+      RadialDistance d[2];
+      d[0] = radial_distance(px, lx, pk(qy.x, qy.x), pk(ly.x, ly.x));
+      d[1] = radial_distance(px, lx, pk(qy.y, qy.y), pk(ly.y, ly.y));
+      auto lane = [](f2 v, int q) { return (q & 1) ? v.y : v.x; };
+      f2 c2[2], s2[2];
+      float tq[4];
+      const float4* r4[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float r0 = lane(d[q >> 1].r0, q);
+        const int i = min(max(__float2int_rn(r0 * inv_spacing) - t.lo, 0), t.count - 1);
+        tq[q] = ((r0 - float(i + t.lo) * spacing) + lane(d[q >> 1].corr, q)) * pl.inv_half;
+        r4[q] = rec + i * RQ;
+      }
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const f2 yr = r ? pk(Yr.y, Yr.y) : pk(Yr.x, Yr.x);
+        c2[r] = pmul(psub(Xr, yr), padd(Xr, yr));
+        s2[r] = pmul(X2, yr);
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const f2 u = radial_eval(r4[q], tq[q]);
+        const f2 v = radial_eval(r4[q] + RQ / 3, tq[q]);
+        const f2 w = radial_eval(r4[q] + 2 * (RQ / 3), tq[q]);
+        const float c = lane(c2[q >> 1], q), s = lane(s2[q >> 1], q), x = lane(Xr, q);
+        ex[q] = pfma(pk(c, c), v, padd(ex[q], u));
+        ey[q] = pfma(pk(s, s), v, ey[q]);
+        ez[q] = pfma(pk(x, x), w, ez[q]);
+        if (kHolo) m1[q] += fmaxf(fabsf(u.x), fabsf(u.y));
+      }
+    }
+  }
+  int mark = 0;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const long long col = tx + cx + (q & 1) * kStepX;
+    const long long row = ty + cy + (q >> 1) * kStepY;
+    if (col >= pl.nx || row >= pl.ny) continue;
+    const long long pix = row * pl.nx + col;
+    cplx<float> e[3] = {mk(ex[q].x, ex[q].y), mk(ey[q].x, ey[q].y), mk(ez[q].x, ez[q].y)};
+    const long long npts = pl.nx * pl.ny;
+    if (kHolo) {
+      const float h = intensity<float>(e);
+      float* o = reinterpret_cast<float*>(out) + size_t(item) * npts;
+      if (radial_needs_fp64(h, m1[q]))
+        mark |= 1 << q;
+      else
+        o[pix] = h;
+    } else {
+      float2* o = reinterpret_cast<float2*>(out) + size_t(item) * 3 * npts;
+      for (int c = 0; c < 3; ++c) o[c * npts + pix] = make_float2(e[c].re, e[c].im);
+    }
+  }
+  if (kHolo) {
+    if (threadIdx.x == 0) s_marked = 0;
+    // also the barrier after which the table buffers may be overwritten
+    if (!__syncthreads_or(mark)) return;
+    int* list = reinterpret_cast<int*>(buf);  // up to kTile * kTile entries
+    for (int q = 0; q < 4; ++q)
+      if (mark >> q & 1)
+        list[atomicAdd(&s_marked, 1)] =
+            (cy + (q >> 1) * kStepY) * kTile + cx + (q & 1) * kStepX;
+    __syncthreads();
+    auto where = [&](int l, double* x, double* y) {
+      const long long col = tx + l % kTile, row = ty + l / kTile;
+      *x = pl.x0 + double(col);
+      *y = pl.y0 + double(row);
+      return row * pl.nx + col;
+    };
+    radial_resum64(pl, list, s_marked, where, spheres, pb, pe, nodes,
+                   reinterpret_cast<float*>(out) + size_t(item) * pl.nx * pl.ny);
+  }
+}
+
+// The same from an explicit pixel list in the plane (points [3][npts]; the
+// plan's grid is its bounding box): one thread per pixel, the coefficients
+// of its own intervals read through the caches.  The values are the grid
+// kernel's to the rounding of the polynomials.
+constexpr int kListThreads = 128;
+template <bool kHolo>
+__global__ void __launch_bounds__(kListThreads)
+k_points_radial(RadialPlan pl, const double* __restrict__ points, long long npts,
+                const lmb_sphere* __restrict__ spheres, const int* __restrict__ item_start,
+                const float* __restrict__ table, const double* __restrict__ nodes, void* out) {
+  __shared__ int s_list[kListThreads], s_marked;
+  const int item = blockIdx.y;
+  const int pb = item_start[item], pe = item_start[item + 1];
+  const long long base = (long long)blockIdx.x * kListThreads, pix = base + threadIdx.x;
+  bool mark = false;
+  if (pix < npts) {
+    const double x = points[pix], y = points[npts + pix];
+    const float inv_spacing = float(1. / pl.spacing), spacing = float(pl.spacing);
+    constexpr int RQ = RADIAL_REC / 4;
+    f2 ex = pk(0.f, 0.f), ey = ex, ez = ex;
+    float m1 = 0.f;
+    for (int p = pb; p < pe; ++p) {
+      // the grid kernel's arithmetic, x and y in the two lanes
+      const double dx = x - spheres[p].x_p, dy = y - spheres[p].y_p;
+      const double ax = rint(dx * 1024.) * (1. / 1024.), ay = rint(dy * 1024.) * (1. / 1024.);
+      const f2 X = pk(float(ax), float(ay)), rx = pk(float(dx - ax), float(dy - ay));
+      const f2 px = pmul(X, X);
+      const f2 lx = pfma(padd(rx, rx), pfma(pk(0.5f, 0.5f), rx, X), pfma(X, X, pneg(px)));
+      const f2 Xr = padd(X, rx);
+      const RadialDistance d = radial_distance(pk(px.x, px.x), pk(lx.x, lx.x),
+                                               pk(px.y, px.y), pk(lx.y, lx.y));
+      const int i =
+          min(max(__float2int_rn(d.r0.x * inv_spacing), 0), pl.intervals - 1);
+      const float t = ((d.r0.x - float(i) * spacing) + d.corr.x) * pl.inv_half;
+      const float4* r = reinterpret_cast<const float4*>(
+          table + (size_t(p) * pl.intervals + i) * RADIAL_REC);
+      const f2 u = radial_eval(r, t), v = radial_eval(r + RQ / 3, t),
+               w = radial_eval(r + 2 * (RQ / 3), t);
+      const float c = (Xr.x - Xr.y) * (Xr.x + Xr.y), s = (Xr.x + Xr.x) * Xr.y;
+      ex = pfma(pk(c, c), v, padd(ex, u));
+      ey = pfma(pk(s, s), v, ey);
+      ez = pfma(pk(Xr.x, Xr.x), w, ez);
+      if (kHolo) m1 += fmaxf(fabsf(u.x), fabsf(u.y));
+    }
+    const cplx<float> e[3] = {mk(ex.x, ex.y), mk(ey.x, ey.y), mk(ez.x, ez.y)};
+    if (kHolo) {
+      const float h = intensity<float>(e);
+      mark = radial_needs_fp64(h, m1);
+      if (!mark) reinterpret_cast<float*>(out)[size_t(item) * npts + pix] = h;
+    } else {
+      float2* o = reinterpret_cast<float2*>(out) + size_t(item) * 3 * npts;
+      for (int c = 0; c < 3; ++c) o[c * npts + pix] = make_float2(e[c].re, e[c].im);
+    }
+  }
+  if (kHolo) {
+    if (threadIdx.x == 0) s_marked = 0;
+    if (!__syncthreads_or(mark)) return;
+    if (mark) s_list[atomicAdd(&s_marked, 1)] = threadIdx.x;
+    __syncthreads();
+    auto where = [&](int l, double* x, double* y) {
+      *x = points[base + l];
+      *y = points[npts + base + l];
+      return base + l;
+    };
+    radial_resum64(pl, s_list, s_marked, where, spheres, pb, pe, nodes,
+                   reinterpret_cast<float*>(out) + size_t(item) * npts);
+  }
+}
+
+constexpr size_t kSmemLimit = size_t(200) * 1024;
+
+// float4 of the intervals that a tile's pixels can span, with the margins of
+// TileParticle.
+size_t radial_buffer(double spacing) {
+  return (size_t((kTile - 1) * 1.4142135623730951 / spacing) + 7) * (RADIAL_REC / 4);
+}
+
+size_t up256(size_t v) { return (v + 255) / 256 * 256; }
+
+size_t table_bytes(int nparticles, int intervals) {
+  return up256(sizeof(float) * RADIAL_REC * size_t(nparticles) * size_t(intervals));
+}
+
+size_t node_bytes(int nparticles, int intervals) {
+  return up256(sizeof(double) * RADIAL_FUNCS * size_t(nparticles) *
+               (size_t(intervals) + 2 * RADIAL_SIDE));
+}
+
+int grid_common(bool holo, const lmb_grid* grid, const lmb_sphere* spheres,
+                const double* points, long long npts, const int* item_start, int nitems,
+                int nparticles, int intervals, const double* ab, const int* nmax,
+                int nmax_cap, double k, int flags, double aberr, void* out, void* workspace, size_t workspace_bytes,
+                void* stream) {
+  if (nitems < 0 || nparticles < 0 || nmax_cap < 1 || nmax_cap > LMB_NMAX_LIMIT)
+    return LMB_ERR_ARG;
+  if (!grid || grid->nx < 0 || grid->ny < 0 || (points && npts < 0)) return LMB_ERR_ARG;
+  if (nitems == 0 || grid->nx == 0 || grid->ny == 0 || (points && npts == 0))
+    return LMB_OK;
+  if (!spheres || !item_start || !ab || !nmax || !out || intervals < 1) return LMB_ERR_ARG;
+  if (!(flags & LMB_CARTESIAN) || (flags & LMB_FP64)) return LMB_ERR_UNSUPPORTED;
+  if (!isfinite(aberr) || !(k > 0.) || nparticles > 65535 || nitems > 65535)
+    return LMB_ERR_ARG;
+  const long long tx = (grid->nx + kTile - 1) / kTile, ty = (grid->ny + kTile - 1) / kTile;
+  if (tx > 0x7fffffffLL || ty > 65535 || (npts + kListThreads - 1) / kListThreads > 0x7fffffffLL)
+    return LMB_ERR_ARG;
+  if (!workspace || workspace_bytes < lmb_radial_workspace_bytes(nparticles, intervals))
+    return LMB_ERR_WORKSPACE;
+  RadialPlan pl;
+  pl.spacing = radial_spacing(k);
+  if (!(pl.spacing > 0.)) return LMB_ERR_UNSUPPORTED;
+  pl.x0 = grid->x0;
+  pl.y0 = grid->y0;
+  pl.z = grid->z;
+  pl.nx = grid->nx;
+  pl.ny = grid->ny;
+  pl.k = k;
+  pl.aberr = aberr;
+  pl.inv_half = float(2. / pl.spacing);
+  pl.intervals = intervals;
+  pl.flags = flags;
+  const RadialMatrix A = radial_matrix();
+  float* table = reinterpret_cast<float*>(workspace);
+  double* nodes = reinterpret_cast<double*>(reinterpret_cast<char*>(workspace) +
+                                            table_bytes(nparticles, intervals));
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (nparticles > 0) {
+    const size_t smem = sizeof(double) * RADIAL_FUNCS * kNodeThreads +
+                        sizeof(Quad<double>) * 2 * (size_t(nmax_cap) + 1);
+    LMB_CK(smem_attr((const void*)k_radial_table, smem));
+    const dim3 g(unsigned((intervals + kChunk - 1) / kChunk), unsigned(nparticles));
+    k_radial_table<<<g, kNodeThreads, smem, st>>>(
+        pl, A, spheres, reinterpret_cast<const zd*>(ab), nmax, nmax_cap + 1, table, nodes);
+    LMB_CK(cudaGetLastError());
+  }
+  if (points) {
+    auto list = holo ? k_points_radial<true> : k_points_radial<false>;
+    const dim3 g{unsigned((npts + kListThreads - 1) / kListThreads), unsigned(nitems)};
+    list<<<g, kListThreads, 0, st>>>(pl, points, npts, spheres, item_start, table, nodes, out);
+    LMB_CK(cudaGetLastError());
+    return LMB_OK;
+  }
+  const size_t buffer = radial_buffer(pl.spacing);
+  const size_t smem = std::max(kStages * sizeof(float4) * buffer,
+                               sizeof(int) * size_t(kTile * kTile));
+  auto fn = holo ? k_field_radial<true> : k_field_radial<false>;
+  if (smem > kSmemLimit) return LMB_ERR_UNSUPPORTED;
+  LMB_CK(smem_attr((const void*)fn, smem));
+  const dim3 g{unsigned(tx), unsigned(ty), unsigned(nitems)};
+  fn<<<g, kPixThreads, smem, st>>>(pl, spheres, item_start, table, nodes, int(buffer), out);
+  LMB_CK(cudaGetLastError());
+  return LMB_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int lmb_grid_probe(const double* coords, long long npts, unsigned long long* out,
+                   void* stream) {
+  if (npts < 1 || !coords || !out) return LMB_ERR_ARG;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const unsigned blocks = unsigned(std::min<long long>((npts + 255) / 256, 1184));
+  k_probe_init<<<1, 1, 0, st>>>(npts, out);
+  k_probe_row<<<blocks, 256, 0, st>>>(coords, npts, out);
+  k_probe_check<<<blocks, 256, 0, st>>>(coords, npts, out);
+  k_probe_bounds<<<1, 1, 0, st>>>(out);
+  LMB_CK(cudaGetLastError());
+  return LMB_OK;
+}
+
+int lmb_radial_intervals(const lmb_grid* grid, long long npts, const lmb_sphere* spheres,
+                         int n, double k, double magnification, int flags, double aberration) {
+  if (!grid || !spheres || n < 1 || grid->nx < 1 || grid->ny < 1) return 0;
+  if (!(flags & LMB_CARTESIAN) || (flags & LMB_FP64)) return 0;
+  if (!(k > 0.) || !isfinite(k) || !(magnification > 0.) || !isfinite(aberration)) return 0;
+  if (!isfinite(grid->x0) || !isfinite(grid->y0) || !isfinite(grid->z)) return 0;
+  const double spacing = radial_spacing(k);
+  if (!(spacing > 0.)) return 0;
+  // a tile's intervals fit in shared memory
+  if (kStages * sizeof(float4) * radial_buffer(spacing) > kSmemLimit) return 0;
+  double far = 0.;
+  for (int i = 0; i < n; ++i) {
+    const lmb_sphere& s = spheres[i];
+    const double reach = radial_reach(grid->x0, grid->y0, grid->nx, grid->ny, s.x_p, s.y_p);
+    const double dz = fabs(grid->z - s.z_p);
+    // offsets up to 8192 px split exactly in FP32 (radial_distance)
+    if (!(reach < 8000.) || !(s.a_p > 0.) || !isfinite(s.z_p)) return 0;
+    if (!(k * (dz - s.a_p / magnification) >= RADIAL_CLEARANCE)) return 0;
+    // the aberration's phase turns by at most |c| / (2 |z_p|) per pixel, at
+    // rho = |z_p|, where the field's own band ends at 0.7 k
+    if (aberration != 0. && !(0.5 * fabs(aberration) <= 0.2 * k * fabs(s.z_p))) return 0;
+    if (reach > far) far = reach;
+  }
+  const int count = radial_count(far, spacing);
+  // A node costs about as much as two pixels' direct sums.
+  if (double(npts) < 2. * (count + 2 * RADIAL_SIDE))
+    return 0;
+  return count;
+}
+
+size_t lmb_radial_workspace_bytes(int nparticles, int intervals) {
+  if (nparticles < 0 || intervals < 1) return 0;
+  return table_bytes(nparticles, intervals) + node_bytes(nparticles, intervals);
+}
+
+int lmb_field_grid(const lmb_grid* grid, const double* points, long long npts,
+                   const lmb_sphere* spheres, const int* item_start,
+                   int nitems, int nparticles, int intervals, const double* ab,
+                   const int* nmax, int nmax_cap, double k, int flags, double aberration,
+                   void* out, void* workspace, size_t workspace_bytes, void* stream) {
+  return grid_common(false, grid, spheres, points, npts, item_start, nitems, nparticles, intervals, ab,
+                     nmax, nmax_cap, k, flags, aberration, out, workspace, workspace_bytes,
+                     stream);
+}
+
+int lmb_hologram_grid(const lmb_grid* grid, const double* points, long long npts,
+                      const lmb_sphere* spheres, const int* item_start,
+                      int nitems, int nparticles, int intervals, const double* ab,
+                      const int* nmax, int nmax_cap, double k, int flags, double aberration,
+                      void* out, void* workspace, size_t workspace_bytes, void* stream) {
+  return grid_common(true, grid, spheres, points, npts, item_start, nitems, nparticles, intervals, ab,
+                     nmax, nmax_cap, k, flags, aberration, out, workspace, workspace_bytes,
+                     stream);
+}
+
+}  // extern "C"

@@ -1,0 +1,172 @@
+// Radial tables: the field of a sphere in a plane z = const.
+//
+// At the pixels of one plane, everything that theory/LorenzMie.py:183-342
+// sums over the orders depends on the distance rho from the sphere's axis
+// alone; the azimuth phi enters only through the projection:
+//   E_x = U + V (x^2 - y^2),  E_y = V 2 x y,  E_z = Z x,
+// with (x, y) the offset from the axis, U = (X1 + X2) / 2, V = (X1 - X2) /
+// (2 rho^2), Z = Z1 / rho, X1 and X2 the x component at phi = 0 and phi = 90
+// degrees and Z1 the z component at phi = 0, phase included.  So the orders are summed in FP64 at equidistant nodes of rho,
+// a few per wavelength, and every pixel interpolates: a 1280x1024 frame
+// needs ~2700 sums a sphere instead of 1.3 million.
+//
+// The field in a plane above the sphere is band-limited: its transverse
+// wave numbers are at most k, plus evanescent waves that have decayed by
+// e^{-kappa d} over the distance d from the sphere.  Hence the node spacing
+// (RADIAL_HALF_WIDTH below) and the condition k d >= RADIAL_CLEARANCE.
+// U, V and Z are even in rho, which gives the nodes at rho < 0.
+//
+// From the nodes each interval of one spacing around node i gets the
+// polynomial of degree RADIAL_COEFS - 1 that interpolates, at the Chebyshev
+// points of the interval, the Lagrange interpolant through the RADIAL_TAPS
+// nodes around i.
+#pragma once
+
+#include "lmb_records.cuh"
+
+namespace lmb {
+
+enum {
+  RADIAL_TAPS = 17,
+  RADIAL_SIDE = RADIAL_TAPS / 2,
+  RADIAL_COEFS = 6,
+  RADIAL_FUNCS = 6,  // U, V, Z as (re, im)
+  // Floats per interval: 9 float4, an odd number, so that eight neighbouring
+  // intervals fall into different shared-memory banks.
+  RADIAL_REC = RADIAL_FUNCS * RADIAL_COEFS
+};
+
+// Node spacing and interval width in radians (k times pixels).  At the band
+// limit the 17-point interpolant is then off by at most 1e-9 (at 1 radian by
+// 2e-6), and the degree-5 polynomial by 2 (0.6 / 4)^6 / 6! = 3e-8: below the
+// FP32 rounding of its coefficients.  Measured against the oracle over radii
+// of 0.4-24 um from 2 px above the sphere on.
+#define RADIAL_SPACING 0.6
+// Distance of the plane from the sphere's surface, k d.
+#define RADIAL_CLEARANCE 1.8
+// The distance (pixels) that stands for the axis itself, where V and Z are
+// limits: there V and Z are off by (k rho)^2 ~ 1e-8 of themselves and the
+// cancellation in V costs as much; near the axis they contribute V rho^2 and
+// Z rho.
+#define RADIAL_AXIS 1e-4
+// Row c: the weights of the nodes in the coefficient of t^c, t = (rho - rho_i)
+// / (half a spacing).
+struct RadialMatrix {
+  double m[RADIAL_COEFS][RADIAL_TAPS];
+};
+
+// The Lagrange weights of the RADIAL_TAPS nodes around one of them at
+// offset x (in spacings).
+LMB_HD void radial_weights(double x, double* w) {
+  // prod_{l != j} (x - l) / (j - l) by prefix and suffix products
+  const double inv[RADIAL_TAPS] = {
+      // 1 / ((-1)^(16-m) m! (16-m)!)
+      1. / 20922789888000., -1. / 1307674368000., 1. / 174356582400.,
+      -1. / 37362124800., 1. / 11496038400., -1. / 4790016000.,
+      1. / 2612736000., -1. / 1828915200., 1. / 1625702400.,
+      -1. / 1828915200., 1. / 2612736000., -1. / 4790016000.,
+      1. / 11496038400., -1. / 37362124800., 1. / 174356582400.,
+      -1. / 1307674368000., 1. / 20922789888000.};
+  double p = 1.;
+  for (int j = 0; j < RADIAL_TAPS; ++j) {
+    w[j] = p * inv[j];
+    p *= x - double(j - RADIAL_SIDE);
+  }
+  p = 1.;
+  for (int j = RADIAL_TAPS - 1; j >= 0; --j) {
+    w[j] *= p;
+    p *= x - double(j - RADIAL_SIDE);
+  }
+}
+
+// Coefficients in powers of t of the polynomial through values at the
+// Chebyshev points t_i = cos(pi (i + 1/2) / RADIAL_COEFS): row c, column i.
+struct RadialPowers {
+  double t[RADIAL_COEFS];
+  double m[RADIAL_COEFS][RADIAL_COEFS];
+  RadialPowers() {
+    const int n = RADIAL_COEFS;
+    const double pi = 3.141592653589793;
+    double tq[RADIAL_COEFS][RADIAL_COEFS] = {};  // T_q in powers
+    tq[0][0] = tq[1][1] = 1.;
+    for (int q = 2; q < n; ++q)
+      for (int p = 0; p < n; ++p)
+        tq[q][p] = (p ? 2. * tq[q - 1][p - 1] : 0.) - tq[q - 2][p];
+    for (int i = 0; i < n; ++i) {
+      t[i] = cos(pi * (i + 0.5) / n);
+      for (int p = 0; p < n; ++p) {
+        m[p][i] = 0.;
+        for (int q = 0; q < n; ++q)
+          m[p][i] += (q ? 2. : 1.) / n * cos(pi * q * (i + 0.5) / n) * tq[q][p];
+      }
+    }
+  }
+};
+
+inline RadialMatrix radial_matrix() {
+  static const RadialPowers P;
+  RadialMatrix A = {};
+  for (int i = 0; i < RADIAL_COEFS; ++i) {
+    double w[RADIAL_TAPS];
+    radial_weights(0.5 * P.t[i], w);
+    for (int c = 0; c < RADIAL_COEFS; ++c)
+      for (int j = 0; j < RADIAL_TAPS; ++j) A.m[c][j] += P.m[c][i] * w[j];
+  }
+  return A;
+}
+
+// U, V, Z (re, im each) at distance rho > 0 (pixels) from the axis of a
+// particle at height zp, in the plane z; dzc = z - zp.  rec: order_record's
+// FP64 records (2 Quads per order).  aberr: see aberration_wave.
+LMB_HD void radial_field(double k, double rho, double dzc, double z, double zp,
+                         bool bohren, double aberr, const Quad<double>* rec,
+                         int nm, double* v) {
+  const Geometry<double> g = geometry<double>(k, rho, 0., dzc, z, zp, bohren);
+  const Sums<double> s = order_sum<double>(g, rec, nm);
+  const double ikr = g.ikr;
+  const zd e0 = (g.sint * ikr * ikr) * s.s0, e1 = ikr * s.s1, e2 = ikr * s.s2;
+  zd ph = g.phase;
+  if (aberr != 0.) {
+    double d[3];
+    ph = ph * conj(aberration_wave<double>(aberr, rho, 0., zp, d));
+  }
+  const zd x1 = ph * (g.sint * e0 + g.mu * e1);
+  const zd x2 = -(ph * e2);
+  const zd zz = ph * (g.mu * e0 - g.sint * e1);
+  const double ir = 1. / rho, h = 0.5 * ir * ir;
+  v[0] = 0.5 * (x1.re + x2.re);
+  v[1] = 0.5 * (x1.im + x2.im);
+  v[2] = h * (x1.re - x2.re);
+  v[3] = h * (x1.im - x2.im);
+  v[4] = ir * zz.re;
+  v[5] = ir * zz.im;
+}
+
+// Distance of a pixel from the axis.  (X, Y): pixel minus particle rounded
+// to 2^-10 px (exact in FP32 up to 8192 px), (a, b) the remainders; lx =
+// X^2's rounding error plus 2 a X + a^2, ly alike.  rho = r0 + corr with an
+// error of ~1e-7 of corr, i.e. far below the FP32 rounding of rho, which at
+// 1500 px would turn the phase by 1e-4 rad.
+struct RadialDistance {
+  f2 r0, corr;
+};
+
+LMB_HD f2 pneg(f2 a) { return pk(-a.x, -a.y); }
+LMB_HD f2 psub(f2 a, f2 b) { return pfma(pk(-1.f, -1.f), b, a); }
+
+LMB_HD RadialDistance radial_distance(f2 px, f2 lx, f2 qy, f2 ly) {
+  const f2 s = padd(px, qy);
+  const f2 bb = psub(s, px);
+  const f2 err = padd(psub(px, psub(s, bb)), psub(qy, bb));  // s + err exact
+  const f2 low = padd(padd(lx, ly), err);
+  const f2 sh = padd(s, low);
+  const f2 sl = padd(psub(s, sh), low);
+  const f2 y = pk(rsqrt_seed(fmaxf(sh.x, 1e-24f)), rsqrt_seed(fmaxf(sh.y, 1e-24f)));
+  RadialDistance d;
+  d.r0 = pmul(sh, y);
+  const f2 e = padd(pfma(pneg(d.r0), d.r0, sh), sl);
+  d.corr = pmul(pmul(pk(0.5f, 0.5f), y), e);
+  return d;
+}
+
+}  // namespace lmb

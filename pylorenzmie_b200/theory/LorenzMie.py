@@ -122,6 +122,7 @@ class LorenzMie(LMObject):
     def _allocate(self):
         '''Invalidate the device copy of the coordinates.'''
         self._coords_dev = None
+        self._grid_dev = None
 
     @property
     def _coords(self):
@@ -131,15 +132,24 @@ class LorenzMie(LMObject):
                 np.ascontiguousarray(self._coordinates)).to(self.device)
         return self._coords_dev
 
+    @property
+    def _grid(self):
+        '''The coordinates as pixels of one plane (K.make_grid), or None;
+        found once for each device copy of the coordinates.'''
+        if self._grid_dev is None:
+            c = self._coords
+            npts = c.shape[1]
+            self._grid_dev = (K.make_grid(
+                self._coordinates[2, 0], npts, K.probe_grid(c).cpu().numpy())
+                if npts else None,)
+        return self._grid_dev[0]
+
     # ------------------------------------------------------------------
     def _prepare(self, particle_lists, deriv=False):
         '''Device spheres, item offsets and Mie coefficients.'''
         flat = [p for plist in particle_lists for p in plist]
         inst = self.instrument
         counts = [len(pl) for pl in particle_lists]
-        item_start = K.to_device_async(
-            np.concatenate([[0], np.cumsum(counts)]).astype(np.int32),
-            self.device)
         rec = _records(flat)
         if len(flat) == 0:
             cap = 1
@@ -153,7 +163,14 @@ class LorenzMie(LMObject):
             raise ValueError(f'a particle needs {cap - 2} partial-wave '
                              f'orders; the limit is '
                              f'{K._native.LMB_NMAX_LIMIT}')
-        sp = K.spheres_tensor(rec, self.device)
+        # one upload: the records, then the items' offsets
+        host = np.empty(12 * len(flat) + len(counts) + 1, dtype=np.int32)
+        host[:12 * len(flat)] = rec.view(np.int32).reshape(-1)
+        host[12 * len(flat)] = 0
+        np.cumsum(counts, out=host[12 * len(flat) + 1:])
+        dev = K.to_device_async(host, self.device)
+        sp = dev[:12 * len(flat)].view(torch.float64).view(-1, 6)
+        item_start = dev[12 * len(flat):]
         if len(flat):
             # The capacity comes from the particles themselves, so the
             # coefficient kernel can fail only on invalid parameters:
@@ -173,24 +190,32 @@ class LorenzMie(LMObject):
                              device=self.device)
             dab, nmax = None, torch.zeros(1, dtype=torch.int32,
                                           device=self.device)
-        return sp, item_start, ab, dab, nmax, cap
+        return sp, item_start, ab, dab, nmax, cap, rec
 
     def _aberration(self):
         '''Coefficient of a spherical-aberration phase applied to every
         particle's field (0: ideal optics; see theory/Aberrated.py).'''
         return 0.
 
+    def _items(self, particle_lists, cartesian, bohren, field):
+        sp, item_start, ab, _, nmax, cap, rec = self._prepare(particle_lists)
+        if not self.double_precision and cartesian and len(rec) and \
+                self._grid is not None:
+            out = K.on_grid(self._grid, self._coords, rec, sp, item_start, ab, nmax, cap,
+                            self.instrument, cartesian, bohren,
+                            self._aberration(), field)
+            if out is not None:
+                return out
+        direct = K.field if field else K.hologram
+        return direct(self._coords, sp, item_start, ab, nmax, cap,
+                      self.instrument.wavenumber(), cartesian, bohren,
+                      self.double_precision, self._aberration())
+
     def _field_items(self, particle_lists, cartesian, bohren):
-        sp, item_start, ab, _, nmax, cap = self._prepare(particle_lists)
-        return K.field(self._coords, sp, item_start, ab, nmax, cap,
-                       self.instrument.wavenumber(), cartesian, bohren,
-                       self.double_precision, self._aberration())
+        return self._items(particle_lists, cartesian, bohren, True)
 
     def _hologram_items(self, particle_lists, cartesian, bohren):
-        sp, item_start, ab, _, nmax, cap = self._prepare(particle_lists)
-        return K.hologram(self._coords, sp, item_start, ab, nmax, cap,
-                          self.instrument.wavenumber(), cartesian, bohren,
-                          self.double_precision, self._aberration())
+        return self._items(particle_lists, cartesian, bohren, False)
 
     # ------------------------------------------------------------------
     def field(self, cartesian=True, bohren=True, device=False):
@@ -248,7 +273,7 @@ class LorenzMie(LMObject):
         if not isinstance(self.particle, Sphere) and not (
                 hasattr(self.particle, 'a_p') and len(self.particle) == 1):
             raise TypeError('jac() supports single Sphere particles only')
-        sp, _, ab, dab, nmax, cap = self._prepare([[self.particle]],
+        sp, _, ab, dab, nmax, cap, _ = self._prepare([[self.particle]],
                                                   deriv=True)
         _, J = K.jacobian(self._coords, sp, ab, dab, nmax, cap,
                           self.instrument.wavenumber(),
@@ -261,7 +286,7 @@ class LorenzMie(LMObject):
 
     def hologram_and_jac(self, bohren=True):
         '''Hologram (npts,) and Jacobian (6, npts) tensors in one pass.'''
-        sp, _, ab, dab, nmax, cap = self._prepare([[self.particle]],
+        sp, _, ab, dab, nmax, cap, _ = self._prepare([[self.particle]],
                                                   deriv=True)
         h, J = K.jacobian(self._coords, sp, ab, dab, nmax, cap,
                           self.instrument.wavenumber(), bohren,

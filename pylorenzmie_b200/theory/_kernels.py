@@ -226,6 +226,74 @@ def field(coords, spheres, item_start, ab, nmax, cap, k, cartesian=True,
     return out
 
 
+def probe_grid(coords):
+    '''Queue the check whether coords (3, npts) is a unit-step pixel grid,
+    or at least in one plane: a device tensor for make_grid.'''
+    out = torch.empty(7, dtype=torch.int64, device=coords.device)
+    _native.check(_native.load().lmb_grid_probe(
+        ptr(coords), coords.shape[1], ptr(out), stream_handle(coords.device)),
+        'lmb_grid_probe')
+    return out
+
+
+def make_grid(z, npts, probed):
+    '''(Grid, whether the pixels are that grid's) of a probed coordinate
+    list in the plane z (a numpy int64 array), the grid being a box around
+    the pixels otherwise; None if they are not in one plane.'''
+    nx, off_grid, off_plane = (int(v) for v in probed[:3])
+    x0, y0, x1, y1 = (float(v) for v in probed[3:].view(np.float64))
+    if off_plane or max(x1 - x0, y1 - y0) > 1e9:
+        return None
+    if off_grid == 0 and npts % nx == 0:
+        return _native.Grid(x0, y0, float(z), nx, npts // nx), True
+    return _native.Grid(x0, y0, float(z), int(np.ceil(x1 - x0)) + 1,
+                        int(np.ceil(y1 - y0)) + 1), False
+
+
+def on_grid(grid, coords, records, spheres, item_start, ab, nmax, cap,
+            instrument, cartesian, bohren, aberration, field=False):
+    '''(nitems, npts) float32 holograms, or with ``field`` (nitems, 3,
+    npts) complex64 fields, of pixels in one plane (make_grid's result)
+    from radial tables (lmb_hologram_grid, lmb_field_grid); None where they
+    do not apply.  records: the spheres' host records.'''
+    grid, full = grid
+    npts = coords.shape[1]
+    lib = _native.load()
+    k = float(instrument.wavenumber())
+    flags = _flags(cartesian, bohren, False)
+    n = len(records)
+    # Images of less than 200x200 pixels: their direct sums take as long as
+    # the tables (10 us) in one launch fewer.  Particles are the table
+    # kernel's grid rows.
+    if n > 65535 or (full and npts < 40000):
+        return None
+    intervals = lib.lmb_radial_intervals(
+        grid, npts, records.ctypes.data, n, k, float(instrument.magnification),
+        flags, float(aberration))
+    if not intervals:
+        return None
+    nbytes = lib.lmb_radial_workspace_bytes(n, intervals)
+    if nbytes > RADIAL_WORKSPACE_LIMIT:
+        return None
+    dev = spheres.device
+    nitems = item_start.shape[0] - 1
+    if field:
+        out = torch.empty((nitems, 3, npts), dtype=torch.complex64, device=dev)
+    else:
+        out = torch.empty((nitems, npts), dtype=torch.float32, device=dev)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    name = 'lmb_field_grid' if field else 'lmb_hologram_grid'
+    _native.check(getattr(lib, name)(
+        grid, None if full else ptr(coords), npts, ptr(spheres),
+        ptr(item_start), nitems, n, intervals, ptr(ab), ptr(nmax), cap, k, flags, float(aberration), ptr(out), ptr(ws),
+        nbytes, stream_handle(dev)), name)
+    return out
+
+
+# radial tables larger than this are not built (the direct sums need none)
+RADIAL_WORKSPACE_LIMIT = 4 << 30
+
+
 def jacobian(coords, spheres, ab, dab, nmax, cap, k, bohren=True,
              aberration=0.):
     '''Holograms (n, npts) and Jacobians (n, 6, npts), float64, FP32 sums;
