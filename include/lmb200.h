@@ -362,9 +362,20 @@ typedef struct lmb_fit_settings {
   int flags;       /* LMB_BOHREN */
   int max_iterations; /* hard cap on evaluations per call, >= 1 */
   int tile_config;    /* launch shape of the evaluation kernel, 0 = default;
-                         see lmb_fit_tile_config */
-  int reserved;
+                         see lmb_fit_tile_config; or LMB_FIT_RADIAL */
+  int reach;          /* with LMB_FIT_RADIAL, >= 0: an upper estimate of a
+                         pixel's distance from its sphere (px), which sets
+                         the room for the tables; 0: unknown */
 } lmb_fit_settings;
+
+/*
+ * lmb_fit_settings.tile_config of the evaluation from radial tables: every
+ * feature's sums over the orders are formed in FP64 at a few distances per
+ * wavelength and its pixels interpolate (a feature whose focal plane cuts or
+ * almost touches its sphere, or whose table finds no room, is summed pixel
+ * by pixel).  The launch shapes of lmb_fit_tile_config sum at every pixel.
+ */
+#define LMB_FIT_RADIAL 100
 
 /*
  * Launch shapes of the fit's evaluation kernel (threads per CTA, pixels per

@@ -25,6 +25,7 @@ LMB_CARTESIAN = 1
 LMB_BOHREN = 2
 LMB_FP64 = 4
 LMB_NMAX_LIMIT = 1024
+LMB_FIT_RADIAL = 100
 
 # struct layouts mirrored from include/lmb200.h
 SPHERE_DTYPE = np.dtype([('x_p', '<f8'), ('y_p', '<f8'), ('z_p', '<f8'),
@@ -43,7 +44,7 @@ class FitSettings(ctypes.Structure):
                 ('gtol', ctypes.c_double), ('factor', ctypes.c_double),
                 ('max_nfev', ctypes.c_int), ('variables', ctypes.c_int),
                 ('flags', ctypes.c_int), ('max_iterations', ctypes.c_int),
-                ('tile_config', ctypes.c_int), ('reserved', ctypes.c_int)]
+                ('tile_config', ctypes.c_int), ('reach', ctypes.c_int)]
 
 
 class FitStats(ctypes.Structure):

@@ -186,7 +186,8 @@ class Frame(Hologram):
             params, res, _ = _fit.fit_items(
                 items, starts, members[0].model.instrument, opt0.variables,
                 opt0.settings, device=members[0].model.device, layers=layers,
-                autotune=len(members) >= 64, aberration=opt0._aberration())
+                autotune=_fit.default_autotune(len(members)),
+                aberration=opt0._aberration())
             for j, f in enumerate(members):
                 f.optimizer._data = np.asarray(items[j][0])
                 f.optimizer.model.coordinates = items[j][2] if \

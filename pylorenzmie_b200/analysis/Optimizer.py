@@ -294,8 +294,9 @@ class Optimizer(LMObject):
         starts    : array (B, 6) of x_p, y_p, z_p, a_p, n_p, k_p (overrides
                     the particles' start values)
         autotune  : time the evaluation kernel's launch shapes once per
-                    problem class and use the fastest (default: batches of
-                    64 features or more)
+                    problem class and use the fastest where the radial
+                    tables do not apply (default: timed only there, for
+                    batches of 64 features or more)
         chunks    : pipeline depth: the batch is fitted in this many parts,
                     each on its own stream, so that converting and copying
                     one part overlaps the fit of the previous one (default:
@@ -317,7 +318,7 @@ class Optimizer(LMObject):
                 getattr(p, 'k_p', 0.)] for p in particles], dtype=float)
         items = [self._pixels(h) for h in holograms]
         if autotune is None:
-            autotune = len(holograms) >= 64
+            autotune = _fit.default_autotune(len(holograms))
         params, res, npix = _fit.fit_items(
             items, starts, self.model.instrument, self.variables,
             self.settings, device=self.model.device, layers=layers,
@@ -333,8 +334,8 @@ class Optimizer(LMObject):
         batches : iterable of (holograms, starts) or (holograms,
                   particles) pairs; starts an array (B, 6), particles a
                   list of Sphere or LayeredSphere start values
-        autotune: time the evaluation kernel's launch shapes on the first
-                  batch (default: when it has 64 features or more)
+        autotune: time the evaluation kernel's launch shapes (default: as
+                  optimize_batch, by the first batch's size)
         depth   : fits running at once; the next batch is converted and
                   copied while they run.  Default 2, which keeps the GPU
                   busy; 4 when the first batch holds LayeredSphere
@@ -362,8 +363,9 @@ class Optimizer(LMObject):
                                        for p in second], dtype=float)
                 if first[0]:
                     first[0] = False
-                    self._stream_tune = (autotune if autotune is not None
-                                         else len(holograms) >= 64)
+                    self._stream_tune = (
+                        autotune if autotune is not None
+                        else _fit.default_autotune(len(holograms)))
                 yield [self._pixels(h) for h in holograms], starts, layers
 
         gen = items()

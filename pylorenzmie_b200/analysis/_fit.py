@@ -4,6 +4,8 @@ Packs crops of normalized holograms into one float32 buffer, copies it to
 the device through pinned memory, runs every feature's Levenberg-Marquardt
 fit in the CUDA library, and returns fitted parameters and statistics.
 '''
+import math
+
 import numpy as np
 import torch
 
@@ -154,6 +156,35 @@ class PackedFeatures:
             f.result()
         return out
 
+    def reach(self, starts):
+        '''An upper estimate of a pixel's distance from its sphere (px) in
+        fits from starts (B, 6): the farthest pixel at the start and 10 px
+        for the sphere to move; inf where it is not known.'''
+        f = self.features
+        if len(f) == 1 and f['nx'][0] > 0:     # without array arithmetic
+            x0, y0, nx, ny, _, _ = f[0].item()
+            x, y = x0 - float(starts[0, 0]), y0 - float(starts[0, 1])
+            r = math.hypot(max(abs(x), abs(x + nx - 1)),
+                           max(abs(y), abs(y + ny - 1))) + 10.
+            return r if math.isfinite(r) else math.inf
+        x, y = f['x0'] - starts[:, 0], f['y0'] - starts[:, 1]
+        x1, y1 = x + (f['nx'] - 1), y + (f['ny'] - 1)
+        if self.coords is not None and self.coords.size:
+            c = self.coords.reshape(-1, 2)
+            listed = f['nx'] == 0
+            if np.all(f['npix'] > 0):
+                at = f['data_offset']
+                lo = np.minimum.reduceat(c, at) - starts[:, :2]
+                hi = np.maximum.reduceat(c, at) - starts[:, :2]
+            else:
+                lo = c.min(axis=0) - starts[:, :2]
+                hi = c.max(axis=0) - starts[:, :2]
+            x, x1 = np.where(listed, lo[:, 0], x), np.where(listed, hi[:, 0], x1)
+            y, y1 = np.where(listed, lo[:, 1], y), np.where(listed, hi[:, 1], y1)
+        r = np.maximum(x * x, x1 * x1) + np.maximum(y * y, y1 * y1)
+        r = float(np.sqrt(r.max())) + 10.
+        return r if np.isfinite(r) else np.inf
+
     @property
     def data(self):
         if self._data is None:
@@ -279,7 +310,7 @@ def upload(packed, starts, device=None):
 def fit_device(d_feat, d_data, d_coords, d_params, nfeatures, total_pixels,
                instrument, variables, settings=None, nmax_cap=None,
                starts_host=None, stats=False, tile_config=0, layers=None,
-               ready=None, wait_seconds=60., aberration=0.):
+               ready=None, wait_seconds=60., aberration=0., reach=0):
     '''Run lmb_fit_batch on device-resident inputs.  d_params is updated in
     place with the fitted values; returns (results tensor (B*80 uint8),
     FitStats or None).  With ``ready`` (a device int32 tensor) the fit is
@@ -287,7 +318,9 @@ def fit_device(d_feat, d_data, d_coords, d_params, nfeatures, total_pixels,
     advances it.  A nonzero ``aberration`` (the coefficient c of the
     spherical-aberration phase, AberratedLorenzMie._aberration) fits the
     aberrated model (lmb_fit_batch_aberrated, or lmb_fit_batch_streamed
-    with the coefficient).'''
+    with the coefficient).  ``tile_config``: a launch shape
+    (lmb_fit_tile_config), or LMB_FIT_RADIAL with ``reach``
+    (PackedFeatures.reach).'''
     dev = d_data.device
     lib = _native.load()
     settings = dict(DEFAULT_SETTINGS if settings is None else settings)
@@ -311,6 +344,7 @@ def fit_device(d_feat, d_data, d_coords, d_params, nfeatures, total_pixels,
     st.flags = _native.LMB_BOHREN
     st.max_iterations = st.max_nfev
     st.tile_config = int(tile_config)
+    st.reach = int(reach)
     fs = _native.FitStats() if stats else None
     if aberration and ready is None:
         if layers is None:
@@ -385,6 +419,50 @@ def default_shape(nfeatures):
     return SMALL_SHAPE if nfeatures < SMALL_BATCH else 0
 
 
+# Reach (k times px) of the features that the evaluation from radial tables
+# takes: the table's room in shared memory, ~650 intervals of 0.65 radian
+# (crops of 500 px at the default magnification).  Measured on a B200 against
+# launch shape 0: an evaluation of 256 features of 201x201 px 1.14 -> 0.13 ms.
+# A table costs ~15 us of serial FP64 work, whatever the pixels, so batches
+# of fewer than SMALL_BATCH features of at most RADIAL_PIXELS pixels (a
+# frame's features on their random subsets) keep SMALL_SHAPE: 32 features of
+# 1460 px 22 against 16 us.  Multilayer spheres keep the sums at every pixel:
+# their uncertainties in a_p and z_p can follow the rounding of the Jacobian
+# (a batch of 24 moved by up to 9e-5 of itself, towards the 64-bit values).
+RADIAL_REACH = 400.
+RADIAL_PIXELS = 4096
+LARGE = 'large'
+
+
+def default_autotune(nfeatures):
+    '''autotune of a batch whose caller does not say: LARGE (where the
+    radial tables do not apply) for 64 features or more.'''
+    return LARGE if nfeatures >= SMALL_BATCH else False
+
+
+def evaluation(packed, starts, instrument, variables, nmax_cap, layers, dev,
+               autotune, aberration):
+    '''(tile_config, reach) of a batch's evaluation kernel: radial tables
+    where they apply, else a launch shape that sums at every pixel, timed
+    with ``autotune`` (LARGE: only if it is needed).'''
+    B = starts.shape[0]
+    reach = 0
+    npix = packed.features['npix']
+    if layers is None and (B >= SMALL_BATCH or (
+            npix[0] if B == 1 else npix.max()) > RADIAL_PIXELS):
+        reach = packed.reach(starts)
+        if reach * float(instrument.wavenumber()) > RADIAL_REACH:
+            reach = 0
+    shape = default_shape(B)
+    if autotune and not aberration and not (reach and autotune is LARGE):
+        from .. import autotune as _tuner     # the aberrated fit has one shape
+        shape = _tuner.tune(packed, starts, instrument, variables, nmax_cap,
+                            layers, dev)
+    if reach:
+        return _native.LMB_FIT_RADIAL, int(np.ceil(reach))
+    return shape, 0
+
+
 def fit_packed(packed, starts, instrument, variables, settings=None,
                device=None, nmax_cap=None, stats=False, layers=None,
                autotune=False, aberration=0.):
@@ -400,15 +478,13 @@ def fit_packed(packed, starts, instrument, variables, settings=None,
     if nmax_cap is None:
         nmax_cap = fit_capacity(starts, float(instrument.n_m),
                                 float(instrument.wavelength), layers)
-    tile_config = default_shape(B)
-    if autotune and not aberration:   # the aberrated fit has one shape
-        from .. import autotune as _tuner
-        tile_config = _tuner.tune(packed, starts, instrument, variables,
-                                  nmax_cap, layers, d_data.device)
+    tile_config, reach = evaluation(packed, starts, instrument, variables,
+                                    nmax_cap, layers, d_data.device, autotune,
+                                    aberration)
     d_res, fs = fit_device(d_feat, d_data, d_coords, d_params, B,
                            packed.total, instrument, variables, settings,
                            nmax_cap, starts, stats, tile_config=tile_config,
-                           layers=layers, aberration=aberration)
+                           layers=layers, aberration=aberration, reach=reach)
     params = d_params.view(torch.float64).reshape(B, 6).cpu().numpy()
     res = d_res[:B * _native.RESULT_DTYPE.itemsize].cpu().numpy().view(
         _native.RESULT_DTYPE).copy()
@@ -486,11 +562,9 @@ def fit_items(items, starts, instrument, variables, settings=None,
     dev = get_device(device)
     nmax_cap = fit_capacity(starts, float(instrument.n_m),
                             float(instrument.wavelength), layers)
-    tile_config = default_shape(B)
-    if autotune and not aberration:   # the aberrated fit has one shape
-        from .. import autotune as _tuner
-        tile_config = _tuner.tune(packed, starts, instrument, variables,
-                                  nmax_cap, layers, dev)
+    tile_config, reach = evaluation(packed, starts, instrument, variables,
+                                    nmax_cap, layers, dev, autotune,
+                                    aberration)
     ranges = split_by_pixels(npix, chunks)
     # pinned layout: [features | starts | coords | data], 256-byte aligned
     pieces = [packed.features.view(np.uint8), starts.view(np.uint8)]
@@ -529,7 +603,7 @@ def fit_items(items, starts, instrument, variables, settings=None,
                               d_params, B, packed.total, instrument,
                               variables, settings, nmax_cap, starts,
                               tile_config, layers, d_ready, wait_seconds,
-                              aberration)
+                              aberration, reach)
     offs = packed.features['data_offset']
     try:
         for k, (a, b) in enumerate(ranges):
@@ -562,13 +636,15 @@ def fit_items(items, starts, instrument, variables, settings=None,
 
 def _fit_streamed(stream, d_feat, d_data, d_coords, d_params, n, total,
                   instrument, variables, settings, nmax_cap, starts,
-                  tile_config, layers, d_ready, wait_seconds, aberration=0.):
+                  tile_config, layers, d_ready, wait_seconds, aberration=0.,
+                  reach=0):
     with torch.cuda.stream(stream):
         d_res, _ = fit_device(d_feat, d_data, d_coords, d_params, n, total,
                               instrument, variables, settings, nmax_cap,
                               starts, False, tile_config=tile_config,
                               layers=layers, ready=d_ready,
-                              wait_seconds=wait_seconds, aberration=aberration)
+                              wait_seconds=wait_seconds, aberration=aberration,
+                              reach=reach)
         params = d_params.view(torch.float64).reshape(n, 6).cpu().numpy()
         res = d_res[:n * _native.RESULT_DTYPE.itemsize].cpu().numpy().view(
             _native.RESULT_DTYPE).copy()
@@ -682,17 +758,18 @@ def fit_stream(batches, instrument, variables, settings=None, device=None,
         _stream_staging.append(_Staging())
     slots = _Slots(depth)
     done_events = [None] * nstage
-    tile_config = None
     k = 0
 
-    def launch(fit_slot, ev, views, B, total, nmax_cap, starts, layers):
+    def launch(fit_slot, ev, views, B, total, nmax_cap, starts, layers,
+               tile_config, reach):
         s_fit = _stream_fit_stream(dev, fit_slot)
         for v in views:
             if v is not None:
                 v.record_stream(s_fit)
         return _stream_worker(depth).submit(
             _fit_after, s_fit, ev, views, B, total, instrument, variables,
-            settings, nmax_cap, starts, tile_config, layers, aberration)
+            settings, nmax_cap, starts, tile_config, layers, aberration,
+            reach)
 
     try:
         for items, starts, layers in batches:
@@ -708,13 +785,9 @@ def fit_stream(batches, instrument, variables, settings=None, device=None,
                 continue
             nmax_cap = fit_capacity(starts, float(instrument.n_m),
                                     float(instrument.wavelength), layers)
-            if tile_config is None:
-                tile_config = default_shape(B)
-                if autotune and not aberration:
-                    from .. import autotune as _tuner
-                    tile_config = _tuner.tune(packed, starts, instrument,
-                                              variables, nmax_cap, layers,
-                                              dev)
+            tile_config, reach = evaluation(packed, starts, instrument,
+                                            variables, nmax_cap, layers, dev,
+                                            autotune, aberration)
             slot = k % nstage
             if done_events[slot] is not None:
                 done_events[slot].synchronize()  # its last copy has landed
@@ -728,7 +801,7 @@ def fit_stream(batches, instrument, variables, settings=None, device=None,
             slots.wait_slot()
             yield from slots.ready()
             slots.submit(launch, npix, ev, views, B, packed.total, nmax_cap,
-                         starts, layers)
+                         starts, layers, tile_config, reach)
             k += 1
         yield from slots.drain()
     finally:
@@ -745,14 +818,16 @@ def _collect(entry):
 
 
 def _fit_after(stream, event, views, n, total, instrument, variables,
-               settings, nmax_cap, starts, tile_config, layers, aberration=0.):
+               settings, nmax_cap, starts, tile_config, layers, aberration=0.,
+               reach=0):
     d_feat, d_data, d_coords, d_params = views
     stream.wait_event(event)
     with torch.cuda.stream(stream):
         d_res, _ = fit_device(d_feat, d_data, d_coords, d_params, n, total,
                               instrument, variables, settings, nmax_cap,
                               starts, False, tile_config=tile_config,
-                              layers=layers, aberration=aberration)
+                              layers=layers, aberration=aberration,
+                              reach=reach)
         params = d_params.view(torch.float64).reshape(n, 6).cpu().numpy()
         res = d_res[:n * _native.RESULT_DTYPE.itemsize].cpu().numpy().view(
             _native.RESULT_DTYPE).copy()

@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "lmb200.h"
+#include "lmb_fit_radial.cuh"
 #include "lmb_kernels.cuh"
 #include "lmb_launch.cuh"
 
@@ -67,6 +68,35 @@ constexpr int kScalarShape = 1;  // scalar loop, used when pair records do not f
 // pair records take 256 B per order: above this they no longer fit in
 // shared memory beside the kernels' own buffers, and the scalar loop runs
 constexpr size_t kPairSmemLimit = size_t(200) * 1024;
+
+// Room for the tables of k_fit_eval_radial.  reach: an upper estimate of a
+// pixel's distance from its sphere (px), 0 if unknown.  The hologram's
+// oscillation is mostly slower than k per pixel, so the room is for that
+// rate; a part that needs more sums the orders at its pixels instead.
+struct RadialFitLaunch {
+  int cap;
+  size_t smem;
+};
+constexpr size_t kRadialFitSmem = size_t(200) * 1024;
+
+RadialFitLaunch radial_fit_launch(double k, int reach, int nmax_cap, bool kp) {
+  const size_t per = sizeof(float4) * fitr_rec(kp) + sizeof(double) * fitr_funcs(kp);
+  const size_t fixed = sizeof(double) * fitr_funcs(kp) * 2 * RADIAL_SIDE +
+                       sizeof(FitrOrder) * (size_t(nmax_cap) + 1);
+  RadialFitLaunch l = {0, 0};
+  // thousands of orders leave no room for the tables
+  if (fixed > kRadialFitSmem / 2) return l;
+  const int most = int((kRadialFitSmem - fixed) / per);
+  l.cap = most;
+  if (reach > 0)
+    l.cap = int(std::min(double(most), reach * k / FITR_SPACING + 8.));
+  // the direct sums' records take the place of the tables
+  const size_t direct = sizeof(Quad<float>) * JAC_QUADS * (size_t(nmax_cap) + 1);
+  while (per * size_t(l.cap) + sizeof(double) * fitr_funcs(kp) * 2 * RADIAL_SIDE < direct)
+    ++l.cap;
+  l.smem = per * size_t(l.cap) + fixed;
+  return l;
+}
 
 struct FitLayout {
   size_t state, ev, base, ab, dab, coef32, nmax, tile_begin, tiles,
@@ -674,6 +704,7 @@ int fit_batch_impl(const lmb_feature* features, int nfeatures,
   // Instrument.wavenumber, theory/Instrument.py:65-70 (same operation order)
   double k = 2. * 3.141592653589793 / wavelength;
   k *= n_m;
+  c.size_per_um = k;
   k *= magnification;
   c.k = k;
   c.inv_noise = 1. / noise;
@@ -691,8 +722,14 @@ int fit_batch_impl(const lmb_feature* features, int nfeatures,
 
   const size_t ab_smem = nlayers > 1 ? layered_scratch_bytes(nmax_cap + 1, nlayers)
                                      : ab_scratch_bytes(nmax_cap + 1);
-  const int shape_index = settings->tile_config;
+  const bool ask_radial = settings->tile_config == LMB_FIT_RADIAL;
+  const int shape_index = ask_radial ? 0 : settings->tile_config;
   if (shape_index < 0 || shape_index >= kNumEvalShapes) return LMB_ERR_ARG;
+  if (ask_radial && settings->reach < 0) return LMB_ERR_ARG;
+  const bool free_kp = c.variables & 32;
+  RadialFitLaunch rl = {0, 0};
+  if (ask_radial) rl = radial_fit_launch(k, settings->reach, nmax_cap, free_kp);
+  const bool radial = rl.cap > 0;
   EvalShape shape = aberr != 0. ? kAberrShapes[0] : kEvalShapes[shape_index];
   // pair records take 256 B per order: above ~800 orders they no longer fit
   // in shared memory next to the reduction buffer, so such batches use the
@@ -705,10 +742,23 @@ int fit_batch_impl(const lmb_feature* features, int nfeatures,
                                        : sizeof(Quad<float>) * JAC_QUADS) *
                            (size_t(nmax_cap) + 1);
   auto eval = shape.fn;
-  const size_t eval_smem = shape.warp_tiles ? coef_smem * (shape.tpb / 32) : coef_smem;
+  size_t eval_smem = shape.warp_tiles ? coef_smem * (shape.tpb / 32) : coef_smem;
+  auto eval_radial = free_kp ? k_fit_eval_radial<true> : k_fit_eval_radial<false>;
+  RadialMatrix rm = {};
+  c.parts = 0;
+  if (radial) {
+    // Parts per feature: enough to give every SM two blocks, while a part
+    // more costs its feature's nodes once more.
+    c.parts = std::max(1, std::min<int>(FITR_MAX_PARTS, 296 / nfeatures));
+    c.parts = std::min(c.parts, std::max(1, L.max_tiles / nfeatures));
+    rm = radial_matrix();
+    shape.tpb = FITR_TPB;
+    eval_smem = rl.smem;
+  }
   LMB_CK(smem_attr((const void*)k_fit_step, ab_smem));
-  LMB_CK(smem_attr((const void*)eval, eval_smem));
-  const int egrid = persistent_grid((const void*)eval, shape.tpb, eval_smem);
+  const void* eval_fn = radial ? (const void*)eval_radial : (const void*)eval;
+  LMB_CK(smem_attr(eval_fn, eval_smem));
+  const int egrid = persistent_grid(eval_fn, shape.tpb, eval_smem);
 
   // Optional timing: one event pair per evaluation launch, plus the span;
   // the events come from a per-thread, per-device pool kept across calls.
@@ -743,7 +793,10 @@ int fit_batch_impl(const lmb_feature* features, int nfeatures,
   auto launch_eval = [&]() -> bool {
     if (cudaMemsetAsync(c.counters + 0, 0, sizeof(int), st) != cudaSuccess) return false;
     if (stats && mark() != cudaSuccess) return false;
-    eval<<<egrid, shape.tpb, eval_smem, st>>>(c);
+    if (radial)
+      eval_radial<<<egrid, shape.tpb, eval_smem, st>>>(c, rm, rl.cap);
+    else
+      eval<<<egrid, shape.tpb, eval_smem, st>>>(c);
     if (stats && mark() != cudaSuccess) return false;
     launches += 1;
     ++evals;

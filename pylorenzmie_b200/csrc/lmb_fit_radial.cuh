@@ -1,0 +1,582 @@
+// Evaluation of the batched fits from radial tables.
+//
+// A feature's pixels lie in the plane z = 0, where the hologram of one
+// sphere at azimuth phi and distance rho from its axis is
+//   H = 1 + M + D (x^2 - y^2),
+// (x, y) the offset from the axis, M = (P + Q) / 2, D = (P - Q) / (2 rho^2),
+// P = |X1|^2 + |Z1|^2 + 2 Re X1 and Q = |X2|^2 + 2 Re X2 (lmb_radial.cuh).
+// M and D and their derivatives with respect to z_p, a_p, n_p (and k_p) are
+// even functions of rho; those with respect to x_p and y_p follow from
+// dM/drho and dD/drho, the slopes of the polynomials.  So a feature's sums
+// over the orders are formed in FP64 at ~100-200 nodes, and its pixels
+// (40 401 in a 201x201 crop) evaluate four pairs of degree-5 polynomials.
+#pragma once
+
+#include "lmb_kernels.cuh"
+#include "lmb_radial.cuh"
+
+namespace lmb {
+
+enum {
+  FITR_TPB = 256,
+  FITR_PAIRS = 4,     // (M, D) and its z_p, a_p, n_p derivatives
+  FITR_MAX_PARTS = 16
+};
+
+// float4 per interval: 3 per pair; an odd number keeps neighbouring
+// intervals in different banks.
+__host__ __device__ constexpr int fitr_rec(bool kp) { return kp ? 15 : 13; }
+__host__ __device__ constexpr int fitr_funcs(bool kp) { return 2 * (FITR_PAIRS + (kp ? 1 : 0)); }
+
+// Node spacing in radians of the hologram's own fastest oscillation (k q per
+// pixel, fitr_rate): the degree-5 polynomials of half a spacing to either
+// side are then off by 2 (0.65 / 4)^6 / 6! = 5e-8 of its amplitude.
+#define FITR_SPACING 0.65
+
+// The fastest oscillation of H along rho, in units of k: the carrier of the
+// interference term turns by k sin(theta), theta the steepest ray from the
+// sphere's edge to the outermost pixel, and |E|^2 by the difference of the
+// directions under which a pixel sees the sphere, at most twice the angle of
+// its edge from its axis.  The sphere's edge is widened by 6 / k for the
+// partial waves beyond the geometric radius.
+__device__ inline float fitr_rate(float k, float a_px, float z, float rho) {
+  const float a = a_px + 6.f / k;
+  const float far = rho + a;
+  const float s1 = far * rsqrtf(far * far + z * z);
+  const float s2 = 2.f * a * rsqrtf(a * a + z * z);
+  return fminf(2.f, fmaxf(0.25f, fmaxf(s1, s2)));
+}
+
+// FP64 order records: alpha, beta and their a_p, n_p derivatives, and what
+// the recurrences take of n alone (a division in their loop would cost as
+// much as all the rest of an order).
+struct FitrOrder {
+  zd v[6];  // alpha, beta, d alpha/da, d beta/da, d alpha/dn, d beta/dn
+  zd z[3];  // n (n+1) times alpha and its derivatives
+  double fn, tn1, cn, en;  // n, 2n - 1, 1 + 1/n, (2n + 1) / (n (n + 1))
+};
+
+struct FitrPlan {      // of one part of a feature, in shared memory
+  double spacing;
+  float ax, rx, ay, ry;  // crop origin minus particle: 2^-10 px part, rest
+  int lo, n;             // intervals
+  int radial;            // 0: sum the orders at every pixel
+};
+
+// A node's geometry beyond Geometry<double>: the factors of the projected
+// sums X1 = ph (A0 S0 + A1 S1), Z1 = ph (B0 S0 + B1 S1), X2 = ph C2 S2.
+struct FitrProjection {
+  double A0, A1, B0, B1, C2;
+};
+__device__ inline FitrProjection fitr_projection(const Geometry<double>& g) {
+  const double w0 = g.sint * g.ikr * g.ikr;
+  FitrProjection q;
+  q.A0 = g.sint * w0;
+  q.A1 = g.mu * g.ikr;
+  q.B0 = g.mu * w0;
+  q.B1 = -g.sint * g.ikr;
+  q.C2 = -g.ikr;
+  return q;
+}
+
+// M, D and their derivatives at a node, times 1/noise: pair j in out[2 j
+// stride], out[(2 j + 1) stride].  The order sums of the value, of one
+// tangent along z_p and of the a_p and n_p derivatives; the empty asm
+// statements keep the compiler from mixing their terms, which would spill
+// (the kernel has 128 registers a thread).
+template <bool kKP>
+__device__ __noinline__ void fitr_node(double k, double rho, double zp, bool bohren,
+                                       double aberr, double inv_noise, const FitrOrder* rec,
+                                       int nm, double* out, int stride) {
+  const Geometry<double> g = geometry<double>(k, rho, 0., -zp, 0., zp, bohren);
+  const double ikr = g.ikr, mu = g.mu, st = g.sint;
+  // d kr / dz_p = k mu, d mu / dz_p = k st^2 / kr
+  const double krz = k * mu, muz = k * st * st * ikr;
+  const zd zero = mk(0., 0.);
+  zd sv[3] = {zero, zero, zero}, sd[3] = {zero, zero, zero};
+  zd sa[3] = {zero, zero, zero}, sn[3] = {zero, zero, zero};
+  {
+    double pim1 = 0., pi = 1., del = 1., dpim1 = 0., dpi = 0., ddel = 0.;
+    zd h2 = g.hm1, h1 = g.h0, hp2 = zero, hp1 = zero;
+    const double s = g.s1mu, ik = g.ikrs, ik2 = g.ikrs * ikr * krz;
+    const double sz = -g.smu * muz;  // of s = 1 - |mu|
+#pragma unroll 1
+    for (int n = 1; n <= nm; ++n) {
+      const FitrOrder& r = rec[n];
+      const double spi = s * pi;
+      const double tau = pim1 + r.fn * (spi - del);
+      const double dspi = sz * pi + s * dpi;
+      const double dtau = dpim1 + r.fn * (dspi - ddel);
+      const double a2 = r.tn1 * ik, a1 = r.fn * ik;
+      const zd h = mk(a2 * h1.re - h2.re, a2 * h1.im - h2.im);
+      const zd dh = mk(a1 * h.re - h1.re, a1 * h.im - h1.im);
+      {
+        const zd X = r.v[0] * dh, Y = r.v[1] * h, Z = r.z[0] * h;
+        sv[0] = sv[0] + pi * Z;
+        sv[1] = sv[1] + tau * X - pi * Y;
+        sv[2] = sv[2] + pi * X - tau * Y;
+        sd[0] = sd[0] + dpi * Z;
+        sd[1] = sd[1] + dtau * X - dpi * Y;
+        sd[2] = sd[2] + dpi * X - dtau * Y;
+      }
+      asm volatile("" ::: "memory");
+      {
+        const zd X = r.v[2] * dh, Y = r.v[3] * h, Z = r.z[1] * h;
+        sa[0] = sa[0] + pi * Z;
+        sa[1] = sa[1] + tau * X - pi * Y;
+        sa[2] = sa[2] + pi * X - tau * Y;
+      }
+      asm volatile("" ::: "memory");
+      {
+        const zd X = r.v[4] * dh, Y = r.v[5] * h, Z = r.z[2] * h;
+        sn[0] = sn[0] + pi * Z;
+        sn[1] = sn[1] + tau * X - pi * Y;
+        sn[2] = sn[2] + pi * X - tau * Y;
+      }
+      asm volatile("" ::: "memory");
+      const double b2 = r.tn1 * ik2, b1 = r.fn * ik2;
+      const zd hp = mk(a2 * hp1.re - b2 * h1.re - hp2.re, a2 * hp1.im - b2 * h1.im - hp2.im);
+      const zd dhp = mk(a1 * hp.re - b1 * h.re - hp1.re, a1 * hp.im - b1 * h.im - hp1.im);
+      {
+        const zd X = r.v[0] * dhp, Y = r.v[1] * hp, Z = r.z[0] * hp;
+        sd[0] = sd[0] + pi * Z;
+        sd[1] = sd[1] + tau * X - pi * Y;
+        sd[2] = sd[2] + pi * X - tau * Y;
+      }
+      // Delta_{n+1} = c_n (Delta_n - s pi_n) - s pi_n
+      del = r.cn * (del - spi) - spi;
+      ddel = r.cn * (ddel - dspi) - dspi;
+      pim1 = pi;
+      pi = pi + del;
+      dpim1 = dpi;
+      dpi = dpi + ddel;
+      h2 = h1;
+      h1 = h;
+      hp2 = hp1;
+      hp1 = hp;
+    }
+  }
+  // undo the parity folding (order_sum_jac); the z tangent of pi~, tau~ and
+  // h~ was carried through s and kr, so component 2 takes the same sign
+  sv[2] = g.smu * sv[2];
+  sd[2] = g.smu * sd[2];
+  sa[2] = g.smu * sa[2];
+  sn[2] = g.smu * sn[2];
+  double rate = (g.sigma != 0. && g.sigma == g.smu) ? -g.s1mu : g.sigma * mu - 1.;
+  rate *= k;
+  zd ph = g.phase;
+  if (aberr != 0.) {
+    double d[3];
+    ph = ph * conj(aberration_wave<double>(aberr, rho, 0., zp, d));
+    rate += d[2];
+  }
+  const FitrProjection q = fitr_projection(g);
+  const double ir2 = 0.5 / (rho * rho);
+  auto put = [&](int pair, double P, double Q) {
+    out[2 * pair * stride] = 0.5 * (P + Q) * inv_noise;
+    out[(2 * pair + 1) * stride] = ir2 * (P - Q) * inv_noise;
+  };
+  const zd x1 = ph * (q.A0 * sv[0] + q.A1 * sv[1]);
+  const zd z1 = ph * (q.B0 * sv[0] + q.B1 * sv[1]);
+  const zd x2 = ph * (q.C2 * sv[2]);
+  put(0, norm2(x1) + norm2(z1) + 2. * x1.re, norm2(x2) + 2. * x2.re);
+  out[0] += inv_noise;  // the reference wave's 1
+  const zd w1 = mk(x1.re + 1., x1.im), w2 = mk(x2.re + 1., x2.im);
+  auto slope = [&](zd d1, zd dz, zd d2, int pair) {
+    put(pair, 2. * (w1.re * d1.re + w1.im * d1.im + z1.re * dz.re + z1.im * dz.im),
+        2. * (w2.re * d2.re + w2.im * d2.im));
+  };
+  {
+    const double w0 = st * ikr * ikr;
+    const double stz = -k * st * mu * ikr, ikz = -ikr * ikr * krz;
+    const double w0z = stz * ikr * ikr + 2. * st * ikr * ikz;
+    const double A0z = stz * w0 + st * w0z, A1z = muz * ikr + mu * ikz;
+    const double B0z = muz * w0 + mu * w0z, B1z = -stz * ikr - st * ikz, C2z = -ikz;
+    const zd d1 =
+        ph * (A0z * sv[0] + A1z * sv[1] + q.A0 * sd[0] + q.A1 * sd[1]) + rate * mul_i(x1);
+    const zd dz =
+        ph * (B0z * sv[0] + B1z * sv[1] + q.B0 * sd[0] + q.B1 * sd[1]) + rate * mul_i(z1);
+    const zd d2 = ph * (C2z * sv[2] + q.C2 * sd[2]) + rate * mul_i(x2);
+    slope(d1, dz, d2, 1);
+  }
+  slope(ph * (q.A0 * sa[0] + q.A1 * sa[1]), ph * (q.B0 * sa[0] + q.B1 * sa[1]),
+        ph * (q.C2 * sa[2]), 2);
+  const zd n1 = ph * (q.A0 * sn[0] + q.A1 * sn[1]), nz = ph * (q.B0 * sn[0] + q.B1 * sn[1]),
+           n2 = ph * (q.C2 * sn[2]);
+  slope(n1, nz, n2, 3);
+  // a_n, b_n are holomorphic in the index: d/dk_p = i d/dn_p
+  if (kKP) slope(mul_i(n1), mul_i(nz), mul_i(n2), 4);
+}
+
+// A pair of functions and their slopes at t: v = (M, D), d = dv/dt.
+__device__ inline void fitr_pair_slope(const float4* r, float t, f2& v, f2& d) {
+  const float4 a = r[0], b = r[1], c = r[2];
+  const f2 tt = pk(t, t);
+  d = pk(c.z, c.w);
+  v = pfma(d, tt, pk(c.x, c.y));
+  d = pfma(d, tt, v);
+  v = pfma(v, tt, pk(b.z, b.w));
+  d = pfma(d, tt, v);
+  v = pfma(v, tt, pk(b.x, b.y));
+  d = pfma(d, tt, v);
+  v = pfma(v, tt, pk(a.z, a.w));
+  d = pfma(d, tt, v);
+  v = pfma(v, tt, pk(a.x, a.y));
+}
+__device__ inline f2 fitr_pair(const float4* r, float t) {
+  const float4 a = r[0], b = r[1], c = r[2];
+  const f2 tt = pk(t, t);
+  f2 v = pfma(pk(c.z, c.w), tt, pk(c.x, c.y));
+  v = pfma(v, tt, pk(b.z, b.w));
+  v = pfma(v, tt, pk(b.x, b.y));
+  v = pfma(v, tt, pk(a.z, a.w));
+  return pfma(v, tt, pk(a.x, a.y));
+}
+
+// The sums of one pixel: f^2, J^T J (packed upper over the six slots) and
+// J^T f, k_p's only with kKP.
+template <bool kKP>
+__device__ inline void fitr_add(float r, const float* J, float* acc) {
+  constexpr int N = kKP ? 6 : 5;
+  acc[0] = fmaf(r, r, acc[0]);
+#pragma unroll
+  for (int a = 0; a < N; ++a) {
+#pragma unroll
+    for (int b = a; b < N; ++b) {
+      const int o = 1 + a * 6 - a * (a - 1) / 2 + (b - a);
+      acc[o] = fmaf(J[a], J[b], acc[o]);
+    }
+    acc[22 + a] = fmaf(J[a], r, acc[22 + a]);
+  }
+}
+
+// One pixel from the table; d: its measured value.
+template <bool kKP>
+__device__ inline void fitr_pixel(const float4* tab, float r0, float corr, float inv_rho,
+                                  float x, float y, float inv_spacing, float spacing, float inv_half, int lo,
+                                  int n, float d, float inv_noise, float* acc) {
+  const int i = min(max(__float2int_rn(r0 * inv_spacing) - lo, 0), n - 1);
+  const float t = ((r0 - float(i + lo) * spacing) + corr) * inv_half;
+  const float4* rec = tab + i * fitr_rec(kKP);
+  f2 v, s;
+  fitr_pair_slope(rec, t, v, s);
+  const float u = (x - y) * (x + y);
+  const float r = fmaf(-d, inv_noise, fmaf(v.y, u, v.x));
+  // dH/dx = cos(phi) B + 2 D x, B = M' + D' (x^2 - y^2)
+  const float B = fmaf(s.y, u, s.x) * (inv_half * inv_rho);
+  float J[6];
+  J[0] = -x * fmaf(2.f, v.y, B);
+  J[1] = -y * fmaf(-2.f, v.y, B);
+#pragma unroll
+  for (int j = 0; j < (kKP ? 4 : 3); ++j) {
+    const f2 w = fitr_pair(rec + 3 * (j + 1), t);
+    J[2 + j] = fmaf(w.y, u, w.x);
+  }
+  fitr_add<kKP>(r, J, acc);
+}
+
+// Sum of acc over the block into out[0..FIT_NSUM) (doubles), fixed order.
+// Each warp halves the values it holds at every step of the butterfly, so
+// that 28 sums take 31 shuffles instead of 140.
+__device__ inline void fitr_reduce(float* acc, float (*red)[32], double* out) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float v[32];
+#pragma unroll
+  for (int j = 0; j < 32; ++j) v[j] = j < FIT_NSUM ? acc[j] : 0.f;
+#pragma unroll
+  for (int w = 16; w > 0; w >>= 1) {
+    const bool up = lane & w;
+#pragma unroll
+    for (int j = 0; j < w; ++j) {
+      const float send = up ? v[j] : v[j + w];
+      const float keep = up ? v[j + w] : v[j];
+      v[j] = keep + __shfl_xor_sync(0xffffffffu, send, w);
+    }
+  }
+  // lane l now holds the warp's sum of value l
+  red[warp][lane] = v[0];
+  __syncthreads();
+  if (threadIdx.x < FIT_NSUM) {
+    float s = 0.f;
+    for (int w = 0; w < FITR_TPB / 32; ++w) s += red[w][threadIdx.x];
+    out[threadIdx.x] = s;
+  }
+  __syncthreads();
+}
+
+// The orders summed at every pixel of tiles [t0, t1), for the parts where
+// the tables do not apply (a plane that cuts or almost touches the sphere).
+__device__ __noinline__ void fitr_direct(const FitCtx& c, int f, const lmb_feature& ft,
+                                         const double* p, int nm, int t0, int t1, int band,
+                                         Quad<float>* coef, float (*red)[32]) {
+  const int nmaxp = c.nmax_cap + 1;
+  stage_coef<float, true>(c.ab + size_t(f) * nmaxp * 2, c.dab + size_t(f) * nmaxp * 4, nm,
+                          coef);
+  __syncthreads();
+  const float inv_noise = float(c.inv_noise);
+  for (int t = t0; t < t1; ++t) {
+    long long a = (long long)t * FITR_TILE, b = a + FITR_TILE;
+    if (ft.nx > 0) {
+      a = (long long)t * band * ft.nx;
+      b = a + (long long)band * ft.nx;
+    }
+    if (b > ft.npix) b = ft.npix;
+    float acc[FIT_NSUM];
+#pragma unroll
+    for (int j = 0; j < FIT_NSUM; ++j) acc[j] = 0.f;
+    for (long long i = a + threadIdx.x; i < b; i += FITR_TPB) {
+      double x, y;
+      fit_pixel_xy(ft, c.coords, i, &x, &y);
+      const double dx = x - p[0], dy = y - p[1];
+      const Geometry<float> g =
+          geometry<float>(c.k, dx, dy, -p[2], 0., p[2], c.flags & LMB_BOHREN);
+      float H, dH[6];
+      if (c.aberr != 0.)
+        holo_jac_pixel<true>(g, coef, nm, float(c.k), &H, dH, c.aberr, dx, dy, p[2]);
+      else
+        holo_jac_pixel<false>(g, coef, nm, float(c.k), &H, dH);
+      const float r = (H - c.data[ft.data_offset + i]) * inv_noise;
+      for (int j = 0; j < 6; ++j) dH[j] *= inv_noise;
+      fitr_add<true>(r, dH, acc);
+    }
+    fitr_reduce(acc, red, c.partial + (size_t)(c.tile_begin[f] + t) * FIT_NSUM);
+  }
+}
+
+// Persistent CTAs pull (feature, part) items: c.parts parts a feature, each
+// a run of its tiles.  A CTA builds the table of its part in shared memory
+// (FP64 nodes, then the polynomials) and evaluates its pixels
+// from it.  A tile's sums do not depend on how the tiles are dealt out.
+// cap: intervals that the table has room for.  Bound by shared-memory
+// bandwidth (12 LDS.128 a pixel) and issue.
+template <bool kKP>
+__global__ void __launch_bounds__(FITR_TPB, 2)
+k_fit_eval_radial(FitCtx c, RadialMatrix A, int cap) {
+  extern __shared__ __align__(16) char smem[];
+  __shared__ float red[FITR_TPB / 32][32];
+  __shared__ FitrPlan s_pl;
+  __shared__ float s_rho[2][FITR_TPB / 32];
+  __shared__ int s_item;
+  constexpr int REC = fitr_rec(kKP), NF = fitr_funcs(kKP);
+  const int nmaxp = c.nmax_cap + 1;
+  float4* tab = reinterpret_cast<float4*>(smem);                       // [cap][REC]
+  double* val = reinterpret_cast<double*>(tab + size_t(cap) * REC);    // [NF][cap + 16]
+  const int vstride = cap + 2 * RADIAL_SIDE;
+  FitrOrder* ord = reinterpret_cast<FitrOrder*>(val + size_t(NF) * vstride);
+  // the direct sums' FP32 records, in the tables' place
+  Quad<float>* direct = reinterpret_cast<Quad<float>*>(smem);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float inv_noise = float(c.inv_noise);
+  for (int n = threadIdx.x; n < nmaxp; n += FITR_TPB) {
+    const double fn = double(n);
+    ord[n].fn = fn;
+    ord[n].tn1 = 2. * fn - 1.;
+    ord[n].cn = n ? 1. + 1. / fn : 0.;
+    ord[n].en = n ? (2. * fn + 1.) / (fn * (fn + 1.)) : 0.;
+  }
+  for (;;) {
+    if (threadIdx.x == 0) s_item = atomicAdd(c.counters, 1);
+    __syncthreads();
+    const int q = s_item;
+    if (q >= c.counters[5]) break;
+    const int item = c.active_tiles[q];
+    const int f = item / c.parts, part = item - f * c.parts;
+    const int nt = c.tile_begin[f + 1] - c.tile_begin[f];
+    const int t0 = int((long long)nt * part / c.parts);
+    const int t1 = int((long long)nt * (part + 1) / c.parts);
+    if (t0 == t1) {
+      __syncthreads();  // s_item is rewritten
+      continue;
+    }
+    const lmb_feature ft = c.features[f];
+    const EvalPoint ep = c.ev[f];
+    const int nm = min(max(c.nmax[f], 0), nmaxp - 1);
+    const int band = ft.nx > 0 ? fitr_band(ft.nx) : 0;
+    const long long i0 = (long long)t0 * FITR_TILE;
+    const long long i1 = min((long long)t1 * FITR_TILE, ft.npix);
+    // ---- the distances of the part's pixels
+    if (ft.nx == 0) {
+      float lo = 3e38f, hi = 0.f;
+      for (long long i = i0 + threadIdx.x; i < i1; i += FITR_TPB) {
+        const float2 xy = reinterpret_cast<const float2*>(c.coords)[ft.data_offset + i];
+        const float dx = xy.x - float(ep.p[0]), dy = xy.y - float(ep.p[1]);
+        const float r = sqrtf(dx * dx + dy * dy);
+        lo = fminf(lo, r);
+        hi = r <= hi ? hi : r;  // NaN passes on to hi
+      }
+      for (int o = 16; o > 0; o >>= 1) {
+        lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        const float h = __shfl_xor_sync(0xffffffffu, hi, o);
+        hi = h <= hi ? hi : h;
+      }
+      if (lane == 0) {
+        s_rho[0][warp] = lo;
+        s_rho[1][warp] = hi;
+      }
+      __syncthreads();
+    }
+    // ---- the plan (warp 0), and the order records meanwhile
+    for (int n = int(threadIdx.x) - 32; n <= nm && n >= 0; n += FITR_TPB - 32) {
+      const zd* ab = c.ab + (size_t(f) * nmaxp + n) * 2;
+      const zd* dab = c.dab + (size_t(f) * nmaxp + n) * 4;
+      const double en = ord[n].en;
+      for (int j = 0; j < 3; ++j) {
+        const zd* s = j == 0 ? ab : dab + 2 * (j - 1);
+        ord[n].v[2 * j] = en * rot_i(s[0], n + 1);
+        ord[n].z[j] = (2. * double(n) + 1.) * rot_i(s[0], n + 1);
+        ord[n].v[2 * j + 1] = en * rot_i(s[1], n);
+      }
+    }
+    if (threadIdx.x == 0) {
+      FitrPlan pl;
+      const float zp = float(fabs(ep.p[2])), k = float(c.k);
+      const double ox = (ft.nx > 0 ? ft.x0 : 0.) - ep.p[0];
+      const double oy = (ft.nx > 0 ? ft.y0 : 0.) - ep.p[1];
+      // nearest and farthest distances; FP32, as the intervals have margins
+      float lo, hi;
+      if (ft.nx > 0) {
+        const float x0 = float(ox), x1 = x0 + float(ft.nx - 1);
+        const float y0 = float(oy) + float(t0 * band);
+        const float y1 =
+            float(oy) + float(min((long long)t1 * band, (long long)ft.ny) - 1);
+        const float nx = x0 > 0.f ? x0 : (x1 < 0.f ? -x1 : 0.f);
+        const float ny = y0 > 0.f ? y0 : (y1 < 0.f ? -y1 : 0.f);
+        const float fx = fmaxf(fabsf(x0), fabsf(x1)), fy = fmaxf(fabsf(y0), fabsf(y1));
+        lo = sqrtf(nx * nx + ny * ny);
+        hi = sqrtf(fx * fx + fy * fy);
+      } else {
+        lo = s_rho[0][0];
+        hi = s_rho[1][0];
+        for (int w = 1; w < FITR_TPB / 32; ++w) {
+          lo = fminf(lo, s_rho[0][w]);
+          hi = s_rho[1][w] <= hi ? hi : s_rho[1][w];
+        }
+      }
+      const double x = c.size_per_um * ep.p[3];  // size parameter
+      float rate = fitr_rate(k, float(x) / k, zp, hi);
+      bool ok = c.k * fabs(ep.p[2]) - x >= RADIAL_CLEARANCE && hi < 8000.f && zp < 1e6f &&
+                isfinite(ep.p[0]) && isfinite(ep.p[1]);
+      if (c.aberr != 0.) {  // the aberration's phase, as lmb_radial_intervals
+        const float turn = 0.5f * fabsf(float(c.aberr)) / zp;
+        ok = ok && turn <= 0.2f * k;
+        rate = fminf(2.f, rate + turn / k);
+      }
+      // a multiple of 1/64 px, so that i * spacing is exact in FP32
+      const float sp = fminf(8.f, floorf(64.f * float(FITR_SPACING) / (k * rate)) * 0.015625f);
+      ok = ok && sp >= 0.0625f;
+      pl.spacing = double(sp);
+      pl.lo = pl.n = 0;
+      if (ok) {
+        const float is = 1.f / sp;
+        pl.lo = max(0, int(lo * is) - 1);
+        pl.n = int(hi * is) + 3 - pl.lo;
+        ok = pl.n <= cap;
+      }
+      const double ax = rint(ox * 1024.) * (1. / 1024.), ay = rint(oy * 1024.) * (1. / 1024.);
+      pl.ax = float(ax);
+      pl.rx = float(ox - ax);
+      pl.ay = float(ay);
+      pl.ry = float(oy - ay);
+      pl.radial = ok;
+      s_pl = pl;
+    }
+    __syncthreads();
+    const FitrPlan pl = s_pl;
+    if (threadIdx.x == 0) {
+      const long long np = ft.nx > 0
+          ? (min((long long)t1 * band, (long long)ft.ny) - (long long)t0 * band) * ft.nx
+          : i1 - i0;
+      atomicAdd(c.work, (unsigned long long)np);
+      atomicAdd(c.work + 1, (unsigned long long)nm *
+                                (unsigned long long)(pl.radial ? pl.n + 2 * RADIAL_SIDE : np));
+    }
+    if (!pl.radial) {
+      fitr_direct(c, f, ft, ep.p, nm, t0, t1, band, direct, red);
+      continue;  // its last barrier follows every read of s_item and s_pl
+    }
+    // ---- nodes, polynomials
+    for (int t = threadIdx.x; t < pl.n + 2 * RADIAL_SIDE; t += FITR_TPB) {
+      const int j = abs(pl.lo - RADIAL_SIDE + t);
+      fitr_node<kKP>(c.k, j ? pl.spacing * double(j) : RADIAL_AXIS, ep.p[2],
+                     c.flags & LMB_BOHREN, c.aberr, c.inv_noise, ord, nm, val + t, vstride);
+    }
+    __syncthreads();
+    for (int w = threadIdx.x; w < pl.n * (NF / 2); w += FITR_TPB) {
+      const int g = w / pl.n, i = w - g * pl.n;
+      const double* s = val + 2 * g * vstride + i;
+      double cr[RADIAL_COEFS], ci[RADIAL_COEFS];
+#pragma unroll
+      for (int j = 0; j < RADIAL_COEFS; ++j) cr[j] = ci[j] = 0.;
+#pragma unroll
+      for (int l = 0; l < RADIAL_TAPS; ++l) {
+        const double x = s[l], y = s[vstride + l];
+#pragma unroll
+        for (int j = 0; j < RADIAL_COEFS; ++j) {
+          cr[j] = fma(A.m[j][l], x, cr[j]);
+          ci[j] = fma(A.m[j][l], y, ci[j]);
+        }
+      }
+      float4* o = tab + size_t(i) * REC + 3 * g;
+#pragma unroll
+      for (int j = 0; j < RADIAL_COEFS; j += 2)
+        o[j / 2] = make_float4(float(cr[j]), float(ci[j]), float(cr[j + 1]), float(ci[j + 1]));
+    }
+    __syncthreads();
+    // ---- pixels
+    const float spacing = float(pl.spacing), inv_spacing = float(1. / pl.spacing);
+    const float inv_half = float(2. / pl.spacing);
+    for (int t = t0; t < t1; ++t) {
+      float acc[FIT_NSUM];
+#pragma unroll
+      for (int j = 0; j < FIT_NSUM; ++j) acc[j] = 0.f;
+      if (ft.nx > 0) {
+        // 8x8 pixels per warp, two per lane (rows y and y + 4): eight lanes
+        // on 4x2 pixels read intervals in different banks
+        const int row0 = t * band, rows = min(band, ft.ny - row0);
+        const int pc = (ft.nx + 7) / 8, np = pc * ((rows + 7) / 8);
+        const int lx = 4 * ((lane >> 3) & 1) + (lane & 3);
+        const int ly = 2 * (lane >> 4) + ((lane >> 2) & 1);
+        for (int w = warp; w < np; w += FITR_TPB / 32) {
+          const int pr = w / pc, col = 8 * (w - pr * pc) + lx, row = row0 + 8 * pr + ly;
+          if (col >= ft.nx || row >= row0 + rows) continue;
+          const bool two = row + 4 < row0 + rows;
+          const float* dp = c.data + ft.data_offset + (long long)row * ft.nx + col;
+          const float d0 = dp[0], d1 = two ? dp[4LL * ft.nx] : 0.f;
+          const float X = pl.ax + float(col);
+          const f2 Y = pk(pl.ay + float(row), pl.ay + float(row + 4));
+          const float px = X * X;
+          const float lx2 = fmaf(2.f * pl.rx, fmaf(0.5f, pl.rx, X), fmaf(X, X, -px));
+          const f2 qy = pmul(Y, Y), ry = pk(pl.ry, pl.ry);
+          const f2 ly2 = pfma(padd(ry, ry), pfma(pk(0.5f, 0.5f), ry, Y), pfma(Y, Y, pneg(qy)));
+          const RadialDistance d = radial_distance(pk(px, px), pk(lx2, lx2), qy, ly2);
+          const float xr = X + pl.rx;
+          const f2 yr = padd(Y, ry);
+          fitr_pixel<kKP>(tab, d.r0.x, d.corr.x, d.y.x, xr, yr.x, inv_spacing, spacing, inv_half,
+                          pl.lo, pl.n, d0, inv_noise, acc);
+          if (two)
+            fitr_pixel<kKP>(tab, d.r0.y, d.corr.y, d.y.y, xr, yr.y, inv_spacing, spacing, inv_half,
+                            pl.lo, pl.n, d1, inv_noise, acc);
+        }
+      } else {
+        const long long a = (long long)t * FITR_TILE, b = min(a + FITR_TILE, ft.npix);
+        for (long long i = a + threadIdx.x; i < b; i += FITR_TPB) {
+          const float2 xy = reinterpret_cast<const float2*>(c.coords)[ft.data_offset + i];
+          const double dx = double(xy.x) - ep.p[0], dy = double(xy.y) - ep.p[1];
+          const double ax = rint(dx * 1024.) * (1. / 1024.);
+          const double ay = rint(dy * 1024.) * (1. / 1024.);
+          const f2 X = pk(float(ax), float(ay)), rx = pk(float(dx - ax), float(dy - ay));
+          const f2 px = pmul(X, X);
+          const f2 lx = pfma(padd(rx, rx), pfma(pk(0.5f, 0.5f), rx, X), pfma(X, X, pneg(px)));
+          const f2 xr = padd(X, rx);
+          const RadialDistance d = radial_distance(pk(px.x, px.x), pk(lx.x, lx.x),
+                                                   pk(px.y, px.y), pk(lx.y, lx.y));
+          fitr_pixel<kKP>(tab, d.r0.x, d.corr.x, d.y.x, xr.x, xr.y, inv_spacing, spacing, inv_half,
+                          pl.lo, pl.n, c.data[ft.data_offset + i], inv_noise, acc);
+        }
+      }
+      fitr_reduce(acc, red, c.partial + (size_t)(c.tile_begin[f] + t) * FIT_NSUM);
+    }
+  }
+}
+
+}  // namespace lmb

@@ -1094,10 +1094,15 @@ struct FitCtx {
   const double* layer_frac;   // [nf][nlayers-1] inner radii / outer radius
   const double* layer_index;  // [nf][nlayers-1][2] inner layer indices
   double n_m, wavelength, k, inv_noise;
+  double size_per_um;  // 2 pi n_m / wavelength: size parameter per um of radius
   double aberr;  // spherical-aberration coefficient c (0: ideal optics)
   LMSettings set;
   int variables, flags, max_iterations;
   int pair_records;    // the evaluation kernel reads stage_pair records
+  // > 0: the evaluation reads radial tables (lmb_fit_radial.cuh), a feature's
+  // tiles dealt out in this many parts; active_tiles then holds feature *
+  // parts + part, and no FP32 records are staged
+  int parts;
   // Streamed admission: features [0, *ready) have their data on the
   // device; the rest wait in LM_PHASE_INIT (counted in counters[4]).  A
   // negative value withdraws the batch.  Null: every feature is ready.
@@ -1109,6 +1114,23 @@ __device__ inline bool feature_valid(const lmb_feature& ft, long long total) {
          (ft.nx == 0 || (ft.nx > 0 && ft.ny > 0 && (long long)ft.nx * ft.ny == ft.npix));
 }
 
+// Tiles of the evaluation from radial tables: bands of rows of a grid
+// feature, a multiple of 8 rows (warps take 8x8 pixels) and FITR_TILE pixels
+// or more, or FITR_TILE pixels of an explicit list.
+enum { FITR_TILE = 2048 };
+__host__ __device__ inline int fitr_band(int nx) {
+  const int r = int((FITR_TILE + 8LL * nx - 1) / (8LL * nx));
+  return 8 * (r > 1 ? r : 1);
+}
+
+__device__ inline int fit_tile_count(const FitCtx& c, const lmb_feature& ft) {
+  if (!feature_valid(ft, c.total_pixels) || ft.npix <= 0) return 0;
+  if (!c.parts) return int((ft.npix + c.tile_pixels - 1) / c.tile_pixels);
+  if (ft.nx == 0) return int((ft.npix + FITR_TILE - 1) / FITR_TILE);
+  const int band = fitr_band(ft.nx);
+  return (ft.ny + band - 1) / band;
+}
+
 // Tile table and state initialisation; one block.
 __global__ void k_fit_setup(FitCtx c) {
   __shared__ int carry;
@@ -1117,11 +1139,7 @@ __global__ void k_fit_setup(FitCtx c) {
   for (int base = 0; base < c.nf; base += blockDim.x) {
     const int f = base + threadIdx.x;
     int nt = 0;
-    if (f < c.nf) {
-      const lmb_feature ft = c.features[f];
-      if (feature_valid(ft, c.total_pixels))
-        nt = ft.npix > 0 ? int((ft.npix + c.tile_pixels - 1) / c.tile_pixels) : 0;
-    }
+    if (f < c.nf) nt = fit_tile_count(c, c.features[f]);
     // inclusive scan of nt across the block (Hillis-Steele in shared memory)
     __shared__ int sc[1024];
     sc[threadIdx.x] = nt;
@@ -1617,7 +1635,7 @@ k_fit_step(FitCtx c) {
   // stage the records together
   if (threadIdx.x == 0) s_st = st;
   __syncthreads();
-  if (s_st == LMB_OK) {
+  if (s_st == LMB_OK && !c.parts) {
     const zd* abf = c.ab + size_t(f) * nmaxp * 2;
     const zd* dabf = c.dab + size_t(f) * nmaxp * 4;
     const int nm = min(c.nmax[f], nmaxp - 1);
@@ -1629,7 +1647,8 @@ k_fit_step(FitCtx c) {
   }
   if (warp != 0) return;
   int base = -1;
-  const int tb = c.tile_begin[f], nt = c.tile_begin[f + 1] - tb;
+  const int tb = c.parts ? f * c.parts : c.tile_begin[f];
+  const int nt = c.parts ? c.parts : c.tile_begin[f + 1] - tb;
   if (lane == 0) {
     if (st != LMB_OK) {
       gs->phase = LM_PHASE_DONE;

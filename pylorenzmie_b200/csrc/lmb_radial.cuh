@@ -146,9 +146,9 @@ LMB_HD void radial_field(double k, double rho, double dzc, double z, double zp,
 // to 2^-10 px (exact in FP32 up to 8192 px), (a, b) the remainders; lx =
 // X^2's rounding error plus 2 a X + a^2, ly alike.  rho = r0 + corr with an
 // error of ~1e-7 of corr, i.e. far below the FP32 rounding of rho, which at
-// 1500 px would turn the phase by 1e-4 rad.
+// 1500 px would turn the phase by 1e-4 rad; y is 1 / rho to a few ulp.
 struct RadialDistance {
-  f2 r0, corr;
+  f2 r0, corr, y;
 };
 
 LMB_HD f2 pneg(f2 a) { return pk(-a.x, -a.y); }
@@ -163,6 +163,7 @@ LMB_HD RadialDistance radial_distance(f2 px, f2 lx, f2 qy, f2 ly) {
   const f2 sl = padd(psub(s, sh), low);
   const f2 y = pk(rsqrt_seed(fmaxf(sh.x, 1e-24f)), rsqrt_seed(fmaxf(sh.y, 1e-24f)));
   RadialDistance d;
+  d.y = y;
   d.r0 = pmul(sh, y);
   const f2 e = padd(pfma(pneg(d.r0), d.r0, sh), sl);
   d.corr = pmul(pmul(pk(0.5f, 0.5f), y), e);
