@@ -746,6 +746,7 @@ int fit_batch_impl(const lmb_feature* features, int nfeatures,
   auto eval_radial = free_kp ? k_fit_eval_radial<true> : k_fit_eval_radial<false>;
   RadialMatrix rm = {};
   c.parts = 0;
+  c.tiles_slot = 5;
   if (radial) {
     // Parts per feature: enough to give every SM two blocks, while a part
     // more costs its feature's nodes once more.
@@ -791,20 +792,18 @@ int fit_batch_impl(const lmb_feature* features, int nfeatures,
            cudaStreamSynchronize(st) == cudaSuccess;
   };
   auto launch_eval = [&]() -> bool {
-    if (cudaMemsetAsync(c.counters + 0, 0, sizeof(int), st) != cudaSuccess) return false;
     if (stats && mark() != cudaSuccess) return false;
     if (radial)
       eval_radial<<<egrid, shape.tpb, eval_smem, st>>>(c, rm, rl.cap);
     else
       eval<<<egrid, shape.tpb, eval_smem, st>>>(c);
     if (stats && mark() != cudaSuccess) return false;
+    c.tiles_slot = 11 - c.tiles_slot;  // the next step fills the other count
     launches += 1;
     ++evals;
     return true;
   };
   auto launch_step = [&]() {
-    cudaMemsetAsync(c.counters + 1, 0, sizeof(int), st);
-    cudaMemsetAsync(c.counters + 4, 0, 2 * sizeof(int), st);  // [4], [5]
     k_fit_step<<<nfeatures, 64, ab_smem, st>>>(c);
     launches += 1;
     ++iterations;
@@ -910,6 +909,11 @@ int fit_batch_impl(const lmb_feature* features, int nfeatures,
                 std::chrono::steady_clock::now() - wait_start).count();
             if (waited > wait_seconds) { status = LMB_ERR_TIMEOUT; break; }
             std::this_thread::sleep_for(std::chrono::microseconds(20));
+            // no evaluation before this step: the count of waiting features
+            if (cudaMemsetAsync(c.counters + 4, 0, sizeof(int), st) != cudaSuccess) {
+              status = LMB_ERR_CUDA;
+              break;
+            }
           }
           launch_step();
         }

@@ -367,6 +367,8 @@ k_fit_eval_radial(FitCtx c, RadialMatrix A, int cap) {
   Quad<float>* direct = reinterpret_cast<Quad<float>*>(smem);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const float inv_noise = float(c.inv_noise);
+  const int ntiles = c.counters[c.tiles_slot];  // (feature, part) items
+  fit_eval_begin(c);
   for (int n = threadIdx.x; n < nmaxp; n += FITR_TPB) {
     const double fn = double(n);
     ord[n].fn = fn;
@@ -378,7 +380,7 @@ k_fit_eval_radial(FitCtx c, RadialMatrix A, int cap) {
     if (threadIdx.x == 0) s_item = atomicAdd(c.counters, 1);
     __syncthreads();
     const int q = s_item;
-    if (q >= c.counters[5]) break;
+    if (q >= ntiles) break;
     const int item = c.active_tiles[q];
     const int f = item / c.parts, part = item - f * c.parts;
     const int nt = c.tile_begin[f + 1] - c.tile_begin[f];

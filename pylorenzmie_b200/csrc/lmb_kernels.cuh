@@ -1084,7 +1084,9 @@ struct FitCtx {
   int2* tiles;         // [max_tiles]
   double* partial;     // [max_tiles][FIT_NSUM]
   int* counters;       // [0] tile queue, [1] running, [2] ntiles, [3] overflow,
-                       // [4] waiting for data, [5] active tiles this round
+                       // [4] waiting for data, [5] and [6] active tiles of
+                       // alternate rounds (tiles_slot)
+  int tiles_slot;      // 5 or 6: the round's count of active tiles
   int* active_tiles;   // [max_tiles] tiles of the features evaluated this
                        // round (filled by k_fit_step, in no fixed order)
   unsigned long long* work;  // [0] pixels, [1] pixel-orders evaluated
@@ -1163,6 +1165,7 @@ __global__ void k_fit_setup(FitCtx c) {
     c.counters[1] = 0;
     c.counters[4] = 0;
     c.counters[5] = 0;
+    c.counters[6] = 0;
     c.work[0] = 0ull;
     c.work[1] = 0ull;
   }
@@ -1201,6 +1204,18 @@ __global__ void k_fit_setup(FitCtx c) {
   }
 }
 
+// Between rounds the kernels reset the counters themselves (a memset each
+// cost ~3 us of a round): the evaluation those that the step before it
+// filled and the host has copied, and the tile count of the round before,
+// which nothing reads any more; the step the evaluation's queue.
+__device__ inline void fit_eval_begin(const FitCtx& c) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    c.counters[1] = 0;
+    c.counters[4] = 0;
+    c.counters[11 - c.tiles_slot] = 0;
+  }
+}
+
 // Evaluation: persistent CTAs pull tiles from an atomic queue.
 template <int TPB, int PPT, int MINB, bool kAberr = false>
 __global__ void __launch_bounds__(TPB, MINB)
@@ -1209,7 +1224,8 @@ k_fit_eval(FitCtx c) {
   Quad<float>* coef = reinterpret_cast<Quad<float>*>(smem);
   __shared__ float red[(TPB / 32) * FIT_NSUM];
   __shared__ int s_tile;
-  const int ntiles = c.counters[5];  // tiles of active features
+  const int ntiles = c.counters[c.tiles_slot];  // tiles of active features
+  fit_eval_begin(c);
   const int nmaxp = c.nmax_cap + 1;
   const bool bohren = c.flags & LMB_BOHREN;
   const float kf = float(c.k);
@@ -1347,7 +1363,8 @@ k_fit_eval_pair(FitCtx c) {
   float4* rec = reinterpret_cast<float4*>(smem);
   __shared__ float red[(TPB / 32) * FIT_NSUM];
   __shared__ int s_tile;
-  const int ntiles = c.counters[5];  // tiles of active features
+  const int ntiles = c.counters[c.tiles_slot];  // tiles of active features
+  fit_eval_begin(c);
   const int nmaxp = c.nmax_cap + 1;
   const bool bohren = c.flags & LMB_BOHREN;
   const float kf = float(c.k);
@@ -1437,7 +1454,8 @@ k_fit_eval_warp(FitCtx c) {
   const int nmaxp = c.nmax_cap + 1;
   Quad<float>* coef = reinterpret_cast<Quad<float>*>(smem) +
                       size_t(warp) * JAC_QUADS * nmaxp;
-  const int ntiles = c.counters[5];  // tiles of active features
+  const int ntiles = c.counters[c.tiles_slot];  // tiles of active features
+  fit_eval_begin(c);
   const bool bohren = c.flags & LMB_BOHREN;
   const float kf = float(c.k);
   const float inv_noise = float(c.inv_noise);
@@ -1602,6 +1620,7 @@ k_fit_step(FitCtx c) {
   const int f = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (f >= c.nf) return;  // the whole block
+  if (f == 0 && threadIdx.x == 0) c.counters[0] = 0;  // the evaluation's queue
   LMState* gs = c.state + f;
   int phase = LM_PHASE_DONE;
   if (warp == 0) {
@@ -1659,7 +1678,7 @@ k_fit_step(FitCtx c) {
       for (int j = 0; j < 6; ++j) c.ev[f].p[j] = s_p[j];
       c.ev[f].active = 1;
       atomicAdd(c.counters + 1, 1);
-      base = atomicAdd(c.counters + 5, nt);  // this feature's tiles join
+      base = atomicAdd(c.counters + c.tiles_slot, nt);  // this feature's tiles join
     }
   }
   base = __shfl_sync(0xffffffffu, base, 0);
