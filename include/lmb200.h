@@ -341,6 +341,24 @@ int lmb_hologram_vjp(const double *coords, long long npts,
                      void *workspace, size_t workspace_bytes, void *stream);
 
 /*
+ * lmb_hologram_vjp for pixels of one plane (grid and points as
+ * lmb_hologram_grid), from radial tables.  host_spheres: the same records in
+ * host memory, from which the tables' size follows.  The workspace function
+ * returns 0 where the tables do not apply (as lmb_radial_intervals; then
+ * lmb_hologram_vjp is to be used).
+ */
+size_t lmb_vjp_grid_workspace_bytes(const lmb_grid *grid, long long npts,
+                                    const lmb_sphere *host_spheres, int n,
+                                    double k, double magnification, int flags);
+int lmb_hologram_vjp_grid(const lmb_grid *grid, const double *points,
+                          long long npts, const lmb_sphere *host_spheres,
+                          const lmb_sphere *spheres, int n, const double *ab,
+                          const double *dab, const int *nmax, int nmax_cap,
+                          double k, double magnification, int flags,
+                          const float *gout, double *grad, void *workspace,
+                          size_t workspace_bytes, void *stream);
+
+/*
  * A feature to fit: a crop of a normalized hologram.  Pixels are either a
  * regular grid (nx > 0: pixel i sits at x = x0 + i % nx, y = y0 + i / nx,
  * npix = nx*ny, as Hologram.flat_coordinates, analysis/Hologram.py:69-77)

@@ -564,6 +564,110 @@ int lmb_hologram_vjp(const double* coords, long long npts,
   return LMB_OK;
 }
 
+// Intervals a sphere for lmb_hologram_vjp_grid, and the node spacing: that of
+// the fastest hologram (fitr_rate).
+static int grad_plan(const lmb_grid* grid, long long npts, const lmb_sphere* spheres, int n,
+                     double k, double magnification, int flags, double* spacing) {
+  if (!grid || !spheres || n < 1 || n > 65535 || grid->nx < 1 || grid->ny < 1 || npts < 1 ||
+      grid->nx > 1000000 || grid->ny > 1000000)
+    return 0;
+  if (!(flags & LMB_CARTESIAN) || (flags & LMB_FP64)) return 0;
+  if (!(k > 0.) || !isfinite(k) || !(magnification > 0.)) return 0;
+  if (!isfinite(grid->x0) || !isfinite(grid->y0) || !isfinite(grid->z)) return 0;
+  double far = 0., rate = 0.;
+  for (int i = 0; i < n; ++i) {
+    const lmb_sphere& s = spheres[i];
+    const double dx = fmax(fabs(grid->x0 - s.x_p), fabs(grid->x0 + double(grid->nx - 1) - s.x_p));
+    const double dy = fmax(fabs(grid->y0 - s.y_p), fabs(grid->y0 + double(grid->ny - 1) - s.y_p));
+    const double reach = sqrt(dx * dx + dy * dy), dz = fabs(grid->z - s.z_p);
+    if (!(reach < 8000.) || !(s.a_p > 0.) || !(dz < 1e6)) return 0;
+    if (!(k * (dz - s.a_p / magnification) >= RADIAL_CLEARANCE)) return 0;
+    far = fmax(far, reach);
+    rate = fmax(rate, double(fitr_rate(float(k), float(s.a_p / magnification), float(dz),
+                                       float(reach))));
+  }
+  // a multiple of 1/64 px, so that i * spacing is exact in FP32
+  const double sp = fmin(8., floor(64. * FITR_SPACING / (k * rate)) / 64.);
+  if (!(sp >= 1. / 16.)) return 0;
+  const int count = int(far / sp) + 2;
+  if (double(npts) < 2. * (count + 2 * RADIAL_SIDE)) return 0;  // as lmb_radial_intervals
+  *spacing = sp;
+  return count;
+}
+
+static size_t grad_node_bytes(int n, int intervals) {
+  return align_up(sizeof(double) * fitr_funcs(true) * size_t(n) *
+                      (size_t(intervals) + 2 * RADIAL_SIDE), 256);
+}
+// Blocks a sphere: two for every SM over the call, at least 2048 pixels each.
+static int grad_parts(long long npts, int n) {
+  const long long most = std::max<long long>(1, npts / FITR_TILE);
+  return int(std::max<long long>(1, std::min<long long>(most, (592 + n - 1) / n)));
+}
+
+size_t lmb_vjp_grid_workspace_bytes(const lmb_grid* grid, long long npts,
+                                    const lmb_sphere* host_spheres, int n, double k,
+                                    double magnification, int flags) {
+  double spacing;
+  const int count = grad_plan(grid, npts, host_spheres, n, k, magnification, flags, &spacing);
+  if (!count) return 0;
+  return grad_node_bytes(n, count) + sizeof(double) * 6 * size_t(n) * grad_parts(npts, n);
+}
+
+int lmb_hologram_vjp_grid(const lmb_grid* grid, const double* points, long long npts,
+                          const lmb_sphere* host_spheres, const lmb_sphere* spheres, int n,
+                          const double* ab, const double* dab, const int* nmax, int nmax_cap,
+                          double k, double magnification, int flags, const float* gout,
+                          double* grad, void* workspace, size_t workspace_bytes,
+                          void* stream) {
+  if (n < 0 || bad_cap(nmax_cap)) return LMB_ERR_ARG;
+  if (n == 0) return LMB_OK;
+  if (!host_spheres || !spheres || !ab || !dab || !nmax || !gout || !grad) return LMB_ERR_ARG;
+  GradPlan pl;
+  const int count =
+      grad_plan(grid, npts, host_spheres, n, k, magnification, flags, &pl.spacing);
+  if (!count) return LMB_ERR_UNSUPPORTED;
+  if (!points && npts != grid->nx * grid->ny) return LMB_ERR_ARG;
+  if (!workspace || workspace_bytes < lmb_vjp_grid_workspace_bytes(grid, npts, host_spheres, n,
+                                                                   k, magnification, flags))
+    return LMB_ERR_WORKSPACE;
+  pl.x0 = grid->x0;
+  pl.y0 = grid->y0;
+  pl.z = grid->z;
+  pl.k = k;
+  pl.nx = grid->nx;
+  pl.ny = grid->ny;
+  pl.npts = npts;
+  pl.points = points;
+  pl.intervals = count;
+  pl.parts = grad_parts(npts, n);
+  pl.flags = flags;
+  double* nodes = reinterpret_cast<double*>(workspace);
+  double* partial = reinterpret_cast<double*>(reinterpret_cast<char*>(workspace) +
+                                              grad_node_bytes(n, count));
+  cudaStream_t st = as_stream(stream);
+  const size_t node_smem = sizeof(FitrOrder) * (size_t(nmax_cap) + 1);
+  LMB_CK(smem_attr((const void*)k_grad_nodes, node_smem));
+  const int nn = count + 2 * RADIAL_SIDE;
+  k_grad_nodes<<<dim3((nn + FITR_NODE_TPB - 1) / FITR_NODE_TPB, n), FITR_NODE_TPB, node_smem,
+                 st>>>(pl, spheres, reinterpret_cast<const zd*>(ab),
+                       reinterpret_cast<const zd*>(dab), nmax, nmax_cap + 1, nodes);
+  LMB_CK(cudaGetLastError());
+  // two blocks an SM: ~110 KB each
+  const size_t per = sizeof(float4) * fitr_rec(true) + sizeof(double) * fitr_funcs(true);
+  const size_t fixed = sizeof(double) * fitr_funcs(true) * 2 * RADIAL_SIDE;
+  const int cap = int(std::min<size_t>(size_t(count), (size_t(108) * 1024 - fixed) / per));
+  const size_t smem = per * size_t(cap) + fixed;
+  LMB_CK(smem_attr((const void*)k_vjp_radial, smem));
+  k_vjp_radial<<<dim3(pl.parts, n), FITR_TPB, smem, st>>>(pl, radial_matrix(), cap, spheres,
+                                                          nodes, gout, partial);
+  LMB_CK(cudaGetLastError());
+  const int nt = n * 6;
+  k_vjp_reduce<<<(nt + 127) / 128, 128, 0, st>>>(partial, pl.parts, n, grad);
+  LMB_CK(cudaGetLastError());
+  return LMB_OK;
+}
+
 int lmb_fit_tile_config(int index, int* threads, int* pixels_per_thread,
                         int* min_blocks) {
   if (index < 0 || index >= kNumEvalShapes) return LMB_ERR_ARG;

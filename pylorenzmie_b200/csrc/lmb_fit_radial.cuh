@@ -39,11 +39,11 @@ __host__ __device__ constexpr int fitr_funcs(bool kp) { return 2 * (FITR_PAIRS +
 // directions under which a pixel sees the sphere, at most twice the angle of
 // its edge from its axis.  The sphere's edge is widened by 6 / k for the
 // partial waves beyond the geometric radius.
-__device__ inline float fitr_rate(float k, float a_px, float z, float rho) {
+__host__ __device__ inline float fitr_rate(float k, float a_px, float z, float rho) {
   const float a = a_px + 6.f / k;
   const float far = rho + a;
-  const float s1 = far * rsqrtf(far * far + z * z);
-  const float s2 = 2.f * a * rsqrtf(a * a + z * z);
+  const float s1 = far * rsqrt_seed(far * far + z * z);
+  const float s2 = 2.f * a * rsqrt_seed(a * a + z * z);
   return fminf(2.f, fmaxf(0.25f, fmaxf(s1, s2)));
 }
 
@@ -83,12 +83,13 @@ __device__ inline FitrProjection fitr_projection(const Geometry<double>& g) {
 // stride], out[(2 j + 1) stride].  The order sums of the value, of one
 // tangent along z_p and of the a_p and n_p derivatives; the empty asm
 // statements keep the compiler from mixing their terms, which would spill
-// (the kernel has 128 registers a thread).
+// where the kernel has 128 registers a thread.  z: the pixels' plane.
 template <bool kKP>
-__device__ __noinline__ void fitr_node(double k, double rho, double zp, bool bohren,
-                                       double aberr, double inv_noise, const FitrOrder* rec,
-                                       int nm, double* out, int stride) {
-  const Geometry<double> g = geometry<double>(k, rho, 0., -zp, 0., zp, bohren);
+__device__ __forceinline__ void fitr_node(double k, double rho, double z, double zp,
+                                          bool bohren, double aberr, double inv_noise,
+                                          const FitrOrder* rec, int nm, double* out,
+                                          int stride) {
+  const Geometry<double> g = geometry<double>(k, rho, 0., z - zp, z, zp, bohren);
   const double ikr = g.ikr, mu = g.mu, st = g.sint;
   // d kr / dz_p = k mu, d mu / dz_p = k st^2 / kr
   const double krz = k * mu, muz = k * st * st * ikr;
@@ -208,6 +209,15 @@ __device__ __noinline__ void fitr_node(double k, double rho, double zp, bool boh
   if (kKP) slope(mul_i(n1), mul_i(nz), mul_i(n2), 4);
 }
 
+// The same as a call, for the kernel whose pixel loop sets its registers.
+template <bool kKP>
+__device__ __noinline__ void fitr_node_call(double k, double rho, double zp, bool bohren,
+                                            double aberr, double inv_noise,
+                                            const FitrOrder* rec, int nm, double* out,
+                                            int stride) {
+  fitr_node<kKP>(k, rho, 0., zp, bohren, aberr, inv_noise, rec, nm, out, stride);
+}
+
 // A pair of functions and their slopes at t: v = (M, D), d = dv/dt.
 __device__ inline void fitr_pair_slope(const float4* r, float t, f2& v, f2& d) {
   const float4 a = r[0], b = r[1], c = r[2];
@@ -250,21 +260,19 @@ __device__ inline void fitr_add(float r, const float* J, float* acc) {
   }
 }
 
-// One pixel from the table; d: its measured value.
+// Hologram and derivatives of one pixel from the table, times 1/noise.
 template <bool kKP>
-__device__ inline void fitr_pixel(const float4* tab, float r0, float corr, float inv_rho,
-                                  float x, float y, float inv_spacing, float spacing, float inv_half, int lo,
-                                  int n, float d, float inv_noise, float* acc) {
+__device__ inline float fitr_lookup(const float4* tab, float r0, float corr, float inv_rho,
+                                    float x, float y, float inv_spacing, float spacing,
+                                    float inv_half, int lo, int n, float* J) {
   const int i = min(max(__float2int_rn(r0 * inv_spacing) - lo, 0), n - 1);
   const float t = ((r0 - float(i + lo) * spacing) + corr) * inv_half;
   const float4* rec = tab + i * fitr_rec(kKP);
   f2 v, s;
   fitr_pair_slope(rec, t, v, s);
   const float u = (x - y) * (x + y);
-  const float r = fmaf(-d, inv_noise, fmaf(v.y, u, v.x));
   // dH/dx = cos(phi) B + 2 D x, B = M' + D' (x^2 - y^2)
   const float B = fmaf(s.y, u, s.x) * (inv_half * inv_rho);
-  float J[6];
   J[0] = -x * fmaf(2.f, v.y, B);
   J[1] = -y * fmaf(-2.f, v.y, B);
 #pragma unroll
@@ -272,7 +280,85 @@ __device__ inline void fitr_pixel(const float4* tab, float r0, float corr, float
     const f2 w = fitr_pair(rec + 3 * (j + 1), t);
     J[2 + j] = fmaf(w.y, u, w.x);
   }
-  fitr_add<kKP>(r, J, acc);
+  return fmaf(v.y, u, v.x);
+}
+
+// The sums of one pixel; d: its measured value.
+template <bool kKP>
+__device__ inline void fitr_pixel(const float4* tab, float r0, float corr, float inv_rho,
+                                  float x, float y, float inv_spacing, float spacing,
+                                  float inv_half, int lo, int n, float d, float inv_noise,
+                                  float* acc) {
+  float J[6];
+  const float h = fitr_lookup<kKP>(tab, r0, corr, inv_rho, x, y, inv_spacing, spacing,
+                                   inv_half, lo, n, J);
+  fitr_add<kKP>(fmaf(-d, inv_noise, h), J, acc);
+}
+
+// The polynomials of intervals [0, n) from the nodes val[function][stride]
+// (the first node RADIAL_SIDE before interval 0's), by the whole block.
+template <int REC, int NF>
+__device__ inline void fitr_polynomials(const RadialMatrix& A, const double* val, int stride,
+                                        int n, float4* tab) {
+  for (int w = threadIdx.x; w < n * (NF / 2); w += FITR_TPB) {
+    const int g = w / n, i = w - g * n;
+    const double* s = val + 2 * g * stride + i;
+    double cr[RADIAL_COEFS], ci[RADIAL_COEFS];
+#pragma unroll
+    for (int j = 0; j < RADIAL_COEFS; ++j) cr[j] = ci[j] = 0.;
+#pragma unroll
+    for (int l = 0; l < RADIAL_TAPS; ++l) {
+      const double x = s[l], y = s[stride + l];
+#pragma unroll
+      for (int j = 0; j < RADIAL_COEFS; ++j) {
+        cr[j] = fma(A.m[j][l], x, cr[j]);
+        ci[j] = fma(A.m[j][l], y, ci[j]);
+      }
+    }
+    float4* o = tab + size_t(i) * REC + 3 * g;
+#pragma unroll
+    for (int j = 0; j < RADIAL_COEFS; j += 2)
+      o[j / 2] = make_float4(float(cr[j]), float(ci[j]), float(cr[j + 1]), float(ci[j + 1]));
+  }
+}
+
+// f(x, y, distance, pixel) for every pixel of rows [row0, row0 + rows) of a
+// grid of nx columns; (ax, rx, ay, ry): the grid's first pixel minus the
+// particle, split as radial_distance wants it.  A warp takes 8x8 pixels, two
+// per lane (rows y and y + 4): eight lanes on 4x2 pixels read intervals in
+// different banks.
+template <typename F>
+__device__ inline void fitr_rows(int nx, int row0, int rows, float ax, float rx, float ay,
+                                 float ry, F f) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int pc = (nx + 7) / 8, np = pc * ((rows + 7) / 8);
+  const int lx = 4 * ((lane >> 3) & 1) + (lane & 3);
+  const int ly = 2 * (lane >> 4) + ((lane >> 2) & 1);
+  for (int w = warp; w < np; w += FITR_TPB / 32) {
+    const int pr = w / pc, col = 8 * (w - pr * pc) + lx, row = row0 + 8 * pr + ly;
+    if (col >= nx || row >= row0 + rows) continue;
+    const float X = ax + float(col);
+    const f2 Y = pk(ay + float(row), ay + float(row + 4));
+    const float px = X * X;
+    const float lx2 = fmaf(2.f * rx, fmaf(0.5f, rx, X), fmaf(X, X, -px));
+    const f2 qy = pmul(Y, Y), r2 = pk(ry, ry);
+    const f2 ly2 = pfma(padd(r2, r2), pfma(pk(0.5f, 0.5f), r2, Y), pfma(Y, Y, pneg(qy)));
+    const RadialDistance d = radial_distance(pk(px, px), pk(lx2, lx2), qy, ly2);
+    f(X + rx, padd(Y, r2), d, (long long)row * nx + col, row + 4 < row0 + rows);
+  }
+}
+
+// The distance of a pixel of a list; (*x, *y): its FP32 offset.
+__device__ inline RadialDistance fitr_list_distance(double dx, double dy, float* x, float* y) {
+  const double ax = rint(dx * 1024.) * (1. / 1024.);
+  const double ay = rint(dy * 1024.) * (1. / 1024.);
+  const f2 X = pk(float(ax), float(ay)), rx = pk(float(dx - ax), float(dy - ay));
+  const f2 px = pmul(X, X);
+  const f2 lx = pfma(padd(rx, rx), pfma(pk(0.5f, 0.5f), rx, X), pfma(X, X, pneg(px)));
+  const f2 xr = padd(X, rx);
+  *x = xr.x;
+  *y = xr.y;
+  return radial_distance(pk(px.x, px.x), pk(lx.x, lx.x), pk(px.y, px.y), pk(lx.y, lx.y));
 }
 
 // Sum of acc over the block into out[0..FIT_NSUM) (doubles), fixed order.
@@ -499,30 +585,11 @@ k_fit_eval_radial(FitCtx c, RadialMatrix A, int cap) {
     // ---- nodes, polynomials
     for (int t = threadIdx.x; t < pl.n + 2 * RADIAL_SIDE; t += FITR_TPB) {
       const int j = abs(pl.lo - RADIAL_SIDE + t);
-      fitr_node<kKP>(c.k, j ? pl.spacing * double(j) : RADIAL_AXIS, ep.p[2],
+      fitr_node_call<kKP>(c.k, j ? pl.spacing * double(j) : RADIAL_AXIS, ep.p[2],
                      c.flags & LMB_BOHREN, c.aberr, c.inv_noise, ord, nm, val + t, vstride);
     }
     __syncthreads();
-    for (int w = threadIdx.x; w < pl.n * (NF / 2); w += FITR_TPB) {
-      const int g = w / pl.n, i = w - g * pl.n;
-      const double* s = val + 2 * g * vstride + i;
-      double cr[RADIAL_COEFS], ci[RADIAL_COEFS];
-#pragma unroll
-      for (int j = 0; j < RADIAL_COEFS; ++j) cr[j] = ci[j] = 0.;
-#pragma unroll
-      for (int l = 0; l < RADIAL_TAPS; ++l) {
-        const double x = s[l], y = s[vstride + l];
-#pragma unroll
-        for (int j = 0; j < RADIAL_COEFS; ++j) {
-          cr[j] = fma(A.m[j][l], x, cr[j]);
-          ci[j] = fma(A.m[j][l], y, ci[j]);
-        }
-      }
-      float4* o = tab + size_t(i) * REC + 3 * g;
-#pragma unroll
-      for (int j = 0; j < RADIAL_COEFS; j += 2)
-        o[j / 2] = make_float4(float(cr[j]), float(ci[j]), float(cr[j + 1]), float(ci[j + 1]));
-    }
+    fitr_polynomials<REC, NF>(A, val, vstride, pl.n, tab);
     __syncthreads();
     // ---- pixels
     const float spacing = float(pl.spacing), inv_spacing = float(1. / pl.spacing);
@@ -532,52 +599,197 @@ k_fit_eval_radial(FitCtx c, RadialMatrix A, int cap) {
 #pragma unroll
       for (int j = 0; j < FIT_NSUM; ++j) acc[j] = 0.f;
       if (ft.nx > 0) {
-        // 8x8 pixels per warp, two per lane (rows y and y + 4): eight lanes
-        // on 4x2 pixels read intervals in different banks
-        const int row0 = t * band, rows = min(band, ft.ny - row0);
-        const int pc = (ft.nx + 7) / 8, np = pc * ((rows + 7) / 8);
-        const int lx = 4 * ((lane >> 3) & 1) + (lane & 3);
-        const int ly = 2 * (lane >> 4) + ((lane >> 2) & 1);
-        for (int w = warp; w < np; w += FITR_TPB / 32) {
-          const int pr = w / pc, col = 8 * (w - pr * pc) + lx, row = row0 + 8 * pr + ly;
-          if (col >= ft.nx || row >= row0 + rows) continue;
-          const bool two = row + 4 < row0 + rows;
-          const float* dp = c.data + ft.data_offset + (long long)row * ft.nx + col;
-          const float d0 = dp[0], d1 = two ? dp[4LL * ft.nx] : 0.f;
-          const float X = pl.ax + float(col);
-          const f2 Y = pk(pl.ay + float(row), pl.ay + float(row + 4));
-          const float px = X * X;
-          const float lx2 = fmaf(2.f * pl.rx, fmaf(0.5f, pl.rx, X), fmaf(X, X, -px));
-          const f2 qy = pmul(Y, Y), ry = pk(pl.ry, pl.ry);
-          const f2 ly2 = pfma(padd(ry, ry), pfma(pk(0.5f, 0.5f), ry, Y), pfma(Y, Y, pneg(qy)));
-          const RadialDistance d = radial_distance(pk(px, px), pk(lx2, lx2), qy, ly2);
-          const float xr = X + pl.rx;
-          const f2 yr = padd(Y, ry);
-          fitr_pixel<kKP>(tab, d.r0.x, d.corr.x, d.y.x, xr, yr.x, inv_spacing, spacing, inv_half,
-                          pl.lo, pl.n, d0, inv_noise, acc);
-          if (two)
-            fitr_pixel<kKP>(tab, d.r0.y, d.corr.y, d.y.y, xr, yr.y, inv_spacing, spacing, inv_half,
-                            pl.lo, pl.n, d1, inv_noise, acc);
-        }
+        const int row0 = t * band;
+        const float* data = c.data + ft.data_offset;
+        fitr_rows(ft.nx, row0, min(band, ft.ny - row0), pl.ax, pl.rx, pl.ay, pl.ry,
+                  [&](float x, f2 y, const RadialDistance& d, long long i, bool two) {
+                    const float d0 = data[i], d1 = two ? data[i + 4LL * ft.nx] : 0.f;
+                    fitr_pixel<kKP>(tab, d.r0.x, d.corr.x, d.y.x, x, y.x, inv_spacing, spacing,
+                                    inv_half, pl.lo, pl.n, d0, inv_noise, acc);
+                    if (two)
+                      fitr_pixel<kKP>(tab, d.r0.y, d.corr.y, d.y.y, x, y.y, inv_spacing,
+                                      spacing, inv_half, pl.lo, pl.n, d1, inv_noise, acc);
+                  });
       } else {
         const long long a = (long long)t * FITR_TILE, b = min(a + FITR_TILE, ft.npix);
         for (long long i = a + threadIdx.x; i < b; i += FITR_TPB) {
           const float2 xy = reinterpret_cast<const float2*>(c.coords)[ft.data_offset + i];
-          const double dx = double(xy.x) - ep.p[0], dy = double(xy.y) - ep.p[1];
-          const double ax = rint(dx * 1024.) * (1. / 1024.);
-          const double ay = rint(dy * 1024.) * (1. / 1024.);
-          const f2 X = pk(float(ax), float(ay)), rx = pk(float(dx - ax), float(dy - ay));
-          const f2 px = pmul(X, X);
-          const f2 lx = pfma(padd(rx, rx), pfma(pk(0.5f, 0.5f), rx, X), pfma(X, X, pneg(px)));
-          const f2 xr = padd(X, rx);
-          const RadialDistance d = radial_distance(pk(px.x, px.x), pk(lx.x, lx.x),
-                                                   pk(px.y, px.y), pk(lx.y, lx.y));
-          fitr_pixel<kKP>(tab, d.r0.x, d.corr.x, d.y.x, xr.x, xr.y, inv_spacing, spacing, inv_half,
+          float x, y;
+          const RadialDistance d = fitr_list_distance(double(xy.x) - ep.p[0],
+                                                      double(xy.y) - ep.p[1], &x, &y);
+          fitr_pixel<kKP>(tab, d.r0.x, d.corr.x, d.y.x, x, y, inv_spacing, spacing, inv_half,
                           pl.lo, pl.n, c.data[ft.data_offset + i], inv_noise, acc);
         }
       }
       fitr_reduce(acc, red, c.partial + (size_t)(c.tile_begin[f] + t) * FIT_NSUM);
     }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Gradients of holograms (the VJP) from the same tables, in two kernels: the
+// nodes of every sphere, one a thread in blocks of FITR_NODE_TPB (the chain
+// of FP64 recurrences is latency-bound, so the nodes are spread over all SMs
+// and each thread may hold its sums in registers); then blocks of rows,
+// which take their range of nodes, form the polynomials and sum g dH/dp.
+
+struct GradPlan {
+  double x0, y0, z, k, spacing;  // first pixel (or the box's corner), plane
+  long long nx, ny, npts;
+  const double* points;  // null: the grid's pixels
+  int intervals;         // room per sphere
+  int parts, flags;
+};
+
+enum { FITR_NODE_TPB = 32 };
+
+// Intervals that cover the pixels of a sphere at (xp, yp).
+__device__ inline int grad_count(const GradPlan& pl, double xp, double yp) {
+  const double dx = fmax(fabs(pl.x0 - xp), fabs(pl.x0 + double(pl.nx - 1) - xp));
+  const double dy = fmax(fabs(pl.y0 - yp), fabs(pl.y0 + double(pl.ny - 1) - yp));
+  return min(pl.intervals, int(sqrt(fma(dx, dx, dy * dy)) / pl.spacing) + 2);
+}
+
+// nodes [nitems][10][intervals + 16]
+__global__ void __launch_bounds__(FITR_NODE_TPB)
+k_grad_nodes(GradPlan pl, const lmb_sphere* __restrict__ spheres,
+             const zd* __restrict__ ab, const zd* __restrict__ dab,
+             const int* __restrict__ nmax, int nmaxp, double* __restrict__ nodes) {
+  extern __shared__ __align__(16) char smem[];
+  FitrOrder* ord = reinterpret_cast<FitrOrder*>(smem);
+  const int item = blockIdx.y;
+  const lmb_sphere sp = spheres[item];
+  const int first = blockIdx.x * FITR_NODE_TPB;
+  const int count = grad_count(pl, sp.x_p, sp.y_p) + 2 * RADIAL_SIDE;
+  if (first >= count) return;  // the whole block
+  const int nm = min(max(nmax[item], 0), nmaxp - 1);
+  for (int n = threadIdx.x; n <= nm; n += FITR_NODE_TPB) {
+    const double fn = double(n);
+    FitrOrder o;
+    o.fn = fn;
+    o.tn1 = 2. * fn - 1.;
+    o.cn = n ? 1. + 1. / fn : 0.;
+    o.en = n ? o.tn1 + 2. : 0.;
+    const double en = n ? o.en / (fn * (fn + 1.)) : 0.;
+    for (int j = 0; j < 3; ++j) {
+      const zd* s = j == 0 ? ab + (size_t(item) * nmaxp + n) * 2
+                           : dab + (size_t(item) * nmaxp + n) * 4 + 2 * (j - 1);
+      o.v[2 * j] = en * rot_i(s[0], n + 1);
+      o.v[2 * j + 1] = en * rot_i(s[1], n);
+      o.z[j] = o.en * rot_i(s[0], n + 1);
+    }
+    ord[n] = o;
+  }
+  __syncthreads();
+  const int t = first + threadIdx.x;
+  if (t >= count) return;
+  const int j = abs(t - RADIAL_SIDE);
+  const int stride = pl.intervals + 2 * RADIAL_SIDE;
+  fitr_node<true>(pl.k, j ? pl.spacing * double(j) : RADIAL_AXIS, pl.z, sp.z_p,
+                  pl.flags & LMB_BOHREN, 0., 1., ord, nm,
+                  nodes + size_t(item) * fitr_funcs(true) * stride + t, stride);
+}
+
+// partial [nitems][parts][6]; cap: intervals that the table has room for.
+__global__ void __launch_bounds__(FITR_TPB, 2)
+k_vjp_radial(GradPlan pl, RadialMatrix A, int cap, const lmb_sphere* __restrict__ spheres,
+             const double* __restrict__ nodes, const float* __restrict__ gout,
+             double* __restrict__ partial) {
+  extern __shared__ __align__(16) char smem[];
+  __shared__ double red[FITR_TPB / 32][6];
+  constexpr int REC = fitr_rec(true), NF = fitr_funcs(true);
+  float4* tab = reinterpret_cast<float4*>(smem);                     // [cap][REC]
+  double* val = reinterpret_cast<double*>(tab + size_t(cap) * REC);  // [NF][cap + 16]
+  const int vstride = cap + 2 * RADIAL_SIDE;
+  const int item = blockIdx.y, part = blockIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const lmb_sphere sp = spheres[item];
+  const int count = grad_count(pl, sp.x_p, sp.y_p);
+  const float* g = gout + size_t(item) * pl.npts;
+  // the part: rows in whole patches of 8, or a run of the list
+  const long long groups = pl.points ? pl.npts : (pl.ny + 7) / 8;
+  const long long b0 = groups * part / pl.parts, b1 = groups * (part + 1) / pl.parts;
+  double acc[6] = {0., 0., 0., 0., 0., 0.};
+  if (b0 < b1) {
+    const double ox = pl.x0 - sp.x_p, oy = pl.y0 - sp.y_p;
+    float rho_lo = 0.f, rho_hi = 3e38f;  // of a list: all of the table
+    const int row0 = pl.points ? 0 : int(8 * b0);
+    const int rows = pl.points ? 0 : int(min(8 * b1, pl.ny) - 8 * b0);
+    if (!pl.points) {
+      const float x0 = float(ox), x1 = x0 + float(pl.nx - 1);
+      const float y0 = float(oy) + float(row0), y1 = y0 + float(rows - 1);
+      const float ex = x0 > 0.f ? x0 : (x1 < 0.f ? -x1 : 0.f);
+      const float ey = y0 > 0.f ? y0 : (y1 < 0.f ? -y1 : 0.f);
+      const float fx = fmaxf(fabsf(x0), fabsf(x1)), fy = fmaxf(fabsf(y0), fabsf(y1));
+      rho_lo = sqrtf(ex * ex + ey * ey);
+      rho_hi = sqrtf(fx * fx + fy * fy);
+    }
+    const float spacing = float(pl.spacing), inv_spacing = 1.f / spacing;
+    const float inv_half = 2.f * inv_spacing;
+    const int hi = rho_hi < 1e9f ? min(count, int(rho_hi * inv_spacing) + 3) : count;
+    const int lo = max(0, min(int(rho_lo * inv_spacing) - 1, hi - 1));
+    const double ax = rint(ox * 1024.) * (1. / 1024.), ay = rint(oy * 1024.) * (1. / 1024.);
+    const float fax = float(ax), frx = float(ox - ax), fay = float(ay), fry = float(oy - ay);
+    const int stride = pl.intervals + 2 * RADIAL_SIDE;
+    const double* src = nodes + size_t(item) * NF * stride;
+    // the table in pieces of cap intervals: a wide part takes several passes
+    for (int at = lo; at < hi; at += cap) {
+      const int n = min(cap, hi - at);
+      __syncthreads();  // the previous piece is no longer read
+      for (int w = threadIdx.x; w < NF * (n + 2 * RADIAL_SIDE); w += FITR_TPB) {
+        const int f = w / (n + 2 * RADIAL_SIDE), i = w - f * (n + 2 * RADIAL_SIDE);
+        val[f * vstride + i] = src[f * stride + at + i];
+      }
+      __syncthreads();
+      fitr_polynomials<REC, NF>(A, val, vstride, n, tab);
+      __syncthreads();
+      // a pixel belongs to the piece that holds its interval (clamped to the
+      // part's range)
+      float sum[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      int in_sum = 0;
+      auto add = [&](float r0, float corr, float iy, float x, float y, long long i) {
+        const int iv = min(max(__float2int_rn(r0 * inv_spacing), lo), hi - 1);
+        if (iv < at || iv >= at + n) return;
+        float J[6];
+        fitr_lookup<true>(tab, r0, corr, iy, x, y, inv_spacing, spacing, inv_half, at, n, J);
+        const float go = g[i];
+#pragma unroll
+        for (int j = 0; j < 6; ++j) sum[j] = fmaf(go, J[j], sum[j]);
+        if (++in_sum == 8) {  // short FP32 sums
+          for (int j = 0; j < 6; ++j) {
+            acc[j] += double(sum[j]);
+            sum[j] = 0.f;
+          }
+          in_sum = 0;
+        }
+      };
+      if (pl.points) {
+        for (long long i = b0 + threadIdx.x; i < b1; i += FITR_TPB) {
+          float x, y;
+          const RadialDistance d = fitr_list_distance(
+              pl.points[i] - sp.x_p, pl.points[pl.npts + i] - sp.y_p, &x, &y);
+          add(d.r0.x, d.corr.x, d.y.x, x, y, i);
+        }
+      } else {
+        fitr_rows(int(pl.nx), row0, rows, fax, frx, fay, fry,
+                  [&](float x, f2 y, const RadialDistance& d, long long i, bool two) {
+                    add(d.r0.x, d.corr.x, d.y.x, x, y.x, i);
+                    if (two) add(d.r0.y, d.corr.y, d.y.y, x, y.y, i + 4 * pl.nx);
+                  });
+      }
+      for (int j = 0; j < 6; ++j) acc[j] += double(sum[j]);
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1)
+    for (int j = 0; j < 6; ++j) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
+  __syncthreads();
+  if (lane == 0)
+    for (int j = 0; j < 6; ++j) red[warp][j] = acc[j];
+  __syncthreads();
+  if (threadIdx.x < 6) {
+    double s = 0.;
+    for (int w = 0; w < FITR_TPB / 32; ++w) s += red[w][threadIdx.x];
+    partial[(size_t(item) * pl.parts + part) * 6 + threadIdx.x] = s;
   }
 }
 

@@ -42,12 +42,18 @@ __global__ void k_probe_init(long long npts, unsigned long long* out) {
 __global__ void k_probe_row(const double* __restrict__ coords, long long npts,
                             unsigned long long* out) {
   const double y0 = coords[npts];
+  unsigned long long first = (unsigned long long)npts;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < npts;
        i += (long long)gridDim.x * blockDim.x)
     if (coords[npts + i] != y0) {
-      atomicMin(out + PROBE_ROW, (unsigned long long)i);
+      first = (unsigned long long)i;
       break;
     }
+  for (int o = 16; o > 0; o >>= 1) first = min(first, __shfl_xor_sync(0xffffffffu, first, o));
+  // most warps find a later index than is already there
+  if ((threadIdx.x & 31) == 0 &&
+      first < *reinterpret_cast<volatile unsigned long long*>(out + PROBE_ROW))
+    atomicMin(out + PROBE_ROW, first);
 }
 
 // How many pixels are not (x0 + column, y0 + row, z0), how many are not

@@ -342,6 +342,32 @@ def hologram_vjp(coords, spheres, ab, dab, nmax, cap, k, gout, bohren=True):
     return grad
 
 
+def vjp_on_grid(grid, coords, records, spheres, ab, dab, nmax, cap,
+                instrument, gout, bohren=True):
+    '''hologram_vjp for pixels of one plane (make_grid's result) from radial
+    tables (lmb_hologram_vjp_grid); None where they do not apply.'''
+    lib = _native.load()
+    grid, full = grid
+    n, npts = len(records), coords.shape[1]
+    k, mag = float(instrument.wavenumber()), float(instrument.magnification)
+    flags = _flags(True, bohren, False)
+    nbytes = lib.lmb_vjp_grid_workspace_bytes(
+        grid, npts, records.ctypes.data, n, k, mag, flags)
+    if not 0 < nbytes <= RADIAL_WORKSPACE_LIMIT:
+        return None
+    dev = coords.device
+    ab, dab, nmax, spheres = _contiguous(ab, dab, nmax, spheres)
+    gout = gout.to(torch.float32).contiguous()
+    grad = torch.empty((n, 6), dtype=torch.float64, device=dev)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    _native.check(lib.lmb_hologram_vjp_grid(
+        grid, None if full else ptr(coords), npts, records.ctypes.data,
+        ptr(spheres), n, ptr(ab), ptr(dab), ptr(nmax), cap, k, mag, flags,
+        ptr(gout), ptr(grad), ptr(ws), nbytes, stream_handle(dev)),
+        'lmb_hologram_vjp_grid')
+    return grad
+
+
 def wiscombe_yang_layers(radii, indices, n_m, wavelength):
     '''Host n_max of one multilayer sphere (radii ascending, complex indices).'''
     k = 2. * np.pi / wavelength * float(np.real(n_m))

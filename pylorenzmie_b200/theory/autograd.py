@@ -20,13 +20,19 @@ from . import _kernels as K
 from .Instrument import Instrument
 
 
-def _prepare(params, instrument):
+def _prepare(params, instrument, host=None):
     p = params.detach().to(torch.float64).contiguous()
     inst = instrument or Instrument()
-    host = p.cpu().numpy()
+    if host is None:
+        host = p.cpu().numpy()
     cap = K.nmax_cap_for(host[:, 3], host[:, 4], host[:, 5], inst.n_m,
                          inst.wavelength)
-    ab, dab, nmax = K.sphere_ab(p, inst.n_m, inst.wavelength, cap, deriv=True)
+    # the capacity covers these spheres, so the coefficients can fail only on
+    # invalid parameters: checked here, without reading the device again
+    if not (np.isfinite(host).all() and (host[:, 3] > 0.).all()):
+        raise ValueError('sphere parameters must be finite with a_p > 0')
+    ab, dab, nmax = K.sphere_ab(p, inst.n_m, inst.wavelength, cap, deriv=True,
+                                check=False)
     return p, inst, cap, ab, dab, nmax
 
 
@@ -43,21 +49,44 @@ class HologramFunction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, params, coordinates, instrument, bohren):
-        p, inst, cap, ab, dab, nmax = _prepare(params, instrument)
-        B = p.shape[0]
+        # the parameters and the pixels' layout in one read-back
+        B, npts = params.shape[0], coordinates.shape[1]
+        grid, host = None, None
+        if B and npts:
+            both = torch.cat([
+                params.detach().to(torch.float64).reshape(-1),
+                coordinates[2, :1],
+                K.probe_grid(coordinates).view(torch.float64)]).cpu().numpy()
+            host = both[:6 * B].reshape(B, 6).copy()
+            grid = K.make_grid(both[6 * B], npts,
+                               both[6 * B + 1:].view(np.int64))
+        p, inst, cap, ab, dab, nmax = _prepare(params, instrument, host)
         item_start = torch.arange(B + 1, dtype=torch.int32, device=p.device)
-        h = K.hologram(coordinates, p, item_start, ab, nmax, cap,
-                       inst.wavenumber(), True, bohren, False)
+        h = None
+        records = None if grid is None else host.view(K.SPHERE_DTYPE).ravel()
+        if grid is not None:
+            h = K.on_grid(grid, coordinates, records, p, item_start, ab, nmax,
+                          cap, inst, True, bohren, 0.)
+        if h is None:
+            h = K.hologram(coordinates, p, item_start, ab, nmax, cap,
+                           inst.wavenumber(), True, bohren, False)
         ctx.save_for_backward(p, coordinates, ab, dab, nmax)
         ctx.inst, ctx.cap, ctx.bohren = inst, cap, bohren
+        ctx.grid, ctx.records = grid, records
         return h
 
     @staticmethod
     def backward(ctx, gout):
         p, coordinates, ab, dab, nmax = ctx.saved_tensors
-        grad = K.hologram_vjp(coordinates, p, ab, dab, nmax, ctx.cap,
-                              ctx.inst.wavenumber(), gout.contiguous(),
-                              ctx.bohren)
+        grad = None
+        if ctx.grid is not None:
+            grad = K.vjp_on_grid(ctx.grid, coordinates, ctx.records, p, ab,
+                                 dab, nmax, ctx.cap, ctx.inst, gout,
+                                 ctx.bohren)
+        if grad is None:
+            grad = K.hologram_vjp(coordinates, p, ab, dab, nmax, ctx.cap,
+                                  ctx.inst.wavenumber(), gout.contiguous(),
+                                  ctx.bohren)
         return grad.to(p.dtype), None, None, None
 
 
