@@ -138,8 +138,8 @@ int lmb_hologram_aberrated(const double *coords, long long npts,
  * Fields and holograms on a unit-step pixel grid in one plane, from radial
  * tables: in a plane the sums over the orders depend on the distance from a
  * sphere's axis alone, so they are formed in FP64 at equidistant distances
- * and interpolated at the pixels (FP32 outputs, within the FP32 rounding of
- * the direct sums; holograms within 2e-5 of FP64 as lmb_hologram).  Pixel
+ * and interpolated at the pixels, within the rounding of the direct sums
+ * (FP32 holograms within 2e-5 of FP64, as lmb_hologram).  Pixel
  * (column, row) lies at (x0 + column, y0 + row, z), row-major outputs.
  *
  * With ``points`` (device, [3][npts], all in the plane z) the pixels are
@@ -157,13 +157,15 @@ int lmb_hologram_aberrated(const double *coords, long long npts,
  *                      apply and the coordinate entry points are to be used:
  *                      a plane closer than k d = 1.8 to a sphere or cutting
  *                      it, distances above 8000 px, spherical components,
- *                      FP64, an aberration phase steeper than a fifth of k,
+ *                      an aberration phase steeper than a fifth of k,
  *                      or too few pixels to pay for the tables.
  * lmb_field_grid / lmb_hologram_grid: as lmb_field_aberrated /
  *                      lmb_hologram_aberrated (aberration 0: ideal optics);
  *                      nparticles = item_start[nitems], intervals from
  *                      lmb_radial_intervals, workspace of
- *                      lmb_radial_workspace_bytes(nparticles, intervals).
+ *                      lmb_radial_workspace_bytes(nparticles, intervals,
+ *                      flags).  LMB_FP64: FP64 tables and outputs, a grid's
+ *                      pixels only.
  */
 typedef struct lmb_grid {
   double x0, y0, z;
@@ -174,7 +176,7 @@ int lmb_grid_probe(const double *coords, long long npts,
 int lmb_radial_intervals(const lmb_grid *grid, long long npts,
                          const lmb_sphere *spheres, int n, double k, double magnification, int flags,
                          double aberration);
-size_t lmb_radial_workspace_bytes(int nparticles, int intervals);
+size_t lmb_radial_workspace_bytes(int nparticles, int intervals, int flags);
 int lmb_field_grid(const lmb_grid *grid, const double *points,
                    long long npts, const lmb_sphere *spheres,
                    const int *item_start, int nitems, int nparticles,

@@ -92,7 +92,7 @@ _SIGNATURES = {
     'lmb_grid_probe': (_i, [_vp, _ll, _vp, _vp]),
     'lmb_radial_intervals': (_i, [ctypes.POINTER(Grid), _ll, _vp, _i, _d, _d,
                                   _i, _d]),
-    'lmb_radial_workspace_bytes': (_sz, [_i, _i]),
+    'lmb_radial_workspace_bytes': (_sz, [_i, _i, _i]),
     'lmb_field_grid': (_i, [ctypes.POINTER(Grid), _vp, _ll, _vp, _vp, _i, _i,
                             _i, _vp, _vp, _i, _d, _i, _d, _vp, _vp, _sz,
                             _vp]),

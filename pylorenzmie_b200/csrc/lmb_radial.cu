@@ -107,8 +107,9 @@ struct RadialPlan {
 
 // Interval width in pixels, a multiple of 1/64 so that i * width is exact
 // in FP32; 0 if k is out of range.
-inline double radial_spacing(double k) {
-  const double w = std::min(floor(64. * RADIAL_SPACING / k) / 64., 64.);
+inline double radial_spacing(double k, bool fp64) {
+  const double r = fp64 ? RADIAL_SPACING64 : RADIAL_SPACING;
+  const double w = std::min(floor(64. * r / k) / 64., 64.);
   return w >= 0.0625 ? w : 0.;
 }
 
@@ -138,10 +139,12 @@ __host__ __device__ inline int radial_count(double reach, double spacing) {
 constexpr int kNodeThreads = 128;
 constexpr int kChunk = kNodeThreads - 2 * RADIAL_SIDE;
 
+// R = float or double: the coefficients' type (double: no nodes are kept).
+template <typename R, int NC>
 __global__ void __launch_bounds__(kNodeThreads)
-k_radial_table(RadialPlan pl, RadialMatrix A, const lmb_sphere* __restrict__ spheres,
+k_radial_table(RadialPlan pl, RadialMatrixN<NC> A, const lmb_sphere* __restrict__ spheres,
                const zd* __restrict__ ab, const int* __restrict__ nmax, int nmaxp,
-               float* __restrict__ table, double* __restrict__ nodes) {
+               R* __restrict__ table, double* __restrict__ nodes) {
   extern __shared__ __align__(16) char smem[];
   double* val = reinterpret_cast<double*>(smem);  // [RADIAL_FUNCS][kNodeThreads]
   Quad<double>* rec = reinterpret_cast<Quad<double>*>(
@@ -164,40 +167,64 @@ k_radial_table(RadialPlan pl, RadialMatrix A, const lmb_sphere* __restrict__ sph
   const int ncap = pl.intervals + 2 * RADIAL_SIDE;
   if (j < count + RADIAL_SIDE) {
     double v[RADIAL_FUNCS];
-    radial_field(pl.k, j ? pl.spacing * double(abs(j)) : RADIAL_AXIS, pl.z - sp.z_p, pl.z,
-                 sp.z_p, pl.flags & LMB_BOHREN, pl.aberr, rec, nm, v);
+    // V and Z at the axis are limits: nearly there for FP32, from their
+    // neighbours (below) for FP64
+    const double axis = sizeof(R) == sizeof(float) ? RADIAL_AXIS : 0.;
+    radial_field(pl.k, j ? pl.spacing * double(abs(j)) : axis, pl.z - sp.z_p, pl.z, sp.z_p,
+                 pl.flags & LMB_BOHREN, pl.aberr, rec, nm, v);
     const int t = threadIdx.x;
     for (int f = 0; f < RADIAL_FUNCS; ++f) val[f * kNodeThreads + t] = v[f];
     // each node is written by the chunk it lies in (the ends by the outer ones)
-    if ((t >= RADIAL_SIDE || i0 == 0) &&
+    if (nodes && (t >= RADIAL_SIDE || i0 == 0) &&
         (t < kNodeThreads - RADIAL_SIDE || i0 + kChunk >= count)) {
       double* out = nodes + (size_t(p) * ncap + (j + RADIAL_SIDE)) * RADIAL_FUNCS;
       for (int f = 0; f < RADIAL_FUNCS; ++f) out[f] = v[f];
     }
   }
   __syncthreads();
+  if (sizeof(R) == sizeof(double) && i0 == 0) {
+    // the even function through the nodes 1..8 and -1..-8, at 0: off by at
+    // most 3e-13 at this spacing
+    if (threadIdx.x >= 2 && threadIdx.x < RADIAL_FUNCS) {
+      double* s = val + threadIdx.x * kNodeThreads + RADIAL_SIDE;
+      double sum = 0., w = 1.;
+      for (int m = 1; m <= RADIAL_SIDE; ++m) {
+        w *= -double(RADIAL_SIDE + 1 - m) / double(RADIAL_SIDE + m);
+        sum -= 2. * w * s[m];
+      }
+      s[0] = sum;
+    }
+    __syncthreads();
+  }
   const int n = min(kChunk, count - i0);
   for (int w = threadIdx.x; w < n * (RADIAL_FUNCS / 2); w += kNodeThreads) {
     const int f = w / n, i = w - f * n;
     const double* s = val + 2 * f * kNodeThreads + i;
-    double cr[RADIAL_COEFS], ci[RADIAL_COEFS];
+    double cr[NC], ci[NC];
 #pragma unroll
-    for (int q = 0; q < RADIAL_COEFS; ++q) cr[q] = ci[q] = 0.;
+    for (int q = 0; q < NC; ++q) cr[q] = ci[q] = 0.;
 #pragma unroll
     for (int l = 0; l < RADIAL_TAPS; ++l) {
       const double x = s[l], y = s[kNodeThreads + l];
 #pragma unroll
-      for (int q = 0; q < RADIAL_COEFS; ++q) {
+      for (int q = 0; q < NC; ++q) {
         cr[q] = fma(A.m[q][l], x, cr[q]);
         ci[q] = fma(A.m[q][l], y, ci[q]);
       }
     }
     // re and im of a coefficient side by side
-    float4* out = reinterpret_cast<float4*>(
-        table + (size_t(p) * pl.intervals + i0 + i) * RADIAL_REC + f * 2 * RADIAL_COEFS);
+    R* out = table + (size_t(p) * pl.intervals + i0 + i) * (RADIAL_FUNCS * NC) + f * 2 * NC;
+    if constexpr (sizeof(R) == sizeof(float)) {
+      static_assert(sizeof(R) == sizeof(double) || NC % 2 == 0, "whole float4");
 #pragma unroll
-    for (int q = 0; q < RADIAL_COEFS; q += 2)
-      out[q / 2] = make_float4(float(cr[q]), float(ci[q]), float(cr[q + 1]), float(ci[q + 1]));
+      for (int q = 0; q < NC; q += 2)
+        reinterpret_cast<float4*>(out)[q / 2] =
+            make_float4(float(cr[q]), float(ci[q]), float(cr[q + 1]), float(ci[q + 1]));
+    } else {
+#pragma unroll
+      for (int q = 0; q < NC; ++q)
+        reinterpret_cast<double2*>(out)[q] = make_double2(cr[q], ci[q]);
+    }
   }
 }
 
@@ -274,6 +301,31 @@ struct TileParticle {
   int lo, count;         // intervals that the tile's pixels use
 };
 
+// The intervals that a tile of w x h pixels at (tx, ty) needs of a particle,
+// at most room of them.
+__device__ inline TileParticle tile_particle(const RadialPlan& pl, const lmb_sphere& sp,
+                                             long long tx, long long ty, int w, int h,
+                                             int room) {
+  const double dx = pl.x0 + double(tx) - sp.x_p, dy = pl.y0 + double(ty) - sp.y_p;
+  TileParticle t;
+  const double ax = rint(dx * 1024.) * (1. / 1024.), ay = rint(dy * 1024.) * (1. / 1024.);
+  t.ax = float(ax);
+  t.rx = float(dx - ax);
+  t.ay = float(ay);
+  t.ry = float(dy - ay);
+  // nearest and farthest distances of the tile's pixels
+  const double ex = double(w - 1), ey = double(h - 1);
+  const double nx = dx > 0. ? dx : (dx + ex < 0. ? -(dx + ex) : 0.);
+  const double ny = dy > 0. ? dy : (dy + ey < 0. ? -(dy + ey) : 0.);
+  const double fx = fmax(fabs(dx), fabs(dx + ex)), fy = fmax(fabs(dy), fabs(dy + ey));
+  const int all = min(pl.intervals, radial_count(radial_reach(pl.x0, pl.y0, pl.nx, pl.ny,
+                                                              sp.x_p, sp.y_p), pl.spacing));
+  t.lo = max(0, min(all - 1, int(sqrt(nx * nx + ny * ny) / pl.spacing) - 1));
+  const int hi = min(all, int(sqrt(fx * fx + fy * fy) / pl.spacing) + 3);
+  t.count = max(1, min(hi - t.lo, room));
+  return t;
+}
+
 constexpr int kTile = 32;          // tiles of 32 x 32 pixels
 constexpr int kPixThreads = 256;   // a 2x2 group each
 constexpr int kTileGroup = 32;     // particles whose TileParticle is staged at once
@@ -331,25 +383,8 @@ k_field_radial(RadialPlan pl, const lmb_sphere* __restrict__ spheres,
     const int G = min(kTileGroup, pe - g0);
     __syncthreads();  // the previous group's data is no longer read
     if (threadIdx.x < G) {
-      const lmb_sphere sp = spheres[g0 + threadIdx.x];
-      const double dx = pl.x0 + double(tx) - sp.x_p, dy = pl.y0 + double(ty) - sp.y_p;
-      TileParticle t;
-      const double ax = rint(dx * 1024.) * (1. / 1024.), ay = rint(dy * 1024.) * (1. / 1024.);
-      t.ax = float(ax);
-      t.rx = float(dx - ax);
-      t.ay = float(ay);
-      t.ry = float(dy - ay);
-      // nearest and farthest distances of the tile's pixels
-      const double e = double(kTile - 1);
-      const double nx = dx > 0. ? dx : (dx + e < 0. ? -(dx + e) : 0.);
-      const double ny = dy > 0. ? dy : (dy + e < 0. ? -(dy + e) : 0.);
-      const double fx = fmax(fabs(dx), fabs(dx + e)), fy = fmax(fabs(dy), fabs(dy + e));
-      const int all = min(pl.intervals,
-                          radial_count(radial_reach(pl.x0, pl.y0, pl.nx, pl.ny, sp.x_p,
-                                                    sp.y_p), pl.spacing));
-      t.lo = max(0, min(all - 1, int(sqrt(nx * nx + ny * ny) / pl.spacing) - 1));
-      const int hi = min(all, int(sqrt(fx * fx + fy * fy) / pl.spacing) + 3);
-      t.count = max(1, min(hi - t.lo, buffer / RQ));
+      const TileParticle t = tile_particle(pl, spheres[g0 + threadIdx.x], tx, ty, kTile,
+                                           kTile, buffer / RQ);
       s_tp[threadIdx.x] = t;
     }
     __syncthreads();
@@ -461,6 +496,105 @@ k_field_radial(RadialPlan pl, const lmb_sphere* __restrict__ spheres,
   }
 }
 
+// FP64 images: the same in double, tiles of 32 x 16 pixels, two pixels (rows
+// y and y + 4) per thread, 8x8 pixels per warp.  27 LDS.128 a pixel and
+// particle: bound by shared memory.
+constexpr int kTileH64 = 16;
+template <bool kHolo>
+__global__ void __launch_bounds__(kPixThreads, 2)
+k_field_radial64(RadialPlan pl, const lmb_sphere* __restrict__ spheres,
+                 const int* __restrict__ item_start, const double* __restrict__ table,
+                 int buffer, int stages, void* out) {
+  extern __shared__ __align__(16) double2 buf64[];  // [stages][buffer]
+  __shared__ TileParticle s_tp[kTileGroup];
+  constexpr int RQ = RADIAL_REC64 / 2;  // double2 per interval
+  const int item = blockIdx.z;
+  const int pb = item_start[item], pe = item_start[item + 1];
+  const long long tx = (long long)blockIdx.x * kTile, ty = (long long)blockIdx.y * kTileH64;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int cx = 8 * (warp & 3) + 4 * ((lane >> 3) & 1) + (lane & 3);
+  const int cy = 8 * (warp >> 2) + 2 * (lane >> 4) + ((lane >> 2) & 1);
+  const double inv_spacing = 1. / pl.spacing, inv_half = 2. / pl.spacing;
+  const double x0 = pl.x0 + double(tx + cx), y0 = pl.y0 + double(ty + cy);
+  double2 e[2][3];
+  for (int q = 0; q < 2; ++q)
+    for (int c = 0; c < 3; ++c) e[q][c] = make_double2(0., 0.);
+  for (int g0 = pb; g0 < pe; g0 += kTileGroup) {
+    const int G = min(kTileGroup, pe - g0);
+    __syncthreads();  // the previous group's data is no longer read
+    if (threadIdx.x < G)
+      s_tp[threadIdx.x] = tile_particle(pl, spheres[g0 + threadIdx.x], tx, ty, kTile,
+                                        kTileH64, buffer / RQ);
+    __syncthreads();
+    auto fetch = [&](int g) {
+      if (g < G) {
+        const TileParticle t = s_tp[g];
+        const double2* src = reinterpret_cast<const double2*>(table) +
+                             (size_t(g0 + g) * pl.intervals + t.lo) * RQ;
+        double2* dst = buf64 + (g % stages) * buffer;
+        for (int i = threadIdx.x; i < t.count * RQ; i += kPixThreads)
+          __pipeline_memcpy_async(dst + i, src + i, 16);
+      }
+      __pipeline_commit();
+    };
+    if (stages > 1) fetch(0);
+    for (int g = 0; g < G; ++g) {
+      if (stages > 1) {
+        fetch(g + 1);
+        __pipeline_wait_prior(1);
+      } else {
+        fetch(g);
+        __pipeline_wait_prior(0);
+      }
+      __syncthreads();  // copy g has landed
+      const TileParticle t = s_tp[g];
+      const double2* rec = buf64 + (g % stages) * buffer;
+      const double dx = x0 - spheres[g0 + g].x_p, dy0 = y0 - spheres[g0 + g].y_p;
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const double dy = dy0 + 4. * q;
+        const double rho = sqrt(fma(dx, dx, dy * dy));
+        const int i = min(max(__double2int_rn(rho * inv_spacing) - t.lo, 0), t.count - 1);
+        const double u = (rho - double(i + t.lo) * pl.spacing) * inv_half;
+        const double2* r = rec + i * RQ;
+        const double c2 = (dx - dy) * (dx + dy), s2 = 2. * dx * dy;
+        double2 v[3];
+#pragma unroll
+        for (int f = 0; f < 3; ++f) {
+          v[f] = r[f * RADIAL_COEFS64 + RADIAL_COEFS64 - 1];
+#pragma unroll
+          for (int j = RADIAL_COEFS64 - 2; j >= 0; --j) {
+            const double2 c = r[f * RADIAL_COEFS64 + j];
+            v[f].x = fma(v[f].x, u, c.x);
+            v[f].y = fma(v[f].y, u, c.y);
+          }
+        }
+        e[q][0].x = fma(c2, v[1].x, e[q][0].x + v[0].x);
+        e[q][0].y = fma(c2, v[1].y, e[q][0].y + v[0].y);
+        e[q][1].x = fma(s2, v[1].x, e[q][1].x);
+        e[q][1].y = fma(s2, v[1].y, e[q][1].y);
+        e[q][2].x = fma(dx, v[2].x, e[q][2].x);
+        e[q][2].y = fma(dx, v[2].y, e[q][2].y);
+      }
+      __syncthreads();  // this buffer is refilled from here on
+    }
+  }
+  const long long npts = pl.nx * pl.ny;
+  for (int q = 0; q < 2; ++q) {
+    const long long col = tx + cx, row = ty + cy + 4 * q;
+    if (col >= pl.nx || row >= pl.ny) continue;
+    const long long pix = row * pl.nx + col;
+    if (kHolo) {
+      const zd t[3] = {mk(e[q][0].x, e[q][0].y), mk(e[q][1].x, e[q][1].y),
+                       mk(e[q][2].x, e[q][2].y)};
+      reinterpret_cast<double*>(out)[size_t(item) * npts + pix] = intensity<double>(t);
+    } else {
+      double2* o = reinterpret_cast<double2*>(out) + size_t(item) * 3 * npts;
+      for (int c = 0; c < 3; ++c) o[c * npts + pix] = e[q][c];
+    }
+  }
+}
+
 // The same from an explicit pixel list in the plane (points [3][npts]; the
 // plan's grid is its bounding box): one thread per pixel, the coefficients
 // of its own intervals read through the caches.  The values are the grid
@@ -540,8 +674,14 @@ size_t radial_buffer(double spacing) {
 
 size_t up256(size_t v) { return (v + 255) / 256 * 256; }
 
-size_t table_bytes(int nparticles, int intervals) {
-  return up256(sizeof(float) * RADIAL_REC * size_t(nparticles) * size_t(intervals));
+size_t radial_buffer64(double spacing) {  // double2
+  const double w = kTile - 1, h = kTileH64 - 1;
+  return (size_t(sqrt(w * w + h * h) / spacing) + 7) * (RADIAL_REC64 / 2);
+}
+
+size_t table_bytes(int nparticles, int intervals, bool fp64) {
+  const size_t rec = fp64 ? sizeof(double) * RADIAL_REC64 : sizeof(float) * RADIAL_REC;
+  return up256(rec * size_t(nparticles) * size_t(intervals));
 }
 
 size_t node_bytes(int nparticles, int intervals) {
@@ -560,16 +700,17 @@ int grid_common(bool holo, const lmb_grid* grid, const lmb_sphere* spheres,
   if (nitems == 0 || grid->nx == 0 || grid->ny == 0 || (points && npts == 0))
     return LMB_OK;
   if (!spheres || !item_start || !ab || !nmax || !out || intervals < 1) return LMB_ERR_ARG;
-  if (!(flags & LMB_CARTESIAN) || (flags & LMB_FP64)) return LMB_ERR_UNSUPPORTED;
+  const bool fp64 = flags & LMB_FP64;
+  if (!(flags & LMB_CARTESIAN) || (fp64 && points)) return LMB_ERR_UNSUPPORTED;
   if (!isfinite(aberr) || !(k > 0.) || nparticles > 65535 || nitems > 65535)
     return LMB_ERR_ARG;
   const long long tx = (grid->nx + kTile - 1) / kTile, ty = (grid->ny + kTile - 1) / kTile;
   if (tx > 0x7fffffffLL || ty > 65535 || (npts + kListThreads - 1) / kListThreads > 0x7fffffffLL)
     return LMB_ERR_ARG;
-  if (!workspace || workspace_bytes < lmb_radial_workspace_bytes(nparticles, intervals))
+  if (!workspace || workspace_bytes < lmb_radial_workspace_bytes(nparticles, intervals, flags))
     return LMB_ERR_WORKSPACE;
   RadialPlan pl;
-  pl.spacing = radial_spacing(k);
+  pl.spacing = radial_spacing(k, fp64);
   if (!(pl.spacing > 0.)) return LMB_ERR_UNSUPPORTED;
   pl.x0 = grid->x0;
   pl.y0 = grid->y0;
@@ -581,19 +722,43 @@ int grid_common(bool holo, const lmb_grid* grid, const lmb_sphere* spheres,
   pl.inv_half = float(2. / pl.spacing);
   pl.intervals = intervals;
   pl.flags = flags;
-  const RadialMatrix A = radial_matrix();
   float* table = reinterpret_cast<float*>(workspace);
+  double* table64 = reinterpret_cast<double*>(workspace);
   double* nodes = reinterpret_cast<double*>(reinterpret_cast<char*>(workspace) +
-                                            table_bytes(nparticles, intervals));
+                                            table_bytes(nparticles, intervals, false));
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (nparticles > 0) {
     const size_t smem = sizeof(double) * RADIAL_FUNCS * kNodeThreads +
                         sizeof(Quad<double>) * 2 * (size_t(nmax_cap) + 1);
-    LMB_CK(smem_attr((const void*)k_radial_table, smem));
     const dim3 g(unsigned((intervals + kChunk - 1) / kChunk), unsigned(nparticles));
-    k_radial_table<<<g, kNodeThreads, smem, st>>>(
-        pl, A, spheres, reinterpret_cast<const zd*>(ab), nmax, nmax_cap + 1, table, nodes);
+    const zd* abz = reinterpret_cast<const zd*>(ab);
+    if (fp64) {
+      auto fn = k_radial_table<double, RADIAL_COEFS64>;
+      LMB_CK(smem_attr((const void*)fn, smem));
+      fn<<<g, kNodeThreads, smem, st>>>(pl, radial_matrix<RADIAL_COEFS64>(), spheres, abz, nmax,
+                                        nmax_cap + 1, table64, nullptr);
+    } else {
+      auto fn = k_radial_table<float, RADIAL_COEFS>;
+      LMB_CK(smem_attr((const void*)fn, smem));
+      fn<<<g, kNodeThreads, smem, st>>>(pl, radial_matrix(), spheres, abz, nmax, nmax_cap + 1,
+                                        table, nodes);
+    }
     LMB_CK(cudaGetLastError());
+  }
+  if (fp64) {
+    const long long rows = (grid->ny + kTileH64 - 1) / kTileH64;
+    const size_t buffer = radial_buffer64(pl.spacing);
+    // two buffers, or one where k is so large that they do not fit
+    const int stages = 2 * sizeof(double2) * buffer <= kSmemLimit ? 2 : 1;
+    const size_t smem = stages * sizeof(double2) * buffer;
+    auto fn = holo ? k_field_radial64<true> : k_field_radial64<false>;
+    if (smem > kSmemLimit || rows > 65535) return LMB_ERR_UNSUPPORTED;
+    LMB_CK(smem_attr((const void*)fn, smem));
+    const dim3 g{unsigned(tx), unsigned(rows), unsigned(nitems)};
+    fn<<<g, kPixThreads, smem, st>>>(pl, spheres, item_start, table64, int(buffer),
+                                   stages, out);
+    LMB_CK(cudaGetLastError());
+    return LMB_OK;
   }
   if (points) {
     auto list = holo ? k_points_radial<true> : k_points_radial<false>;
@@ -634,13 +799,17 @@ int lmb_grid_probe(const double* coords, long long npts, unsigned long long* out
 int lmb_radial_intervals(const lmb_grid* grid, long long npts, const lmb_sphere* spheres,
                          int n, double k, double magnification, int flags, double aberration) {
   if (!grid || !spheres || n < 1 || grid->nx < 1 || grid->ny < 1) return 0;
-  if (!(flags & LMB_CARTESIAN) || (flags & LMB_FP64)) return 0;
+  if (!(flags & LMB_CARTESIAN)) return 0;
+  const bool fp64 = flags & LMB_FP64;
   if (!(k > 0.) || !isfinite(k) || !(magnification > 0.) || !isfinite(aberration)) return 0;
   if (!isfinite(grid->x0) || !isfinite(grid->y0) || !isfinite(grid->z)) return 0;
-  const double spacing = radial_spacing(k);
+  const double spacing = radial_spacing(k, fp64);
   if (!(spacing > 0.)) return 0;
   // a tile's intervals fit in shared memory
-  if (kStages * sizeof(float4) * radial_buffer(spacing) > kSmemLimit) return 0;
+  if ((fp64 ? sizeof(double2) * radial_buffer64(spacing)
+            : kStages * sizeof(float4) * radial_buffer(spacing)) > kSmemLimit)
+    return 0;
+  if (fp64 && grid->ny > 65535LL * kTileH64) return 0;
   double far = 0.;
   for (int i = 0; i < n; ++i) {
     const lmb_sphere& s = spheres[i];
@@ -661,9 +830,10 @@ int lmb_radial_intervals(const lmb_grid* grid, long long npts, const lmb_sphere*
   return count;
 }
 
-size_t lmb_radial_workspace_bytes(int nparticles, int intervals) {
+size_t lmb_radial_workspace_bytes(int nparticles, int intervals, int flags) {
   if (nparticles < 0 || intervals < 1) return 0;
-  return table_bytes(nparticles, intervals) + node_bytes(nparticles, intervals);
+  if (flags & LMB_FP64) return table_bytes(nparticles, intervals, true);
+  return table_bytes(nparticles, intervals, false) + node_bytes(nparticles, intervals);
 }
 
 int lmb_field_grid(const lmb_grid* grid, const double* points, long long npts,

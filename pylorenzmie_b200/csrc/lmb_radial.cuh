@@ -42,6 +42,14 @@ enum {
 // FP32 rounding of its coefficients.  Measured against the oracle over radii
 // of 0.4-24 um from 2 px above the sphere on.
 #define RADIAL_SPACING 0.6
+// The same for FP64 images: at half the spacing the 17-point interpolant is
+// off by at most 1e-14, and a polynomial of degree 8 by 2 (0.3 / 4)^9 / 9! =
+// 4e-16, of a component.
+#define RADIAL_SPACING64 0.3
+enum {
+  RADIAL_COEFS64 = 9,
+  RADIAL_REC64 = RADIAL_FUNCS * RADIAL_COEFS64  // doubles per interval: 27 double2, odd
+};
 // Distance of the plane from the sphere's surface, k d.
 #define RADIAL_CLEARANCE 1.8
 // The distance (pixels) that stands for the axis itself, where V and Z are
@@ -51,9 +59,11 @@ enum {
 #define RADIAL_AXIS 1e-4
 // Row c: the weights of the nodes in the coefficient of t^c, t = (rho - rho_i)
 // / (half a spacing).
-struct RadialMatrix {
-  double m[RADIAL_COEFS][RADIAL_TAPS];
+template <int NC = RADIAL_COEFS>
+struct RadialMatrixN {
+  double m[NC][RADIAL_TAPS];
 };
+typedef RadialMatrixN<> RadialMatrix;
 
 // The Lagrange weights of the RADIAL_TAPS nodes around one of them at
 // offset x (in spacings).
@@ -80,36 +90,37 @@ LMB_HD void radial_weights(double x, double* w) {
 }
 
 // Coefficients in powers of t of the polynomial through values at the
-// Chebyshev points t_i = cos(pi (i + 1/2) / RADIAL_COEFS): row c, column i.
+// Chebyshev points t_i = cos(pi (i + 1/2) / NC): row c, column i.
+template <int NC>
 struct RadialPowers {
-  double t[RADIAL_COEFS];
-  double m[RADIAL_COEFS][RADIAL_COEFS];
+  double t[NC];
+  double m[NC][NC];
   RadialPowers() {
-    const int n = RADIAL_COEFS;
     const double pi = 3.141592653589793;
-    double tq[RADIAL_COEFS][RADIAL_COEFS] = {};  // T_q in powers
+    double tq[NC][NC] = {};  // T_q in powers
     tq[0][0] = tq[1][1] = 1.;
-    for (int q = 2; q < n; ++q)
-      for (int p = 0; p < n; ++p)
+    for (int q = 2; q < NC; ++q)
+      for (int p = 0; p < NC; ++p)
         tq[q][p] = (p ? 2. * tq[q - 1][p - 1] : 0.) - tq[q - 2][p];
-    for (int i = 0; i < n; ++i) {
-      t[i] = cos(pi * (i + 0.5) / n);
-      for (int p = 0; p < n; ++p) {
+    for (int i = 0; i < NC; ++i) {
+      t[i] = cos(pi * (i + 0.5) / NC);
+      for (int p = 0; p < NC; ++p) {
         m[p][i] = 0.;
-        for (int q = 0; q < n; ++q)
-          m[p][i] += (q ? 2. : 1.) / n * cos(pi * q * (i + 0.5) / n) * tq[q][p];
+        for (int q = 0; q < NC; ++q)
+          m[p][i] += (q ? 2. : 1.) / NC * cos(pi * q * (i + 0.5) / NC) * tq[q][p];
       }
     }
   }
 };
 
-inline RadialMatrix radial_matrix() {
-  static const RadialPowers P;
-  RadialMatrix A = {};
-  for (int i = 0; i < RADIAL_COEFS; ++i) {
+template <int NC = RADIAL_COEFS>
+inline RadialMatrixN<NC> radial_matrix() {
+  static const RadialPowers<NC> P;
+  RadialMatrixN<NC> A = {};
+  for (int i = 0; i < NC; ++i) {
     double w[RADIAL_TAPS];
     radial_weights(0.5 * P.t[i], w);
-    for (int c = 0; c < RADIAL_COEFS; ++c)
+    for (int c = 0; c < NC; ++c)
       for (int j = 0; j < RADIAL_TAPS; ++j) A.m[c][j] += P.m[c][i] * w[j];
   }
   return A;

@@ -199,11 +199,10 @@ class LorenzMie(LMObject):
 
     def _items(self, particle_lists, cartesian, bohren, field):
         sp, item_start, ab, _, nmax, cap, rec = self._prepare(particle_lists)
-        if not self.double_precision and cartesian and len(rec) and \
-                self._grid is not None:
-            out = K.on_grid(self._grid, self._coords, rec, sp, item_start, ab, nmax, cap,
-                            self.instrument, cartesian, bohren,
-                            self._aberration(), field)
+        if cartesian and len(rec) and self._grid is not None:
+            out = K.on_grid(self._grid, self._coords, rec, sp, item_start, ab,
+                            nmax, cap, self.instrument, cartesian, bohren,
+                            self._aberration(), field, self.double_precision)
             if out is not None:
                 return out
         direct = K.field if field else K.hologram

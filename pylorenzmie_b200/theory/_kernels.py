@@ -251,36 +251,39 @@ def make_grid(z, npts, probed):
 
 
 def on_grid(grid, coords, records, spheres, item_start, ab, nmax, cap,
-            instrument, cartesian, bohren, aberration, field=False):
-    '''(nitems, npts) float32 holograms, or with ``field`` (nitems, 3,
-    npts) complex64 fields, of pixels in one plane (make_grid's result)
-    from radial tables (lmb_hologram_grid, lmb_field_grid); None where they
-    do not apply.  records: the spheres' host records.'''
+            instrument, cartesian, bohren, aberration, field=False,
+            fp64=False):
+    '''(nitems, npts) holograms, or with ``field`` (nitems, 3, npts)
+    fields, of pixels in one plane (make_grid's result) from radial tables
+    (lmb_hologram_grid, lmb_field_grid), with ``fp64`` in 64 bits; None
+    where they do not apply.  records: the spheres' host records.'''
     grid, full = grid
     npts = coords.shape[1]
     lib = _native.load()
     k = float(instrument.wavenumber())
-    flags = _flags(cartesian, bohren, False)
+    flags = _flags(cartesian, bohren, fp64)
     n = len(records)
     # Images of less than 200x200 pixels: their direct sums take as long as
     # the tables (10 us) in one launch fewer.  Particles are the table
     # kernel's grid rows.
-    if n > 65535 or (full and npts < 40000):
+    if n > 65535 or (full and npts < 40000) or (fp64 and not full):
         return None
     intervals = lib.lmb_radial_intervals(
         grid, npts, records.ctypes.data, n, k, float(instrument.magnification),
         flags, float(aberration))
     if not intervals:
         return None
-    nbytes = lib.lmb_radial_workspace_bytes(n, intervals)
+    nbytes = lib.lmb_radial_workspace_bytes(n, intervals, flags)
     if nbytes > RADIAL_WORKSPACE_LIMIT:
         return None
     dev = spheres.device
     nitems = item_start.shape[0] - 1
     if field:
-        out = torch.empty((nitems, 3, npts), dtype=torch.complex64, device=dev)
+        out = torch.empty((nitems, 3, npts), device=dev,
+                          dtype=torch.complex128 if fp64 else torch.complex64)
     else:
-        out = torch.empty((nitems, npts), dtype=torch.float32, device=dev)
+        out = torch.empty((nitems, npts), device=dev,
+                          dtype=torch.float64 if fp64 else torch.float32)
     ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
     name = 'lmb_field_grid' if field else 'lmb_hologram_grid'
     _native.check(getattr(lib, name)(

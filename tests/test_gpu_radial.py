@@ -66,6 +66,8 @@ def test_grid_images_match_fp64(shape, n, inst, opt, monkeypatch):
     m32 = grid_model(shape, spheres, instrument=instrument, **opt)
     m64 = grid_model(shape, spheres, instrument=instrument,
                      double_precision=True, **opt)
+    m64._coords
+    m64._grid_dev = (None,)                     # direct sums
     h32 = m32.hologram(bohren=bohren)
     h64 = m64.hologram(bohren=bohren)
     assert taken and taken[0] is not None       # the tables were used
@@ -74,6 +76,41 @@ def test_grid_images_match_fp64(shape, n, inst, opt, monkeypatch):
     scale = sum(np.abs(m64.scattered_field(s, bohren=bohren)).max()
                 for s in spheres)
     assert np.abs(f32 - f64).max() <= 1e-6 * scale
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('shape,n,inst,opt', CASES)
+def test_fp64_grid_images_match_direct_sums(shape, n, inst, opt, monkeypatch):
+    '''FP64 tables: 1e-12 of the sum of the particles' largest components
+    (interpolation 1e-14, and the rounding of phases of ~10^3 rad at the
+    nodes and at the pixels, ~1e-13 each).'''
+    from pylorenzmie_b200 import Instrument, workloads
+    from pylorenzmie_b200.theory import _kernels as K
+    opt = dict(opt)
+    p = rows(n, shape, seed=n + len(opt), below=opt.pop('below', False))
+    instrument = Instrument(**inst)
+    if inst:
+        p[:, 2] = np.sign(p[:, 2]) * (p[:, 3] / instrument.magnification +
+                                      4. / instrument.wavenumber() + 30.)
+    bohren = opt.pop('bohren', True)
+    spheres = workloads.spheres(p)
+    taken = []
+    on_grid = K.on_grid
+    monkeypatch.setattr(K, 'on_grid', lambda *a: taken.append(on_grid(*a))
+                        or taken[-1])
+    m = grid_model(shape, spheres, instrument=instrument,
+                   double_precision=True, **opt)
+    d = grid_model(shape, spheres, instrument=instrument,
+                   double_precision=True, **opt)
+    d._coords
+    d._grid_dev = (None,)                       # direct sums
+    f, ref = m.field(bohren=bohren), d.field(bohren=bohren)
+    assert taken and taken[0] is not None
+    scale = sum(np.abs(d.scattered_field(s, bohren=bohren)).max()
+                for s in spheres)
+    assert np.abs(f - ref).max() <= 1e-12 * scale
+    h, ref = m.hologram(bohren=bohren), d.hologram(bohren=bohren)
+    assert np.abs(h - ref).max() <= 2e-12 * scale * (1. + scale)
 
 
 @pytest.mark.gpu
@@ -87,7 +124,7 @@ def test_grid_batch_items():
     h64 = grid_model(shape, lists[0],
                      double_precision=True).batch_hologram(lists)
     assert np.abs(h32 - h64).max() <= 2e-5
-    assert np.all(h32[1] == 1.)
+    assert np.all(h32[1] == 1.) and np.all(h64[1] == 1.)
 
 
 @pytest.mark.gpu
@@ -158,7 +195,7 @@ def test_rule_on_the_host():
     assert intervals(nx=3, ny=3) == 0               # too few pixels
     assert intervals(x0=-9000.) == 0                # too far
     assert intervals(flags=_native.LMB_BOHREN) == 0
-    assert intervals(flags=cart | _native.LMB_FP64) == 0
+    assert intervals(flags=cart | _native.LMB_FP64) > intervals()
     assert intervals(aberration=1e4) == 0
     assert intervals(aberration=20.) > 0
     assert intervals(z_p=np.nan) == 0 and intervals(x_p=np.inf) == 0
