@@ -173,6 +173,8 @@ typedef struct lmb_grid {
 } lmb_grid;
 int lmb_grid_probe(const double *coords, long long npts,
                    unsigned long long *out, void *stream);
+/* The same of coordinates in host memory, out in host memory too. */
+int lmb_grid_probe_host(const double *coords, long long npts, long long *out);
 int lmb_radial_intervals(const lmb_grid *grid, long long npts,
                          const lmb_sphere *spheres, int n, double k, double magnification, int flags,
                          double aberration);
@@ -191,6 +193,34 @@ int lmb_hologram_grid(const lmb_grid *grid, const double *points,
                       int nmax_cap, double k, int flags, double aberration,
                       void *out, void *workspace, size_t workspace_bytes,
                       void *stream);
+
+/*
+ * Fields and holograms from sphere records in host memory, in two calls:
+ * lmb_render_plan (host only) checks the spheres (LMB_ERR_ARG: not finite or
+ * a_p <= 0; LMB_ERR_NMAX: plan->nmax_cap above LMB_NMAX_LIMIT), chooses
+ * tables or direct sums and lays out the workspace; lmb_render_run uploads
+ * the records and offsets (host_item_start [nitems + 1]), computes the
+ * coefficients and renders.  grid: the pixels' layout, NULL if they are not
+ * in one plane; points nonzero: they are a list in that plane, not the grid.
+ * coords: device, [3][npts].  field nonzero: lmb_field's output, else
+ * lmb_hologram's.  The host arrays are read before the call returns.
+ */
+typedef struct lmb_render {
+  int nmax_cap, intervals;
+  size_t spheres, ab, nmax, tables, workspace_bytes;
+} lmb_render;
+int lmb_render_plan(const lmb_grid *grid, int points, long long npts,
+                    const lmb_sphere *host_spheres, int n, int nitems,
+                    double n_m, double wavelength, double k,
+                    double magnification, int flags, double aberration,
+                    lmb_render *plan);
+int lmb_render_run(const lmb_render *plan, const lmb_grid *grid, int points,
+                   const double *coords, long long npts,
+                   const lmb_sphere *host_spheres, int n,
+                   const int *host_item_start, int nitems, double n_m,
+                   double wavelength, double k, int flags, double aberration,
+                   int field, void *out, void *workspace,
+                   size_t workspace_bytes, void *stream);
 
 /*
  * chi^2 = sum over pixels of ((hologram - data) / noise)^2 for each of

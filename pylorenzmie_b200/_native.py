@@ -61,6 +61,13 @@ class Grid(ctypes.Structure):
                 ('ny', ctypes.c_longlong)]
 
 
+class Render(ctypes.Structure):
+    _fields_ = [('nmax_cap', ctypes.c_int), ('intervals', ctypes.c_int),
+                ('spheres', ctypes.c_size_t), ('ab', ctypes.c_size_t),
+                ('nmax', ctypes.c_size_t), ('tables', ctypes.c_size_t),
+                ('workspace_bytes', ctypes.c_size_t)]
+
+
 class LMBError(RuntimeError):
     '''A non-zero status from the CUDA library.'''
 
@@ -90,6 +97,7 @@ _SIGNATURES = {
     'lmb_hologram_aberrated': (_i, [_vp, _ll, _vp, _vp, _i, _vp, _vp, _i,
                                     _d, _i, _d, _vp, _vp]),
     'lmb_grid_probe': (_i, [_vp, _ll, _vp, _vp]),
+    'lmb_grid_probe_host': (_i, [_vp, _ll, _vp]),
     'lmb_radial_intervals': (_i, [ctypes.POINTER(Grid), _ll, _vp, _i, _d, _d,
                                   _i, _d]),
     'lmb_radial_workspace_bytes': (_sz, [_i, _i, _i]),
@@ -99,6 +107,11 @@ _SIGNATURES = {
     'lmb_hologram_grid': (_i, [ctypes.POINTER(Grid), _vp, _ll, _vp, _vp, _i,
                                _i, _i, _vp, _vp, _i, _d, _i, _d, _vp, _vp,
                                _sz, _vp]),
+    'lmb_render_plan': (_i, [ctypes.POINTER(Grid), _i, _ll, _vp, _i, _i, _d, _d,
+                             _d, _d, _i, _d, ctypes.POINTER(Render)]),
+    'lmb_render_run': (_i, [ctypes.POINTER(Render), ctypes.POINTER(Grid), _i,
+                            _vp, _ll, _vp, _i, _vp, _i, _d, _d, _d, _i, _d,
+                            _i, _vp, _vp, _sz, _vp]),
     'lmb_jacobian': (_i, [_vp, _ll, _vp, _i, _vp, _vp, _vp, _i, _d, _i, _vp,
                           _vp, _vp]),
     'lmb_de_trial': (_i, [_i, _i, _vp, _i, _i, _vp, _vp, _vp, _i, _d, _d,

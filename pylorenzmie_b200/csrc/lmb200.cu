@@ -668,6 +668,134 @@ int lmb_hologram_vjp_grid(const lmb_grid* grid, const double* points, long long 
   return LMB_OK;
 }
 
+int lmb_render_plan(const lmb_grid* grid, int points, long long npts,
+                    const lmb_sphere* host_spheres, int n, int nitems, double n_m,
+                    double wavelength, double k, double magnification, int flags,
+                    double aberration, lmb_render* plan) {
+  if (n < 0 || nitems < 0 || npts < 0 || !plan || (n > 0 && !host_spheres)) return LMB_ERR_ARG;
+  if (!(wavelength > 0.) || !(n_m > 0.)) return LMB_ERR_ARG;
+  int cap = 1;
+  for (int i = 0; i < n; ++i) {
+    const lmb_sphere& s = host_spheres[i];
+    if (!isfinite(s.x_p) || !isfinite(s.y_p) || !isfinite(s.z_p) || !isfinite(s.a_p) ||
+        !isfinite(s.n_p) || !isfinite(s.k_p) || !(s.a_p > 0.))
+      return LMB_ERR_ARG;
+    // mie_setup's n_max; doubles beyond int's range need too many orders
+    const double x = 2. * 3.141592653589793 / wavelength * n_m * s.a_p;
+    const zd m = mk(s.n_p / n_m, s.k_p / n_m);
+    if (!(x < 1e7) || !(hypot(x * m.re, x * m.im) < 1e9)) {
+      plan->nmax_cap = 1 << 30;
+      return LMB_ERR_NMAX;
+    }
+    cap = std::max(cap, wiscombe_yang(x, m) + 2);
+  }
+  plan->nmax_cap = cap;
+  if (cap > LMB_NMAX_LIMIT) return LMB_ERR_NMAX;
+  // Tables from 30 000 pixels times particles on: below, the direct sums
+  // take no longer (8 us for a 64x64 image of one sphere, as the tables) and
+  // are one launch fewer.
+  plan->intervals = 0;
+  if (grid && !(points && (flags & LMB_FP64)) && n <= 65535 &&
+      (points || double(npts) * n >= 30000.))
+    plan->intervals = lmb_radial_intervals(grid, npts, host_spheres, n, k, magnification, flags,
+                                           aberration);
+  size_t tables = plan->intervals ? lmb_radial_workspace_bytes(n, plan->intervals, flags) : 0;
+  if (tables > (size_t(4) << 30)) {
+    plan->intervals = 0;
+    tables = 0;
+  }
+  size_t off = 0;
+  auto take = [&](size_t bytes) {
+    const size_t o = off;
+    off = align_up(off + bytes, 256);
+    return o;
+  };
+  plan->spheres = take(sizeof(lmb_sphere) * size_t(n) + sizeof(int) * (size_t(nitems) + 1));
+  plan->ab = take(sizeof(zd) * 2 * (size_t(cap) + 1) * std::max(n, 1));
+  plan->nmax = take(sizeof(int) * 2 * size_t(std::max(n, 1)));
+  plan->tables = take(tables);
+  plan->workspace_bytes = off;
+  return LMB_OK;
+}
+
+}  // extern "C"
+
+namespace {
+// Small host arrays reach the device as a kernel's parameters: no pinned
+// buffer, no copy engine, and no wait for the stream.
+template <int BYTES>
+struct Upload {
+  unsigned int w[BYTES / 4];
+};
+template <int BYTES>
+__global__ void k_upload(const __grid_constant__ Upload<BYTES> u, int words, unsigned int* dst) {
+  for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = u.w[i];
+}
+template <int BYTES>
+cudaError_t upload_part(const unsigned int* src, int words, unsigned int* dst, cudaStream_t st) {
+  Upload<BYTES> u;
+  memcpy(u.w, src, size_t(words) * 4);
+  k_upload<BYTES><<<1, 256, 0, st>>>(u, words, dst);
+  return cudaGetLastError();
+}
+cudaError_t upload(const void* src, size_t bytes, void* dst, cudaStream_t st) {
+  const unsigned int* s = static_cast<const unsigned int*>(src);
+  unsigned int* d = static_cast<unsigned int*>(dst);
+  for (size_t left = bytes / 4; left;) {
+    const int n = int(std::min<size_t>(left, 4096));
+    const cudaError_t e = n <= 128    ? upload_part<512>(s, n, d, st)
+                          : n <= 896  ? upload_part<3584>(s, n, d, st)
+                                      : upload_part<16384>(s, n, d, st);
+    if (e != cudaSuccess) return e;
+    s += n;
+    d += n;
+    left -= n;
+  }
+  return cudaSuccess;
+}
+}  // namespace
+
+extern "C" {
+
+int lmb_render_run(const lmb_render* plan, const lmb_grid* grid, int points,
+                   const double* coords, long long npts, const lmb_sphere* host_spheres, int n,
+                   const int* host_item_start, int nitems, double n_m, double wavelength,
+                   double k, int flags, double aberration, int field, void* out,
+                   void* workspace, size_t workspace_bytes, void* stream) {
+  if (!plan || n < 0 || nitems < 0 || npts < 0 || bad_cap(plan->nmax_cap)) return LMB_ERR_ARG;
+  if (nitems == 0 || npts == 0) return LMB_OK;
+  if ((n > 0 && !host_spheres) || !host_item_start || !out) return LMB_ERR_ARG;
+  if (!workspace || workspace_bytes < plan->workspace_bytes) return LMB_ERR_WORKSPACE;
+  cudaStream_t st = as_stream(stream);
+  char* ws = static_cast<char*>(workspace);
+  lmb_sphere* spheres = reinterpret_cast<lmb_sphere*>(ws + plan->spheres);
+  int* item_start = reinterpret_cast<int*>(spheres + n);
+  double* ab = reinterpret_cast<double*>(ws + plan->ab);
+  int* nmax = reinterpret_cast<int*>(ws + plan->nmax);
+  // records and offsets, which lie side by side, in one launch where they fit
+  const size_t rec = sizeof(lmb_sphere) * size_t(n), off = sizeof(int) * (size_t(nitems) + 1);
+  unsigned char both[3584];
+  if (rec + off <= sizeof(both)) {
+    if (n) memcpy(both, host_spheres, rec);
+    memcpy(both + rec, host_item_start, off);
+    LMB_CK(upload(both, rec + off, spheres, st));
+  } else {
+    LMB_CK(upload(host_spheres, rec, spheres, st));
+    LMB_CK(upload(host_item_start, off, item_start, st));
+  }
+  int status = lmb_sphere_ab(spheres, n, n_m, wavelength, plan->nmax_cap, ab, nullptr, nmax,
+                             nmax + n, stream);
+  if (status != LMB_OK) return status;
+  if (plan->intervals) {
+    auto fn = field ? lmb_field_grid : lmb_hologram_grid;
+    return fn(grid, points ? coords : nullptr, npts, spheres, item_start, nitems, n,
+              plan->intervals, ab, nmax, plan->nmax_cap, k, flags, aberration, out,
+              ws + plan->tables, plan->workspace_bytes - plan->tables, stream);
+  }
+  return field_common(!field, coords, npts, spheres, item_start, nitems, ab, nmax,
+                      plan->nmax_cap, k, flags, out, stream, aberration);
+}
+
 int lmb_fit_tile_config(int index, int* threads, int* pixels_per_thread,
                         int* min_blocks) {
   if (index < 0 || index >= kNumEvalShapes) return LMB_ERR_ARG;

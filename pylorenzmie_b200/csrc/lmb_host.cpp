@@ -2,8 +2,10 @@
 // many crops to float32 into one (pinned) staging buffer, on a persistent
 // pool of native threads so that the caller's interpreter lock is not
 // involved and small portions of a streamed batch convert at full speed.
+#include <math.h>
 #include <stddef.h>
 #include <stdint.h>
+#include <string.h>
 
 #include <algorithm>
 #include <condition_variable>
@@ -168,6 +170,31 @@ extern "C" int lmb_pack_crops(const void* const* sources,
     return LMB_OK;
   }
   pool().run(job);
+  return LMB_OK;
+}
+
+// lmb_grid_probe of coordinates in host memory.
+extern "C" int lmb_grid_probe_host(const double* coords, long long npts, long long* out) {
+  if (npts < 1 || !coords || !out) return LMB_ERR_ARG;
+  const double *x = coords, *y = coords + npts, *z = coords + 2 * npts;
+  long long nx = 0;
+  while (nx < npts && y[nx] == y[0]) ++nx;
+  if (nx == 0) nx = npts;  // y[0] is NaN
+  long long off = 0, plane = 0;
+  double b[4] = {x[0], y[0], x[0], y[0]};
+  for (long long r = 0, i = 0; i < npts; ++r)
+    for (long long c = 0; c < nx && i < npts; ++c, ++i) {
+      if (!(x[i] == x[0] + double(c)) || !(y[i] == y[0] + double(r)) || !(z[i] == z[0])) ++off;
+      if (!isfinite(x[i]) || !isfinite(y[i]) || !isfinite(z[i]) || z[i] != z[0]) ++plane;
+      b[0] = std::min(b[0], x[i]);
+      b[1] = std::min(b[1], y[i]);
+      b[2] = std::max(b[2], x[i]);
+      b[3] = std::max(b[3], y[i]);
+    }
+  out[0] = nx;
+  out[1] = off;
+  out[2] = plane;
+  memcpy(out + 3, b, sizeof(b));
   return LMB_OK;
 }
 

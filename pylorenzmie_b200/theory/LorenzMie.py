@@ -43,7 +43,13 @@ def _row(p):
 
 def _records(particles):
     '''SPHERE_DTYPE records (r_p + r_0, a_p, n_p, k_p) of a particle list.'''
-    return np.array([_row(p) for p in particles], dtype=K.SPHERE_DTYPE)
+    if all(type(p) is Sphere for p in particles):
+        rows = [(p.x_p + p.x_0, p.y_p + p.y_0, p.z_p + p.z_0, p.a_p, p.n_p,
+                 p.k_p) for p in particles]
+    else:
+        rows = [_row(p) for p in particles]
+    return np.array(rows, dtype=float).reshape(-1, 6).view(
+        K.SPHERE_DTYPE).reshape(-1)
 
 
 class LorenzMie(LMObject):
@@ -137,11 +143,15 @@ class LorenzMie(LMObject):
         '''The coordinates as pixels of one plane (K.make_grid), or None;
         found once for each device copy of the coordinates.'''
         if self._grid_dev is None:
-            c = self._coords
-            npts = c.shape[1]
-            self._grid_dev = (K.make_grid(
-                self._coordinates[2, 0], npts, K.probe_grid(c).cpu().numpy())
-                if npts else None,)
+            host = self._coordinates
+            npts = host.shape[1]
+            found = None
+            if 0 < npts <= 16384:      # less than the launches would take
+                found = K.probe_host(np.ascontiguousarray(host))
+            elif npts:
+                found = K.probe_grid(self._coords).cpu().numpy()
+            self._grid_dev = (None if found is None else
+                              K.make_grid(host[2, 0], npts, found),)
         return self._grid_dev[0]
 
     # ------------------------------------------------------------------
@@ -198,8 +208,15 @@ class LorenzMie(LMObject):
         return 0.
 
     def _items(self, particle_lists, cartesian, bohren, field):
+        flat = [p for plist in particle_lists for p in plist]
+        if not any(type(p) is not Sphere and K.is_layered(p) for p in flat):
+            coords = self._coords
+            return K.render(self._grid, coords, _records(flat),
+                            [len(pl) for pl in particle_lists],
+                            self.instrument, cartesian, bohren,
+                            self._aberration(), field, self.double_precision)
         sp, item_start, ab, _, nmax, cap, rec = self._prepare(particle_lists)
-        if cartesian and len(rec) and self._grid is not None:
+        if cartesian and self._grid is not None:
             out = K.on_grid(self._grid, self._coords, rec, sp, item_start, ab,
                             nmax, cap, self.instrument, cartesian, bohren,
                             self._aberration(), field, self.double_precision)

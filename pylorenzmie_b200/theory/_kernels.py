@@ -236,6 +236,15 @@ def probe_grid(coords):
     return out
 
 
+def probe_host(coords):
+    '''probe_grid of a host array (3, npts): its values at once.'''
+    out = np.empty(7, dtype=np.int64)
+    _native.check(_native.load().lmb_grid_probe_host(
+        coords.ctypes.data, coords.shape[1], out.ctypes.data),
+        'lmb_grid_probe_host')
+    return out
+
+
 def make_grid(z, npts, probed):
     '''(Grid, whether the pixels are that grid's) of a probed coordinate
     list in the plane z (a numpy int64 array), the grid being a box around
@@ -343,6 +352,47 @@ def hologram_vjp(coords, spheres, ab, dab, nmax, cap, k, gout, bohren=True):
                                        stream_handle(dev)),
                   'lmb_hologram_vjp')
     return grad
+
+
+def render(grid, coords, records, counts, instrument, cartesian, bohren,
+           aberration, field, fp64):
+    '''(nitems, npts) holograms or (nitems, 3, npts) fields of homogeneous
+    spheres given by host records, item i the next counts[i] of them, in two
+    native calls (lmb_render_plan, lmb_render_run).  grid: make_grid's
+    result or None.'''
+    lib = _native.load()
+    dev = coords.device
+    n, nitems, npts = len(records), len(counts), coords.shape[1]
+    n_m, lam = float(instrument.n_m), float(instrument.wavelength)
+    k, aberration = float(instrument.wavenumber()), float(aberration)
+    flags = _flags(cartesian, bohren, fp64)
+    box, full = grid if grid is not None else (None, True)
+    host = records.ctypes.data
+    plan = _native.Render()
+    status = lib.lmb_render_plan(
+        box, not full, npts, host, n, nitems, n_m, lam, k,
+        float(instrument.magnification), flags, aberration, plan)
+    if status == _native.LMB_ERR_ARG and n_m > 0. and lam > 0.:
+        raise ValueError('particle parameters must be finite with a_p > 0')
+    if status == _native.LMB_ERR_NMAX:
+        raise ValueError(f'a particle needs {plan.nmax_cap - 2} partial-wave '
+                         f'orders; the limit is {_native.LMB_NMAX_LIMIT}')
+    _native.check(status, 'lmb_render_plan')
+    start = np.zeros(nitems + 1, dtype=np.int32)
+    np.cumsum(counts, out=start[1:])
+    if field:
+        out = torch.empty((nitems, 3, npts), device=dev,
+                          dtype=torch.complex128 if fp64 else torch.complex64)
+    else:
+        out = torch.empty((nitems, npts), device=dev,
+                          dtype=torch.float64 if fp64 else torch.float32)
+    ws = torch.empty(plan.workspace_bytes, dtype=torch.uint8, device=dev)
+    _native.check(lib.lmb_render_run(
+        plan, box, not full, coords.data_ptr(), npts, host, n,
+        start.ctypes.data, nitems, n_m, lam, k, flags, aberration, field,
+        out.data_ptr(), ws.data_ptr(), plan.workspace_bytes,
+        stream_handle(dev)), 'lmb_render_run')
+    return out
 
 
 def vjp_on_grid(grid, coords, records, spheres, ab, dab, nmax, cap,

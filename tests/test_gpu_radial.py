@@ -18,6 +18,23 @@ def grid_model(shape, particles, **kwargs):
                **kwargs)
 
 
+def uses_tables(model, spheres, bohren):
+    '''Whether lmb_render_plan chooses the tables for these images.'''
+    from pylorenzmie_b200 import _native
+    from pylorenzmie_b200.theory import _kernels as K
+    from pylorenzmie_b200.theory.LorenzMie import _records
+    rec = _records(spheres)
+    inst = model.instrument
+    plan = _native.Render()
+    grid, full = model._grid
+    assert full and _native.load().lmb_render_plan(
+        grid, 0, model.coordinates.shape[1], rec.ctypes.data, len(rec), 1,
+        inst.n_m, inst.wavelength, inst.wavenumber(), inst.magnification,
+        K._flags(True, bohren, model.double_precision), model._aberration(),
+        plan) == _native.LMB_OK
+    return plan.intervals > 0
+
+
 def rows(n, shape, seed, below=False):
     rng = np.random.default_rng(seed)
     p = np.zeros((n, 6))
@@ -48,9 +65,8 @@ CASES = [
 
 @pytest.mark.gpu
 @pytest.mark.parametrize('shape,n,inst,opt', CASES)
-def test_grid_images_match_fp64(shape, n, inst, opt, monkeypatch):
+def test_grid_images_match_fp64(shape, n, inst, opt):
     from pylorenzmie_b200 import Instrument, workloads
-    from pylorenzmie_b200.theory import _kernels as K
     opt = dict(opt)
     p = rows(n, shape, seed=n + len(opt), below=opt.pop('below', False))
     instrument = Instrument(**inst)
@@ -59,10 +75,6 @@ def test_grid_images_match_fp64(shape, n, inst, opt, monkeypatch):
                                       4. / instrument.wavenumber() + 30.)
     bohren = opt.pop('bohren', True)
     spheres = workloads.spheres(p)
-    taken = []
-    on_grid = K.on_grid
-    monkeypatch.setattr(K, 'on_grid', lambda *a: taken.append(on_grid(*a))
-                        or taken[-1])
     m32 = grid_model(shape, spheres, instrument=instrument, **opt)
     m64 = grid_model(shape, spheres, instrument=instrument,
                      double_precision=True, **opt)
@@ -70,7 +82,7 @@ def test_grid_images_match_fp64(shape, n, inst, opt, monkeypatch):
     m64._grid_dev = (None,)                     # direct sums
     h32 = m32.hologram(bohren=bohren)
     h64 = m64.hologram(bohren=bohren)
-    assert taken and taken[0] is not None       # the tables were used
+    assert uses_tables(m32, spheres, bohren)
     assert np.abs(h32 - h64).max() <= 2e-5
     f32, f64 = m32.field(bohren=bohren), m64.field(bohren=bohren)
     scale = sum(np.abs(m64.scattered_field(s, bohren=bohren)).max()
@@ -80,12 +92,11 @@ def test_grid_images_match_fp64(shape, n, inst, opt, monkeypatch):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize('shape,n,inst,opt', CASES)
-def test_fp64_grid_images_match_direct_sums(shape, n, inst, opt, monkeypatch):
+def test_fp64_grid_images_match_direct_sums(shape, n, inst, opt):
     '''FP64 tables: 1e-12 of the sum of the particles' largest components
     (interpolation 1e-14, and the rounding of phases of ~10^3 rad at the
     nodes and at the pixels, ~1e-13 each).'''
     from pylorenzmie_b200 import Instrument, workloads
-    from pylorenzmie_b200.theory import _kernels as K
     opt = dict(opt)
     p = rows(n, shape, seed=n + len(opt), below=opt.pop('below', False))
     instrument = Instrument(**inst)
@@ -94,10 +105,6 @@ def test_fp64_grid_images_match_direct_sums(shape, n, inst, opt, monkeypatch):
                                       4. / instrument.wavenumber() + 30.)
     bohren = opt.pop('bohren', True)
     spheres = workloads.spheres(p)
-    taken = []
-    on_grid = K.on_grid
-    monkeypatch.setattr(K, 'on_grid', lambda *a: taken.append(on_grid(*a))
-                        or taken[-1])
     m = grid_model(shape, spheres, instrument=instrument,
                    double_precision=True, **opt)
     d = grid_model(shape, spheres, instrument=instrument,
@@ -105,7 +112,7 @@ def test_fp64_grid_images_match_direct_sums(shape, n, inst, opt, monkeypatch):
     d._coords
     d._grid_dev = (None,)                       # direct sums
     f, ref = m.field(bohren=bohren), d.field(bohren=bohren)
-    assert taken and taken[0] is not None
+    assert uses_tables(m, spheres, bohren)
     scale = sum(np.abs(d.scattered_field(s, bohren=bohren)).max()
                 for s in spheres)
     assert np.abs(f - ref).max() <= 1e-12 * scale
@@ -136,8 +143,14 @@ def test_grid_probe():
                    np.full((1, 40 * 53), 3.)])
 
     def probe(a):
-        t = torch.from_numpy(np.ascontiguousarray(a)).cuda()
-        return K.make_grid(a[2, 0], a.shape[1], K.probe_grid(t).cpu().numpy())
+        a = np.ascontiguousarray(a)
+        found = K.probe_grid(torch.from_numpy(a).cuda()).cpu().numpy()
+        host = K.probe_host(a)
+        assert found[1] == 0 or host[1] > 0
+        assert (found[2] > 0) == (host[2] > 0)
+        if not found[2]:
+            assert np.array_equal(found, host)
+        return K.make_grid(a[2, 0], a.shape[1], found)
     g, full = probe(c)
     assert full and (g.x0, g.y0, g.z, g.nx, g.ny) == (2.5, -7., 3., 53, 40)
     for j, i, v in ((0, 700, 1e-12), (1, 2119, 1.)):
