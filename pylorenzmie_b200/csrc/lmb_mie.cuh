@@ -13,11 +13,14 @@
 // n_max is treated as locally constant, as the reference's JAX Jacobian does
 // (theory/jaxLorenzMie.py:354-361).
 //
-// The phases are split so that a warp forms the per-order quotients n/z,
-// n/z^2, n/x, n/x^2 on all lanes, runs the two downward recurrences on two
-// lanes and then computes a_n, b_n for all n in parallel.  On the
-// recurrences' dependent chains each complex reciprocal is conj(w)/|w|^2
-// with one reciprocal (recip).
+// Homogeneous spheres run linear forms of the two upward and of the inside's
+// recurrence, which have no reciprocal on their serial chains and leave the
+// quotients to the lanes: mie_inside_waves steps q with
+// D1_n = q_(n-1)/q_n - n/z, mie_psi and mie_zeta step psi and zeta
+// from the medium's D1.  mie_d1_inside (for spheres whose q leaves FP64's
+// range, |m| of a tenth at hundreds of orders) and mie_upward (for layered
+// spheres, whose layers take longer than it beside them) step the
+// logarithmic derivatives themselves.
 #pragma once
 
 #include "lmb_math.cuh"
@@ -168,55 +171,153 @@ LMB_HD void mie_upward(const MieScalars& s, const double* nxs,
   }
 }
 
-// a_n, b_n (out[0], out[1]) and, if dout != 0, their derivatives
+// Start of the downward waves at n_max: they grow by up to the ratio of the
+// waves at n_max and at the origin, which 2^-400 leaves room for.
+#define LMB_MIE_START 3.872591914849318e-121
+
+// Inside, q_n by q_(n-1) = ((2n+1)/z) q_n - q_(n+1) from q_(nmax+1) such
+// that D1_nmax = 0; iz = 1/z.  One thread; two dependent fused multiply-adds
+// an order.
+LMB_HD void mie_inside_waves(int nmax, zd iz, zd* q) {
+  zd q1 = mk(LMB_MIE_START, 0.);
+  zd q0 = (double(nmax) * LMB_MIE_START) * iz;
+  q[nmax] = q1;
+  q[nmax - 1] = q0;
+  double c = 2. * nmax - 1.;
+  for (int n = nmax - 1; n > 0; --n, c -= 2.) {
+    const double wr = c * iz.re, wi = c * iz.im;
+    const zd t = mk(fma(wr, q0.re, fma(-wi, q0.im, -q1.re)),
+                    fma(wr, q0.im, fma(wi, q0.re, -q1.im)));
+    q1 = q0;
+    q0 = t;
+    q[n - 1] = t;
+  }
+}
+
+// Order n's quotient r = q_n / q_(n-1) gives D1_(n-1) = n/z - r, and the
+// tangent's recurrence dD1_(n-1) = r^2 dD1_n - (r^2 + 1) n/z^2 its
+// coefficients rr[n] and d1inz[n-1].
+LMB_HD void mie_inside_order(int n, zd iz, const zd* q, zd* d1in, zd* rr,
+                             zd* d1inz) {
+  const zd r = q[n] * recip(q[n - 1]);
+  d1in[n - 1] = double(n) * iz - r;
+  if (rr == 0) return;
+  const zd r2 = r * r;
+  const zd nz2 = double(n) * (iz * iz);
+  rr[n] = r2;
+  d1inz[n - 1] = -1. * ((r2 + 1.) * nz2);
+}
+
+// The tangent's recurrence, in place over d1inz.  One thread.
+LMB_HD void mie_inside_tangent(int nmax, const zd* rr, zd* d1inz) {
+  zd d = mk(0., 0.);
+  d1inz[nmax] = d;
+  for (int n = nmax; n > 0; --n) {
+    const zd r2 = rr[n], e = d1inz[n - 1];
+    d = mk(fma(r2.re, d.re, fma(-r2.im, d.im, e.re)),
+           fma(r2.re, d.im, fma(r2.im, d.re, e.im)));
+    d1inz[n - 1] = d;
+  }
+}
+
+// psi's factors psi_n / psi_(n-1) = n/x - D1_(n-1) and their d/dx, in place
+// over nx, nx2.
+LMB_HD void mie_psi_order(int n, const double* d1, const double* d1x,
+                          double* nx, double* nx2) {
+  nx[n] = nx[n] - d1[n - 1];
+  nx2[n] = -nx2[n] - d1x[n - 1];
+}
+
+// psi_n and d/dx from its factors t, tx.  One thread; one dependent multiply
+// (psi) and fused multiply-add (psix) an order.
+LMB_HD void mie_psi(int nmax, double sx, double cx, const double* t,
+                    const double* tx, double* psi, double* psix) {
+  double p = sx, px = cx;
+  psi[0] = p;
+  psix[0] = px;
+  for (int n = 1; n <= nmax; ++n) {
+    px = fma(px, t[n], p * tx[n]);
+    p = p * t[n];
+    psi[n] = p;
+    psix[n] = px;
+  }
+}
+
+// 1/psi_n and its negative d/dx.
+LMB_HD void mie_psi_inverse(int n, const double* psi, const double* psix,
+                            double* ip, double* ipx) {
+  const double i = rcp_d(psi[n]);
+  ip[n] = i;
+  ipx[n] = (psix[n] * i) * i;
+}
+
+// One part (0: real, 1: imaginary) of zeta_n and its d/dx, z, zx at stride
+// 2.  With D3_n = D1_n + i/(psi_n zeta_n) the reference's step
+// zeta_(n+1) = zeta_n ((n+1)/x - D3_n) is zeta_n psi_(n+1)/psi_n - i/psi_n
+// for n >= 1, so each part is a real recurrence with one dependent fused
+// multiply-add an order; zeta_1 comes from D3_0 = i.
+LMB_HD void mie_zeta(int nmax, int part, double x, double sx, double cx,
+                     const double* t, const double* tx, const double* ip,
+                     const double* ipx, double* z, double* zx) {
+  const double ix = 1. / x, k = part ? 1. : 0.;
+  // zeta_0 = (sx, -cx) and its d/dx (cx, sx), times 1/x - i
+  const double a0 = part ? -cx : sx, b0 = part ? sx : cx;
+  const double ao = part ? -sx : -cx, bo = part ? -cx : sx;
+  double z0 = fma(a0, ix, ao), x0 = b0 * ix + bo - a0 * (ix * ix);
+  z[0] = a0;
+  zx[0] = b0;
+  z[2] = z0;
+  zx[2] = x0;
+  for (int n = 1; n < nmax; ++n) {
+    x0 = fma(t[n + 1], x0, fma(tx[n + 1], z0, k * ipx[n]));
+    z0 = fma(t[n + 1], z0, -(k * ip[n]));
+    z[2 * (n + 1)] = z0;
+    zx[2 * (n + 1)] = x0;
+  }
+}
+
+// a_n (which = 0) or b_n (which = 1) for 1 <= n <= nmax, and if dout != 0
+// its d/da_p and d/dn_p at dout[0] and dout[2].  Eqs. (5) and (6) differ in
+// the factor of D1 alone: 1/m or m.
+LMB_HD zd mie_coefficient_one(const MieScalars& s, int n, int which,
+                              const zd* d1in, const zd* d1inz,
+                              const double* psi, const double* psix,
+                              const zd* zeta, const zd* zetax, zd* dout) {
+  const double x = s.x;
+  const zd m = s.m;
+  const double nx = double(n) / x;
+  const zd im = recip(m);
+  const zd mu = which ? m : im;
+  const zd ha = d1in[n];
+  const double ps = psi[n], ps1 = psi[n - 1];
+  const zd ze = zeta[n], ze1 = zeta[n - 1];
+  const zd f = ha * mu + nx;
+  const zd idn = recip(f * ze - ze1);
+  const zd v = (f * ps - ps1) * idn;
+  if (dout == 0) return v;
+  const double nx2 = nx / x;
+  const zd hz = d1inz[n];
+  const double psx = psix[n], ps1x = psix[n - 1];
+  const zd zex = zetax[n], ze1x = zetax[n - 1];
+  const zd nu = which ? mk(1., 0.) : -1. * (im * im);  // d mu / dm
+  const zd f_x = (m * hz) * mu - nx2;
+  const zd f_m = (x * hz) * mu + ha * nu;
+  const zd v_x = ((f_x * ps + f * psx - ps1x) - v * (f_x * ze + f * zex - ze1x)) * idn;
+  const zd v_m = (f_m * ps - v * (f_m * ze)) * idn;
+  dout[0] = s.k * v_x;
+  dout[2] = (1. / s.n_m) * v_m;
+  return v;
+}
+
+// Both a_n, b_n (out[0], out[1]) and, if dout != 0, their derivatives
 // dout = {da/da_p, db/da_p, da/dn_p, db/dn_p}, for 1 <= n <= nmax.
 LMB_HD void mie_coefficient(const MieScalars& s, int n, const zd* d1in,
                             const zd* d1inz, const double* psi,
                             const double* psix, const zd* zeta,
                             const zd* zetax, zd* out, zd* dout) {
-  const double x = s.x;
-  const zd m = s.m;
-  const double nx = double(n) / x;
-  const double nx2 = nx / x;
-  const zd ha = d1in[n];
-  const zd hz = d1inz[n];
-  const zd ha_x = m * hz;           // d/dx of D1(m x)
-  const zd ha_m = x * hz;           // d/dm of D1(m x)
-  const double ps = psi[n], ps1 = psi[n - 1];
-  const double psx = psix[n], ps1x = psix[n - 1];
-  const zd ze = zeta[n], ze1 = zeta[n - 1];
-  const zd zex = zetax[n], ze1x = zetax[n - 1];
-
-  // a_n, Eq. (5): fac = Ha/m + n/x
-  const zd im = recip(m);
-  const zd fa = ha * im + nx;
-  const zd numa = fa * ps - ps1;
-  const zd dena = fa * ze - ze1;
-  const zd ida = recip(dena);
-  const zd a = numa * ida;
-  // b_n, Eq. (6): fac = Hb m + n/x
-  const zd fb = ha * m + nx;
-  const zd numb = fb * ps - ps1;
-  const zd denb = fb * ze - ze1;
-  const zd idb = recip(denb);
-  const zd b = numb * idb;
-  out[0] = a;
-  out[1] = b;
-  if (dout == 0) return;
-
-  const zd fa_x = ha_x * im - nx2;
-  const zd fa_m = ha_m * im - ha * (im * im);
-  const zd fb_x = ha_x * m - nx2;
-  const zd fb_m = ha_m * m + ha;
-  const zd a_x = ((fa_x * ps + fa * psx - ps1x) - a * (fa_x * ze + fa * zex - ze1x)) * ida;
-  const zd a_m = (fa_m * ps - a * (fa_m * ze)) * ida;
-  const zd b_x = ((fb_x * ps + fb * psx - ps1x) - b * (fb_x * ze + fb * zex - ze1x)) * idb;
-  const zd b_m = (fb_m * ps - b * (fb_m * ze)) * idb;
-  const double inm = 1. / s.n_m;
-  dout[0] = s.k * a_x;
-  dout[1] = s.k * b_x;
-  dout[2] = inm * a_m;
-  dout[3] = inm * b_m;
+  for (int j = 0; j < 2; ++j)
+    out[j] = mie_coefficient_one(s, n, j, d1in, d1inz, psi, psix, zeta, zetax,
+                                 dout ? dout + j : (zd*)0);
 }
 
 }  // namespace lmb
