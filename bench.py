@@ -325,15 +325,22 @@ def b200_arm(args):
         b['d_params'].copy_(b['d_params0'])
         return _fit.fit_device(b['d_feat'], b['d_data'], None, b['d_params'],
                                B, npix * B, inst, variables, None, b['cap'],
-                               b['start'], stats, tile_config=tile_config)
+                               b['start'], stats, tile_config=tile_config,
+                               reach=b['reach'])
 
-    from pylorenzmie_b200 import autotune
+    # the evaluation kernel as fit_packed chooses it: radial tables where
+    # they apply, else an autotuned launch shape
     b0 = batches[0]
     if args.tile_config is None:
-        tile_config = autotune.tune(b0['packed'], b0['start'], inst,
-                                    variables, b0['cap'], None, dev)
+        tile_config = _fit.evaluation(b0['packed'], b0['start'], inst,
+                                      variables, b0['cap'], None, dev,
+                                      _fit.LARGE, 0.)[0]
     else:
         tile_config = int(args.tile_config)
+    radial = tile_config == _native.LMB_FIT_RADIAL
+    for b in batches:
+        b['reach'] = (int(np.ceil(b['packed'].reach(b['start'])))
+                      if radial else 0)
 
     peak = ctypes.c_double()
     _native.check(lib.lmb_measure_fp32_peak(ctypes.byref(peak),
@@ -373,30 +380,46 @@ def b200_arm(args):
     launches = sum(s.eval_launches for s in stats)
     pixels = sum(s.pixels for s in stats)
     porders = sum(s.pixel_orders for s in stats)
-    flop_per_launch = (292. * porders + 476. * pixels) / launches
     avg_ms = eval_ms / launches
-    achieved = flop_per_launch / (avg_ms * 1e-3) / 1e12
     peak_tf = peak.value / 1e12
-    traffic = None
-    tfile = ROOT / 'profiles' / 'traffic.json'
-    if tfile.exists():
-        try:
-            t = json.loads(tfile.read_text()).get('k_fit_eval')
-            if t:
-                traffic = t['bytes_per_launch_full_batch']
-        except Exception:
-            traffic = None
-    roofline = {'bound': 'fp32', 'achieved': achieved, 'peak': peak_tf,
-                'unit': 'TFLOP/s', 'frac': achieved / peak_tf,
-                'traffic': traffic, 'kernel': 'k_fit_eval',
-                'peak_source': 'measured FP32 FMA throughput of this GPU '
-                               '(lmb_measure_fp32_peak, same run); '
-                               'MEASURED_PEAKS.json has no FP32 CUDA-core '
-                               'figure',
-                'flop_per_launch': flop_per_launch,
-                'avg_launch_ms': avg_ms,
-                'work': '292 FLOP per pixel-order + 476 FLOP per pixel '
-                        '(value + 6-column Jacobian + normal equations)'}
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
+    if radial:
+        # every pixel reads its interval's four pairs of polynomials from
+        # shared memory (192 bytes), which bounds the kernel
+        smem_tb = 192. * pixels / (eval_ms * 1e-3) / 1e12
+        roofline = {'bound': 'shared memory', 'achieved': smem_tb,
+                    'unit': 'TB/s', 'kernel': 'k_fit_eval_radial',
+                    'peak_source': 'SMs x 128 bytes x median SM clock of '
+                                   'this run',
+                    'avg_launch_ms': avg_ms,
+                    'work': '12 16-byte shared-memory loads per pixel; '
+                            '~210 FP32 FLOP per pixel; FP64 order sums at '
+                            'the nodes of the tables',
+                    'pixels_per_launch': pixels / launches,
+                    'node_orders_per_launch': porders / launches}
+    else:
+        flop_per_launch = (292. * porders + 476. * pixels) / launches
+        achieved = flop_per_launch / (avg_ms * 1e-3) / 1e12
+        traffic = None
+        tfile = ROOT / 'profiles' / 'traffic.json'
+        if tfile.exists():
+            try:
+                t = json.loads(tfile.read_text()).get('k_fit_eval')
+                if t:
+                    traffic = t['bytes_per_launch_full_batch']
+            except Exception:
+                traffic = None
+        roofline = {'bound': 'fp32', 'achieved': achieved, 'peak': peak_tf,
+                    'unit': 'TFLOP/s', 'frac': achieved / peak_tf,
+                    'traffic': traffic, 'kernel': 'k_fit_eval',
+                    'peak_source': 'measured FP32 FMA throughput of this GPU '
+                                   '(lmb_measure_fp32_peak, same run); '
+                                   'MEASURED_PEAKS.json has no FP32 CUDA-core '
+                                   'figure',
+                    'flop_per_launch': flop_per_launch,
+                    'avg_launch_ms': avg_ms,
+                    'work': '292 FLOP per pixel-order + 476 FLOP per pixel '
+                            '(value + 6-column Jacobian + normal equations)'}
     gpu_launches = sum(s.kernel_launches for s in stats)
 
     # end to end through the public API with host crops
@@ -461,14 +484,19 @@ def b200_arm(args):
         ns['reference_optimizer_vs_oracle_fit_max_abs'] = \
             ref_opt['max_abs_diff_vs_port']
 
-    # the FP32 peak from the clock: SMs x 128 FP32 lanes x 2 FLOP x MHz
+    # the peaks from the clock: SMs x 128 bytes of shared memory, SMs x 128
+    # FP32 lanes x 2 FLOP
     csum = clocks.summary()
     if csum.get('sm_mhz'):
-        sms = torch.cuda.get_device_properties(dev).multi_processor_count
-        clk_peak = sms * 128 * 2 * csum['sm_mhz'] * 1e6 / 1e12
-        roofline['peak_clock_derived'] = clk_peak
-        roofline['frac_clock_derived'] = achieved / clk_peak
+        hz = csum['sm_mhz'] * 1e6
         roofline['sm_mhz_median'] = csum['sm_mhz']
+        if radial:
+            roofline['peak'] = sms * 128 * hz / 1e12
+            roofline['frac'] = roofline['achieved'] / roofline['peak']
+        else:
+            clk_peak = sms * 128 * 2 * hz / 1e12
+            roofline['peak_clock_derived'] = clk_peak
+            roofline['frac_clock_derived'] = achieved / clk_peak
 
     if world > 1:
         tdist.destroy_process_group()
