@@ -11,8 +11,10 @@ analytic-Jacobian slot ``jac()``/``jac_params`` of jaxLorenzMie
 ``method = 'b200 numpy'`` contains 'numpy', so the reference's own
 Optimizer (analysis/Optimizer.py:54, 64-65) accepts this model as well.
 
-All compute runs in the CUDA library: Mie coefficients in FP64, the
-per-pixel sums in FP32 (``double_precision=True`` selects the FP64 sums).
+All compute runs in the CUDA library: Mie coefficients in FP64; the pixels
+of one plane from tables of FP64 sums over their distance from each sphere's
+axis, others by FP32 sums of their own (``double_precision=True`` selects
+FP64 throughout).
 Results come back as numpy float64/complex128 by default, like the
 reference; ``device=True`` returns the CUDA tensor instead (the precedent
 of cupyLorenzMie, theory/cupyLorenzMie.py:80, 100).

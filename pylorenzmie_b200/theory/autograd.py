@@ -2,11 +2,13 @@
 
 ``hologram(params, coordinates, instrument)`` returns the (B, npts) FP32
 holograms of B single spheres, params (B, 6) = (x_p, y_p, z_p, a_p, n_p,
-k_p).  Its backward pass is the hand-written VJP kernel
-(``lmb_hologram_vjp``): it recomputes the Bessel and angular recurrences
-pixel by pixel in forward mode and reduces g * dH/dparam over the pixels,
-so nothing per order or per pixel is stored between forward and backward
-(only the O(n_max) Mie coefficients and their parameter derivatives).
+k_p).  Its backward pass is a hand-written VJP kernel that reduces
+g * dH/dparam over the pixels, from radial tables of the hologram's
+derivatives where the pixels lie in a plane clear of the spheres
+(``lmb_hologram_vjp_grid``), else from recurrences run again pixel by pixel
+(``lmb_hologram_vjp``).  Nothing per order or per pixel is stored between
+forward and backward (only the O(n_max) Mie coefficients and their parameter
+derivatives).
 ``jacobian`` returns the full per-pixel 6-column Jacobian instead.
 
 No reference counterpart runs here: the reference torch backend is not
