@@ -351,22 +351,30 @@ static int chi2_launch(const double* coords, long long npts, const double* data,
       reinterpret_cast<char*>(workspace) +
       align_up(size_t(nb) * size_t(nitems) * sizeof(double), 256));
   const dim3 grid{unsigned(nb), unsigned(nitems)};
-  if (flags & LMB_FP64) {
-    const size_t smem = sizeof(Quad<double>) * 2 * (size_t(nmax_cap) + 1);
-    LMB_CK(smem_attr((const void*)k_chi2<double>, smem));
-    k_chi2<double><<<grid, tpb, smem, st>>>(
-        coords, npts, crop_start, item_crop, ncrops, spheres, item_start,
-        reinterpret_cast<const zd*>(ab), nmax, nmax_cap + 1, k, flags, aberr,
-        data, 1. / noise, partial, partial_bad);
-  } else {
-    const size_t smem = sizeof(Quad<float>) * 2 * (size_t(nmax_cap) + 1);
-    LMB_CK(smem_attr((const void*)k_chi2<float>, smem));
-    k_chi2<float><<<grid, tpb, smem, st>>>(
-        coords, npts, crop_start, item_crop, ncrops, spheres, item_start,
-        reinterpret_cast<const zd*>(ab), nmax, nmax_cap + 1, k, flags, aberr,
-        data, 1. / noise, partial, partial_bad);
-  }
-  LMB_CK(cudaGetLastError());
+  // Up to eight blocks, the portable cluster size, add their sums themselves.
+  const bool cluster = nb <= 8;
+  const bool fp64 = flags & LMB_FP64;
+  const size_t smem = (fp64 ? sizeof(Quad<double>) : sizeof(Quad<float>)) * 2 *
+                      (size_t(nmax_cap) + 1);
+  auto fn = fp64 ? (cluster ? k_chi2<double, true> : k_chi2<double, false>)
+                 : (cluster ? k_chi2<float, true> : k_chi2<float, false>);
+  LMB_CK(smem_attr((const void*)fn, smem));
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid;
+  config.blockDim = dim3(tpb);
+  config.dynamicSmemBytes = smem;
+  config.stream = st;
+  cudaLaunchAttribute size;
+  size.id = cudaLaunchAttributeClusterDimension;
+  size.val.clusterDim.x = unsigned(nb);
+  size.val.clusterDim.y = size.val.clusterDim.z = 1;
+  config.attrs = &size;
+  config.numAttrs = cluster ? 1 : 0;
+  LMB_CK(cudaLaunchKernelEx(&config, fn, coords, npts, crop_start, item_crop, ncrops, spheres,
+                            item_start, reinterpret_cast<const zd*>(ab), nmax, nmax_cap + 1, k,
+                            flags, aberr, data, 1. / noise, partial, partial_bad, chi2,
+                            nonfinite));
+  if (cluster) return LMB_OK;
   k_chi2_reduce<<<(nitems + 127) / 128, 128, 0, st>>>(partial, partial_bad, nb,
                                                        nitems, chi2, nonfinite);
   LMB_CK(cudaGetLastError());
