@@ -105,14 +105,6 @@ struct RadialPlan {
   int flags;
 };
 
-// Interval width in pixels, a multiple of 1/64 so that i * width is exact
-// in FP32; 0 if k is out of range.
-inline double radial_spacing(double k, bool fp64) {
-  const double r = fp64 ? RADIAL_SPACING64 : RADIAL_SPACING;
-  const double w = std::min(floor(64. * r / k) / 64., 64.);
-  return w >= 0.0625 ? w : 0.;
-}
-
 // Largest distance of a particle from the grid's pixels.
 __host__ __device__ inline double radial_reach(double x0, double y0, long long nx,
                                                long long ny, double xp, double yp) {
@@ -256,44 +248,14 @@ __device__ void radial_resum64(const RadialPlan& pl, const int* list, int F, Whe
     const long long pix = where(list[live ? f : F - 1], &x, &y);
     double e[6] = {0., 0., 0., 0., 0., 0.};
     for (int p = pb + sub; live && p < pe; p += group) {
-      const double dx = x - spheres[p].x_p, dy = y - spheres[p].y_p;
-      const double rho = sqrt(dx * dx + dy * dy);
-      const double u = rho / pl.spacing;
-      const int j = min(int(u + 0.5), pl.intervals - 1);
-      double w[RADIAL_TAPS], v[RADIAL_FUNCS];
-      radial_weights(u - double(j), w);
-      for (int c = 0; c < RADIAL_FUNCS; ++c) v[c] = 0.;
-      const double2* s =
-          reinterpret_cast<const double2*>(nodes + (size_t(p) * ncap + j) * RADIAL_FUNCS);
-#pragma unroll
-      for (int l = 0; l < RADIAL_TAPS; ++l)
-        for (int c = 0; c < RADIAL_FUNCS / 2; ++c) {
-          const double2 n = s[l * (RADIAL_FUNCS / 2) + c];
-          v[2 * c] = fma(w[l], n.x, v[2 * c]);
-          v[2 * c + 1] = fma(w[l], n.y, v[2 * c + 1]);
-        }
-      const double c2 = dx * dx - dy * dy, s2 = 2. * dx * dy;
-      for (int c = 0; c < 2; ++c) {
-        e[c] += v[c] + c2 * v[2 + c];
-        e[2 + c] += s2 * v[2 + c];
-        e[4 + c] += dx * v[4 + c];
-      }
+      radial_point64(x - spheres[p].x_p, y - spheres[p].y_p, pl.spacing, pl.intervals,
+                     reinterpret_cast<const d2*>(nodes + size_t(p) * ncap * RADIAL_FUNCS), e);
     }
     for (int o = group >> 1; o > 0; o >>= 1)
       for (int c = 0; c < 6; ++c) e[c] += __shfl_xor_sync(0xffffffffu, e[c], o);
     const zd t[3] = {mk(e[0], e[1]), mk(e[2], e[3]), mk(e[4], e[5])};
     if (live && sub == 0) out[pix] = float(intensity<double>(t));
   }
-}
-
-// The bound on an FP32 pixel's error from the tables: the field of a
-// particle is off by at most RADIAL_FIELD_REL |E_p| (coefficients and
-// Horner's rule in FP32), with |E_p| <= 1.8 max(|Re U|, |Im U|) wherever it
-// is large; |H - H64| <= 2 sqrt(H) sum_p of that.
-#define RADIAL_FIELD_REL 4e-7f
-
-__device__ inline bool radial_needs_fp64(float h, float m1) {
-  return 2.f * sqrtf(fmaxf(h, 0.f)) * (1.8f * RADIAL_FIELD_REL) * m1 > HOLO_TOL;
 }
 
 struct TileParticle {
@@ -333,17 +295,6 @@ __device__ inline TileParticle tile_particle(const RadialPlan& pl, const lmb_sph
 constexpr int kTile = 32;          // tiles of 32 x 32 pixels
 constexpr int kPixThreads = 256;   // a 2x2 group each
 constexpr int kTileGroup = 32;     // particles whose TileParticle is staged at once
-
-// One complex function (re, im) at t: degree RADIAL_COEFS - 1.
-__device__ inline f2 radial_eval(const float4* r, float t) {
-  const float4 a = r[0], b = r[1], c = r[2];
-  const f2 tt = pk(t, t);
-  f2 v = pfma(pk(c.z, c.w), tt, pk(c.x, c.y));
-  v = pfma(v, tt, pk(b.z, b.w));
-  v = pfma(v, tt, pk(b.x, b.y));
-  v = pfma(v, tt, pk(a.z, a.w));
-  return pfma(v, tt, pk(a.x, a.y));
-}
 
 // One block per 32x32-pixel tile and item, 4 pixels per thread.  For each
 // particle the intervals that the tile needs (its distances span at most
@@ -464,7 +415,7 @@ k_field_radial(RadialPlan pl, const lmb_sphere* __restrict__ spheres,
         ex[q] = pfma(pk(c, c), v, padd(ex[q], u));
         ey[q] = pfma(pk(s, s), v, ey[q]);
         ez[q] = pfma(pk(x, x), w, ez[q]);
-        if (kHolo) m1[q] += fmaxf(fabsf(u.x), fabsf(u.y));
+        if (kHolo) m1[q] += radial_bound(u, v, w, c, s, x);
       }
     }
   }
@@ -632,36 +583,16 @@ k_points_radial(RadialPlan pl, const double* __restrict__ points, long long npts
   if (pix < npts) {
     const double x = points[pix], y = points[npts + pix];
     const float inv_spacing = float(1. / pl.spacing), spacing = float(pl.spacing);
-    constexpr int RQ = RADIAL_REC / 4;
-    f2 ex = pk(0.f, 0.f), ey = ex, ez = ex;
-    float m1 = 0.f;
-    for (int p = pb; p < pe; ++p) {
-      // the grid kernel's arithmetic, x and y in the two lanes
-      const double dx = x - spheres[p].x_p, dy = y - spheres[p].y_p;
-      const double ax = rint(dx * 1024.) * (1. / 1024.), ay = rint(dy * 1024.) * (1. / 1024.);
-      const f2 X = pk(float(ax), float(ay)), rx = pk(float(dx - ax), float(dy - ay));
-      const f2 px = pmul(X, X);
-      const f2 lx = pfma(padd(rx, rx), pfma(pk(0.5f, 0.5f), rx, X), pfma(X, X, pneg(px)));
-      const f2 Xr = padd(X, rx);
-      const RadialDistance d = radial_distance(pk(px.x, px.x), pk(lx.x, lx.x),
-                                               pk(px.y, px.y), pk(lx.y, lx.y));
-      const int i =
-          min(max(__float2int_rn(d.r0.x * inv_spacing), 0), pl.intervals - 1);
-      const float t = ((d.r0.x - float(i) * spacing) + d.corr.x) * pl.inv_half;
-      const float4* r = reinterpret_cast<const float4*>(
-          table + (size_t(p) * pl.intervals + i) * RADIAL_REC);
-      const f2 u = radial_eval(r, t), v = radial_eval(r + RQ / 3, t),
-               w = radial_eval(r + 2 * (RQ / 3), t);
-      const float c = (Xr.x - Xr.y) * (Xr.x + Xr.y), s = (Xr.x + Xr.x) * Xr.y;
-      ex = pfma(pk(c, c), v, padd(ex, u));
-      ey = pfma(pk(s, s), v, ey);
-      ez = pfma(pk(Xr.x, Xr.x), w, ez);
-      if (kHolo) m1 += fmaxf(fabsf(u.x), fabsf(u.y));
-    }
-    const cplx<float> e[3] = {mk(ex.x, ex.y), mk(ey.x, ey.y), mk(ez.x, ez.y)};
+    RadialSum r = {pk(0.f, 0.f), pk(0.f, 0.f), pk(0.f, 0.f), 0.f};
+    for (int p = pb; p < pe; ++p)
+      radial_point(x - spheres[p].x_p, y - spheres[p].y_p, inv_spacing, spacing, pl.inv_half,
+                   pl.intervals,
+                   reinterpret_cast<const f4*>(table + size_t(p) * pl.intervals * RADIAL_REC),
+                   r);
+    const cplx<float> e[3] = {mk(r.ex.x, r.ex.y), mk(r.ey.x, r.ey.y), mk(r.ez.x, r.ez.y)};
     if (kHolo) {
       const float h = intensity<float>(e);
-      mark = radial_needs_fp64(h, m1);
+      mark = radial_needs_fp64(h, r.m1);
       if (!mark) reinterpret_cast<float*>(out)[size_t(item) * npts + pix] = h;
     } else {
       float2* o = reinterpret_cast<float2*>(out) + size_t(item) * 3 * npts;

@@ -57,6 +57,14 @@ enum {
 // cancellation in V costs as much; near the axis they contribute V rho^2 and
 // Z rho.
 #define RADIAL_AXIS 1e-4
+// Interval width in pixels, a multiple of 1/64 so that i * width is exact
+// in FP32; 0 if k is out of range.
+inline double radial_spacing(double k, bool fp64) {
+  const double r = fp64 ? RADIAL_SPACING64 : RADIAL_SPACING;
+  const double w = fmin(floor(64. * r / k) / 64., 64.);
+  return w >= 0.0625 ? w : 0.;
+}
+
 // Row c: the weights of the nodes in the coefficient of t^c, t = (rho - rho_i)
 // / (half a spacing).
 template <int NC = RADIAL_COEFS>
@@ -162,6 +170,27 @@ struct RadialDistance {
   f2 r0, corr, y;
 };
 
+// Quads and pairs as the kernels load them.
+#if defined(__CUDACC__)
+typedef float4 f4;
+typedef double2 d2;
+#else
+struct f4 {
+  float x, y, z, w;
+};
+struct d2 {
+  double x, y;
+};
+#endif
+
+LMB_HD int radial_round(float v) {
+#if defined(__CUDA_ARCH__)
+  return __float2int_rn(v);
+#else
+  return int(nearbyintf(v));
+#endif
+}
+
 LMB_HD f2 pneg(f2 a) { return pk(-a.x, -a.y); }
 LMB_HD f2 psub(f2 a, f2 b) { return pfma(pk(-1.f, -1.f), b, a); }
 
@@ -179,6 +208,103 @@ LMB_HD RadialDistance radial_distance(f2 px, f2 lx, f2 qy, f2 ly) {
   const f2 e = padd(pfma(pneg(d.r0), d.r0, sh), sl);
   d.corr = pmul(pmul(pk(0.5f, 0.5f), y), e);
   return d;
+}
+
+// One complex function (re, im) at t: degree RADIAL_COEFS - 1.
+LMB_HD f2 radial_eval(const f4* r, float t) {
+  const f4 a = r[0], b = r[1], c = r[2];
+  const f2 tt = pk(t, t);
+  f2 v = pfma(pk(c.z, c.w), tt, pk(c.x, c.y));
+  v = pfma(v, tt, pk(b.z, b.w));
+  v = pfma(v, tt, pk(b.x, b.y));
+  v = pfma(v, tt, pk(a.z, a.w));
+  return pfma(v, tt, pk(a.x, a.y));
+}
+
+// The bound on an FP32 pixel's error from the tables.  A particle's field
+//   E_x = U + c V,  E_y = s V,  E_z = x Z
+// is off by at most RADIAL_FIELD_REL times |U| + |V| (|c| + |s|) + |x Z|, |.|
+// the larger of the real and the imaginary part's: the coefficients, Horner's
+// rule and c and s are rounded to FP32, and U may cancel against c V (behind
+// a large sphere of high index, near its axis, both are up to a hundred times
+// E).  The hologram is off by at most 2 sqrt(H) times the sum over the
+// particles.  On the CPU build, over 2.4 million pixels of spheres of 0.3-24
+// um, indices to 2.6, from 1.8 / k above the sphere on: the field is off by
+// at most 2.4e-7 of that, an unmarked pixel's hologram by at most 7.2e-6.
+// 1.8 |U|, what |E| comes to where U does not cancel, keeps the error of
+// ordinary images lower still: 7.6e-8 for 8.3e-8 of the hologram over a batch
+// of 128 images.
+#define RADIAL_FIELD_REL 4e-7f
+
+LMB_HD float radial_bound(f2 u, f2 v, f2 w, float c, float s, float x) {
+  const float mu = fmaxf(fabsf(u.x), fabsf(u.y));
+  const float mv = fmaxf(fabsf(v.x), fabsf(v.y));
+  const float mw = fmaxf(fabsf(w.x), fabsf(w.y));
+  return fmaxf(1.8f * mu, fmaf(mw, fabsf(x), fmaf(mv, fabsf(c) + fabsf(s), mu)));
+}
+
+LMB_HD bool radial_needs_fp64(float h, float m1) {
+  return 2.f * sqrtf(fmaxf(h, 0.f)) * RADIAL_FIELD_REL * m1 > HOLO_TOL;
+}
+
+// FP32 field (re, im) of one pixel, summed over the particles, and its bound.
+struct RadialSum {
+  f2 ex, ey, ez;
+  float m1;
+};
+
+// Adds a particle's field at the offset (dx, dy) from its axis, the grid
+// kernel's arithmetic with x and y in the two lanes.  table: the particle's
+// intervals.
+LMB_HD void radial_point(double dx, double dy, float inv_spacing, float spacing,
+                         float inv_half, int intervals, const f4* table, RadialSum& s) {
+  constexpr int RQ = RADIAL_REC / 4;
+  const double ax = rint(dx * 1024.) * (1. / 1024.), ay = rint(dy * 1024.) * (1. / 1024.);
+  const f2 X = pk(float(ax), float(ay)), rx = pk(float(dx - ax), float(dy - ay));
+  const f2 px = pmul(X, X);
+  const f2 lx = pfma(padd(rx, rx), pfma(pk(0.5f, 0.5f), rx, X), pfma(X, X, pneg(px)));
+  const f2 Xr = padd(X, rx);
+  const RadialDistance d =
+      radial_distance(pk(px.x, px.x), pk(lx.x, lx.x), pk(px.y, px.y), pk(lx.y, lx.y));
+  const int r = radial_round(d.r0.x * inv_spacing);
+  const int i = r < 0 ? 0 : r < intervals ? r : intervals - 1;
+  const float t = ((d.r0.x - float(i) * spacing) + d.corr.x) * inv_half;
+  const f4* rec = table + size_t(i) * RQ;
+  const f2 u = radial_eval(rec, t), v = radial_eval(rec + RQ / 3, t),
+           w = radial_eval(rec + 2 * (RQ / 3), t);
+  const float c = (Xr.x - Xr.y) * (Xr.x + Xr.y), s2 = (Xr.x + Xr.x) * Xr.y;
+  s.ex = pfma(pk(c, c), v, padd(s.ex, u));
+  s.ey = pfma(pk(s2, s2), v, s.ey);
+  s.ez = pfma(pk(Xr.x, Xr.x), w, s.ez);
+  s.m1 += radial_bound(u, v, w, c, s2, Xr.x);
+}
+
+// The same in FP64, straight from the particle's nodes (the first
+// RADIAL_SIDE before the axis), e: (re, im) of E_x, E_y, E_z.
+LMB_HD void radial_point64(double dx, double dy, double spacing, int intervals,
+                           const d2* nodes, double* e) {
+  const double rho = sqrt(dx * dx + dy * dy);
+  const double u = rho / spacing;
+  const int j = int(u + 0.5) < intervals ? int(u + 0.5) : intervals - 1;
+  double w[RADIAL_TAPS], v[RADIAL_FUNCS];
+  radial_weights(u - double(j), w);
+  for (int c = 0; c < RADIAL_FUNCS; ++c) v[c] = 0.;
+  const d2* s = nodes + size_t(j) * (RADIAL_FUNCS / 2);
+#if defined(__CUDACC__)
+#pragma unroll
+#endif
+  for (int l = 0; l < RADIAL_TAPS; ++l)
+    for (int c = 0; c < RADIAL_FUNCS / 2; ++c) {
+      const d2 n = s[l * (RADIAL_FUNCS / 2) + c];
+      v[2 * c] = fma(w[l], n.x, v[2 * c]);
+      v[2 * c + 1] = fma(w[l], n.y, v[2 * c + 1]);
+    }
+  const double c2 = dx * dx - dy * dy, s2 = 2. * dx * dy;
+  for (int c = 0; c < 2; ++c) {
+    e[c] += v[c] + c2 * v[2 + c];
+    e[2 + c] += s2 * v[2 + c];
+    e[4 + c] += dx * v[4 + c];
+  }
 }
 
 }  // namespace lmb

@@ -14,6 +14,7 @@
 #include "lmb_lm.cuh"
 #include "lmb_mie.cuh"
 #include "lmb_pixel.cuh"
+#include "lmb_radial.cuh"
 #include "lmb_records.cuh"
 
 using namespace lmb;
@@ -462,3 +463,106 @@ API void h_lm_result(void* p, long long npix, double* x, int* info, int* nfev,
 
 API int h_sym6(int i, int j) { return sym6(i, j); }
 
+// The nodes of one sphere's radial table as k_radial_table forms them:
+// [count + 2 RADIAL_SIDE][RADIAL_FUNCS], node j at distance (j - RADIAL_SIDE)
+// spacing.  axis 0: the node at the axis from its neighbours (FP64 tables).
+static std::vector<double> radial_nodes(const Quad<double>* rec, int nmax, double k, double z,
+                                        double zp, bool bohren, double aberr, double spacing,
+                                        int count, double axis) {
+  std::vector<double> v(size_t(RADIAL_FUNCS) * (count + 2 * RADIAL_SIDE));
+  for (int j = -RADIAL_SIDE; j < count + RADIAL_SIDE; ++j)
+    radial_field(k, j ? spacing * double(abs(j)) : axis, z - zp, z, zp, bohren, aberr, rec,
+                 nmax, &v[RADIAL_FUNCS * (j + RADIAL_SIDE)]);
+  if (axis == 0.)
+    for (int f = 2; f < RADIAL_FUNCS; ++f) {
+      double* s = &v[RADIAL_FUNCS * RADIAL_SIDE + f];
+      double sum = 0., w = 1.;
+      for (int m = 1; m <= RADIAL_SIDE; ++m) {
+        w *= -double(RADIAL_SIDE + 1 - m) / double(RADIAL_SIDE + m);
+        sum -= 2. * w * s[RADIAL_FUNCS * m];
+      }
+      s[0] = sum;
+    }
+  return v;
+}
+
+template <typename R, int NC>
+static std::vector<R> radial_polynomials(const std::vector<double>& nodes, int count) {
+  const RadialMatrixN<NC> A = radial_matrix<NC>();
+  std::vector<R> out(size_t(count) * RADIAL_FUNCS * NC);
+  for (int i = 0; i < count; ++i)
+    for (int f = 0; f < RADIAL_FUNCS; ++f)
+      for (int q = 0; q < NC; ++q) {
+        double c = 0.;
+        for (int l = 0; l < RADIAL_TAPS; ++l)
+          c = fma(A.m[q][l], nodes[size_t(RADIAL_FUNCS) * (i + l) + f], c);
+        out[(size_t(i) * (RADIAL_FUNCS / 2) + f / 2) * 2 * NC + 2 * q + (f & 1)] = R(c);
+      }
+  return out;
+}
+
+// Field [3][npts] complex and hologram [npts] of one sphere p at coords
+// [2][npts] of the plane z from its radial table.  fp64 0: as
+// k_points_radial, marked[i] 1 where the bound asks for the FP64 sum, holo[i]
+// then that sum; fp64 1: as k_field_radial64.
+API void h_radial(const double* coords, long long npts, double z, const double* p,
+                  const double* ab, int nmax, double k, int flags, double aberr, int fp64,
+                  double* field, double* holo, int* marked) {
+  std::vector<Quad<double>> rec(2 * (nmax + 1));
+  stage<double>(ab, 0, nmax, rec.data(), 2);
+  const double spacing = radial_spacing(k, fp64);
+  double far = 0.;
+  for (long long i = 0; i < npts; ++i)
+    far = fmax(far, hypot(coords[i] - p[0], coords[npts + i] - p[1]));
+  const int count = int(far / spacing) + 2;
+  const std::vector<double> nodes =
+      radial_nodes(rec.data(), nmax, k, z, p[2], flags & 2, aberr, spacing, count,
+                   fp64 ? 0. : RADIAL_AXIS);
+  if (!fp64) {
+    const std::vector<float> table = radial_polynomials<float, RADIAL_COEFS>(nodes, count);
+    const float inv_spacing = float(1. / spacing), inv_half = float(2. / spacing);
+    for (long long i = 0; i < npts; ++i) {
+      const double dx = coords[i] - p[0], dy = coords[npts + i] - p[1];
+      RadialSum s = {pk(0.f, 0.f), pk(0.f, 0.f), pk(0.f, 0.f), 0.f};
+      radial_point(dx, dy, inv_spacing, float(spacing), inv_half, count,
+                   reinterpret_cast<const f4*>(table.data()), s);
+      const cplx<float> e[3] = {mk(s.ex.x, s.ex.y), mk(s.ey.x, s.ey.y), mk(s.ez.x, s.ez.y)};
+      for (int c = 0; c < 3; ++c) {
+        field[2 * (c * npts + i)] = e[c].re;
+        field[2 * (c * npts + i) + 1] = e[c].im;
+      }
+      const float h = intensity<float>(e);
+      marked[i] = radial_needs_fp64(h, s.m1);
+      holo[i] = h;
+      if (marked[i]) {
+        double r[6] = {0., 0., 0., 0., 0., 0.};
+        radial_point64(dx, dy, spacing, count, reinterpret_cast<const d2*>(nodes.data()), r);
+        const zd t[3] = {mk(r[0], r[1]), mk(r[2], r[3]), mk(r[4], r[5])};
+        holo[i] = float(intensity<double>(t));
+      }
+    }
+    return;
+  }
+  const std::vector<double> table = radial_polynomials<double, RADIAL_COEFS64>(nodes, count);
+  for (long long i = 0; i < npts; ++i) {
+    const double dx = coords[i] - p[0], dy = coords[npts + i] - p[1];
+    const double rho = sqrt(fma(dx, dx, dy * dy));
+    int j = int(nearbyint(rho / spacing));
+    if (j > count - 1) j = count - 1;
+    const double u = (rho - double(j) * spacing) * (2. / spacing);
+    zd v[3];
+    for (int f = 0; f < 3; ++f) {
+      const double* r = &table[(size_t(j) * 3 + f) * 2 * RADIAL_COEFS64];
+      v[f] = mk(0., 0.);
+      for (int q = RADIAL_COEFS64 - 1; q >= 0; --q)
+        v[f] = mk(fma(v[f].re, u, r[2 * q]), fma(v[f].im, u, r[2 * q + 1]));
+    }
+    const zd e[3] = {v[0] + ((dx - dy) * (dx + dy)) * v[1], (2. * dx * dy) * v[1], dx * v[2]};
+    for (int c = 0; c < 3; ++c) {
+      field[2 * (c * npts + i)] = e[c].re;
+      field[2 * (c * npts + i) + 1] = e[c].im;
+    }
+    holo[i] = intensity<double>(e);
+    marked[i] = 0;
+  }
+}

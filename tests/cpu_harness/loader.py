@@ -63,6 +63,9 @@ def load():
     lib.h_jacobian_pair.argtypes = [_dp, ctypes.c_longlong, _dp, _dp, _dp,
                                     ctypes.c_int, ctypes.c_double,
                                     ctypes.c_int, _dp, _dp]
+    lib.h_radial.argtypes = [_dp, ctypes.c_longlong, ctypes.c_double, _dp,
+                             _dp, ctypes.c_int, ctypes.c_double, ctypes.c_int,
+                             ctypes.c_double, ctypes.c_int, _dp, _dp, _ip]
     lib.h_lm_new.restype = ctypes.c_void_p
     lib.h_lm_new.argtypes = [ctypes.c_int, _ip, _dp] + [ctypes.c_double] * 4 + [ctypes.c_int]
     lib.h_lm_free.argtypes = [ctypes.c_void_p]
@@ -203,6 +206,23 @@ class Harness:
                                  ptr(nmax, _ip), cap, k, 3 | (0 if flag else 8),
                                  ptr(holo, fp), ptr(terms, fp))
         return holo, terms
+
+    def radial(self, coords, p, ab, k, z=0., bohren=True, aberration=0.,
+               fp64=False):
+        '''(3, npts) complex field, hologram (npts,) and the pixels summed
+        again in FP64 (npts,) of one sphere from its radial table, coords
+        (2, npts) in the plane z.'''
+        c = np.ascontiguousarray(coords, dtype=float)
+        npts = c.shape[1]
+        n, a, _ = self._pack_ab(ab)
+        out = np.zeros((3, npts, 2))
+        holo = np.zeros(npts)
+        marked = np.zeros(npts, np.int32)
+        pv = np.asarray(p, dtype=float)
+        self.lib.h_radial(ptr(c), npts, float(z), ptr(pv), ptr(a), n, k,
+                          1 | (2 if bohren else 0), float(aberration),
+                          int(fp64), ptr(out), ptr(holo), ptr(marked, _ip))
+        return out[..., 0] + 1j * out[..., 1], holo, marked > 0
 
     def jacobian_aberrated(self, coords, p, ab, dab, k, aberration,
                            bohren=True, fp64=False):
