@@ -155,8 +155,9 @@ int lmb_hologram_aberrated(const double *coords, long long npts,
  *                      these n spheres (host records, a_p the outer radius)
  *                      need for npts pixels, or 0 where the tables do not
  *                      apply and the coordinate entry points are to be used:
- *                      a plane closer than k d = 1.8 to a sphere or cutting
- *                      it, distances above 8000 px, spherical components,
+ *                      a plane closer than k d = 13 to a sphere's centre or
+ *                      1.8 (LMB_FP64: 5.5) to its surface, or cutting it,
+ *                      distances above 8000 px, spherical components,
  *                      an aberration phase steeper than a fifth of k,
  *                      or too few pixels to pay for the tables.
  * lmb_field_grid / lmb_hologram_grid: as lmb_field_aberrated /

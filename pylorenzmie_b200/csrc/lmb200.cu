@@ -589,7 +589,7 @@ static int grad_plan(const lmb_grid* grid, long long npts, const lmb_sphere* sph
     const double dy = fmax(fabs(grid->y0 - s.y_p), fabs(grid->y0 + double(grid->ny - 1) - s.y_p));
     const double reach = sqrt(dx * dx + dy * dy), dz = fabs(grid->z - s.z_p);
     if (!(reach < 8000.) || !(s.a_p > 0.) || !(dz < 1e6)) return 0;
-    if (!(k * (dz - s.a_p / magnification) >= RADIAL_CLEARANCE)) return 0;
+    if (!radial_clear(k, dz, s.a_p / magnification, false)) return 0;
     far = fmax(far, reach);
     rate = fmax(rate, double(fitr_rate(float(k), float(s.a_p / magnification), float(dz),
                                        float(reach))));

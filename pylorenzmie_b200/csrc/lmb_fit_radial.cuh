@@ -549,8 +549,8 @@ k_fit_eval_radial(FitCtx c, RadialMatrix A, int cap) {
       }
       const double x = c.size_per_um * ep.p[3];  // size parameter
       float rate = fitr_rate(k, float(x) / k, zp, hi);
-      bool ok = c.k * fabs(ep.p[2]) - x >= RADIAL_CLEARANCE && hi < 8000.f && zp < 1e6f &&
-                isfinite(ep.p[0]) && isfinite(ep.p[1]);
+      bool ok = radial_clear(c.k, fabs(ep.p[2]), x / c.k, false) && hi < 8000.f &&
+                zp < 1e6f && isfinite(ep.p[0]) && isfinite(ep.p[1]);
       if (c.aberr != 0.) {  // the aberration's phase, as lmb_radial_intervals
         const float turn = 0.5f * fabsf(float(c.aberr)) / zp;
         ok = ok && turn <= 0.2f * k;

@@ -767,7 +767,7 @@ int lmb_radial_intervals(const lmb_grid* grid, long long npts, const lmb_sphere*
     const double dz = fabs(grid->z - s.z_p);
     // offsets up to 8192 px split exactly in FP32 (radial_distance)
     if (!(reach < 8000.) || !(s.a_p > 0.) || !isfinite(s.z_p)) return 0;
-    if (!(k * (dz - s.a_p / magnification) >= RADIAL_CLEARANCE)) return 0;
+    if (!radial_clear(k, dz, s.a_p / magnification, fp64)) return 0;
     // the aberration's phase turns by at most |c| / (2 |z_p|) per pixel, at
     // rho = |z_p|, where the field's own band ends at 0.7 k
     if (aberration != 0. && !(0.5 * fabs(aberration) <= 0.2 * k * fabs(s.z_p))) return 0;

@@ -48,3 +48,44 @@ def test_holograms_within_the_bound(h, a, n, mag, gap, side):
     ab, _, H = direct(h, c, p, a, n, 0., k)
     _, got, _ = h.radial(c, p, ab, k)
     assert np.all(np.abs(got - H) <= 2e-5 + 6e-8 * H)
+
+
+def nearest(a, n, kp, k, mag, fp64):
+    '''The least distance of the plane from the sphere's centre (px) at
+    which the library takes the tables.'''
+    from pylorenzmie_b200 import _native
+    lib = _native.load()
+    flags = (_native.LMB_CARTESIAN | _native.LMB_BOHREN |
+             (_native.LMB_FP64 if fp64 else 0))
+    s = np.zeros(1, dtype=_native.SPHERE_DTYPE)
+
+    def accepted(z):
+        s[0] = 150., 150., z, a, n, kp
+        return lib.lmb_radial_intervals(
+            _native.Grid(0., 0., 0., 300, 300), 90000, s.ctypes.data, 1, k,
+            mag, flags, 0.) > 0
+    lo, hi = a / mag, a / mag + 100.
+    assert accepted(hi) and not accepted(lo)
+    while hi - lo > 1e-6:
+        mid = 0.5 * (lo + hi)
+        lo, hi = (lo, mid) if accepted(mid) else (mid, hi)
+    return hi
+
+
+@pytest.mark.parametrize('n,kp', [(1.36, 0.), (1.45, 0.), (2.6, 0.),
+                                  (0.2, 3.)])
+@pytest.mark.parametrize('fp64', [False, True])
+def test_fields_wherever_the_tables_are_taken(h, n, kp, fp64):
+    '''Within 1e-6 (FP64: 1e-12) of the field's largest component, the
+    bounds of the fields of the library, as close to the plane as the library
+    takes the tables, from spheres of a few nm on.'''
+    k = field.wavenumber(1.34, 0.447, 0.048)
+    rng = np.random.default_rng(7)
+    for a in (0.005, 0.02, 0.05, 0.1, 0.2, 0.27, 0.3, 0.414, 0.5, 0.75, 2.5,
+              6., 24.):
+        c = pixels(rng, 400, 60.)
+        p = [0., 0., nearest(a, n, kp, k, 0.048, fp64)]
+        ab, E, _ = direct(h, c, p, a, n, kp, k)
+        got, _, _ = h.radial(c, p, ab, k, fp64=fp64)
+        err = np.abs(got - E).max() / np.abs(E).max()
+        assert err <= (1e-12 if fp64 else 1e-6), (a, err)
