@@ -159,21 +159,25 @@ k_radial_table(RadialPlan pl, RadialMatrixN<NC> A, const lmb_sphere* __restrict_
   const int ncap = pl.intervals + 2 * RADIAL_SIDE;
   if (j < count + RADIAL_SIDE) {
     double v[RADIAL_FUNCS];
-    // V and Z at the axis are limits: nearly there for FP32, from their
-    // neighbours (below) for FP64
-    const double axis = sizeof(R) == sizeof(float) ? RADIAL_AXIS : 0.;
-    radial_field(pl.k, j ? pl.spacing * double(abs(j)) : axis, pl.z - sp.z_p, pl.z, sp.z_p,
-                 pl.flags & LMB_BOHREN, pl.aberr, rec, nm, v);
-    const int t = threadIdx.x;
-    for (int f = 0; f < RADIAL_FUNCS; ++f) val[f * kNodeThreads + t] = v[f];
-    // each node is written by the chunk it lies in (the ends by the outer ones)
-    if (nodes && (t >= RADIAL_SIDE || i0 == 0) &&
-        (t < kNodeThreads - RADIAL_SIDE || i0 + kChunk >= count)) {
-      double* out = nodes + (size_t(p) * ncap + (j + RADIAL_SIDE)) * RADIAL_FUNCS;
-      for (int f = 0; f < RADIAL_FUNCS; ++f) out[f] = v[f];
-    }
+    // V and Z at the axis are limits.  FP32: the threads of nodes 0 and -1
+    // take two distances near it, node -1 being the image of node 1.  FP64:
+    // from the neighbours (below).
+    const double step = sizeof(R) == sizeof(float) ? RADIAL_AXIS_STEP / pl.k : 0.;
+    const double rho = j == 0 ? step
+                       : j == -1 && step > 0. ? 2. * step : pl.spacing * double(abs(j));
+    radial_field(pl.k, rho, pl.z - sp.z_p, pl.z, sp.z_p, pl.flags & LMB_BOHREN, pl.aberr, rec,
+                 nm, v);
+    for (int f = 0; f < RADIAL_FUNCS; ++f) val[f * kNodeThreads + threadIdx.x] = v[f];
   }
   __syncthreads();
+  if (sizeof(R) == sizeof(float) && i0 == 0) {
+    if (threadIdx.x < RADIAL_FUNCS) {
+      double* s = val + threadIdx.x * kNodeThreads + RADIAL_SIDE;
+      s[0] = (4. * s[0] - s[-1]) * (1. / 3.);
+      s[-1] = s[1];
+    }
+    __syncthreads();
+  }
   if (sizeof(R) == sizeof(double) && i0 == 0) {
     // the even function through the nodes 1..8 and -1..-8, at 0: off by at
     // most 3e-13 at this spacing
@@ -187,6 +191,15 @@ k_radial_table(RadialPlan pl, RadialMatrixN<NC> A, const lmb_sphere* __restrict_
       s[0] = sum;
     }
     __syncthreads();
+  }
+  if (nodes && j < count + RADIAL_SIDE) {
+    // each node is written by the chunk it lies in (the ends by the outer ones)
+    const int t = threadIdx.x;
+    if ((t >= RADIAL_SIDE || i0 == 0) &&
+        (t < kNodeThreads - RADIAL_SIDE || i0 + kChunk >= count)) {
+      double* out = nodes + (size_t(p) * ncap + (j + RADIAL_SIDE)) * RADIAL_FUNCS;
+      for (int f = 0; f < RADIAL_FUNCS; ++f) out[f] = val[f * kNodeThreads + t];
+    }
   }
   const int n = min(kChunk, count - i0);
   for (int w = threadIdx.x; w < n * (RADIAL_FUNCS / 2); w += kNodeThreads) {
@@ -224,7 +237,7 @@ k_radial_table(RadialPlan pl, RadialMatrixN<NC> A, const lmb_sphere* __restrict_
 // Pixels.
 
 // FP64 values of the marked pixels of a tile, interpolated straight from
-// the FP64 nodes (17 points, error ~1e-12): for the pixels whose FP32 value
+// the FP64 nodes (17 points, off by ~1e-9 of the field): for the pixels whose FP32 value
 // may be off by more than HOLO_TOL, a few per thousand.  A tile's marked
 // pixels sit together, so the particles of a pixel are spread over lanes: a
 // group of lanes (the next power of two from the particle count, up to the

@@ -70,11 +70,14 @@ LMB_HD bool radial_clear(double k, double dz, double a, bool fp64) {
          k * (dz - a) >= (fp64 ? RADIAL_CLEARANCE64 : RADIAL_CLEARANCE);
 }
 
-// The distance (pixels) that stands for the axis itself, where V and Z are
-// limits: there V and Z are off by (k rho)^2 ~ 1e-8 of themselves and the
-// cancellation in V costs as much; near the axis they contribute V rho^2 and
-// Z rho.
+// The fits' distance (pixels) that stands for the axis itself, where D and its
+// derivatives are limits: they are off by (k rho)^2 ~ 1e-8 of themselves there
+// and the cancellation in D costs as much.
 #define RADIAL_AXIS 1e-4
+// The axis of FP32 images (radians): U, V and Z as (4 f(h) - f(2 h)) / 3, off
+// by 4 h^4 = 6e-11 of a component and by 4e-11 from the cancellation in V.
+// (FP64 tables take it from their neighbours, k_radial_table.)
+#define RADIAL_AXIS_STEP 2e-3
 // Interval width in pixels, a multiple of 1/64 so that i * width is exact
 // in FP32; 0 if k is out of range.
 inline double radial_spacing(double k, bool fp64) {

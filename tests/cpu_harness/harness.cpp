@@ -465,15 +465,22 @@ API int h_sym6(int i, int j) { return sym6(i, j); }
 
 // The nodes of one sphere's radial table as k_radial_table forms them:
 // [count + 2 RADIAL_SIDE][RADIAL_FUNCS], node j at distance (j - RADIAL_SIDE)
-// spacing.  axis 0: the node at the axis from its neighbours (FP64 tables).
+// spacing.  The axis: from two distances near it, or (fp64) its neighbours.
 static std::vector<double> radial_nodes(const Quad<double>* rec, int nmax, double k, double z,
                                         double zp, bool bohren, double aberr, double spacing,
-                                        int count, double axis) {
+                                        int count, bool fp64) {
   std::vector<double> v(size_t(RADIAL_FUNCS) * (count + 2 * RADIAL_SIDE));
   for (int j = -RADIAL_SIDE; j < count + RADIAL_SIDE; ++j)
-    radial_field(k, j ? spacing * double(abs(j)) : axis, z - zp, z, zp, bohren, aberr, rec,
-                 nmax, &v[RADIAL_FUNCS * (j + RADIAL_SIDE)]);
-  if (axis == 0.)
+    radial_field(k, spacing * double(abs(j)), z - zp, z, zp, bohren, aberr, rec, nmax,
+                 &v[RADIAL_FUNCS * (j + RADIAL_SIDE)]);
+  if (!fp64) {
+    double a[2][RADIAL_FUNCS];
+    for (int j = 0; j < 2; ++j)
+      radial_field(k, (j + 1) * (RADIAL_AXIS_STEP / k), z - zp, z, zp, bohren, aberr, rec, nmax,
+                   a[j]);
+    for (int f = 0; f < RADIAL_FUNCS; ++f)
+      v[RADIAL_FUNCS * RADIAL_SIDE + f] = (4. * a[0][f] - a[1][f]) * (1. / 3.);
+  } else {
     for (int f = 2; f < RADIAL_FUNCS; ++f) {
       double* s = &v[RADIAL_FUNCS * RADIAL_SIDE + f];
       double sum = 0., w = 1.;
@@ -483,6 +490,7 @@ static std::vector<double> radial_nodes(const Quad<double>* rec, int nmax, doubl
       }
       s[0] = sum;
     }
+  }
   return v;
 }
 
@@ -517,7 +525,7 @@ API void h_radial(const double* coords, long long npts, double z, const double* 
   const int count = int(far / spacing) + 2;
   const std::vector<double> nodes =
       radial_nodes(rec.data(), nmax, k, z, p[2], flags & 2, aberr, spacing, count,
-                   fp64 ? 0. : RADIAL_AXIS);
+                   fp64);
   if (!fp64) {
     const std::vector<float> table = radial_polynomials<float, RADIAL_COEFS>(nodes, count);
     const float inv_spacing = float(1. / spacing), inv_half = float(2. / spacing);

@@ -89,3 +89,19 @@ def test_fields_wherever_the_tables_are_taken(h, n, kp, fp64):
         got, _, _ = h.radial(c, p, ab, k, fp64=fp64)
         err = np.abs(got - E).max() / np.abs(E).max()
         assert err <= (1e-12 if fp64 else 1e-6), (a, err)
+
+
+@pytest.mark.parametrize('a,n,mag,gap', [
+    (6.30, 2.225, 0.048, 2.26), (20.5, 1.99, 0.048, 2.3),
+    (18.0170928, 2.33393022, 0.048, 50.3), (19.7, 2.15, 0.03, 12.)])
+def test_pixels_summed_again_are_fp64(h, a, n, mag, gap):
+    '''Half a unit in the last place of FP32, and 3e-9 of the hologram: the
+    nodes are interpolated to 1e-9 of the field, and H is its square.'''
+    k = field.wavenumber(1.34, 0.447, mag)
+    c = pixels(np.random.default_rng(int(100 * a)), 6000, 30.)
+    p = [0., 0., a / mag + gap]
+    ab, _, H = direct(h, c, p, a, n, 0., k)
+    _, got, marked = h.radial(c, p, ab, k)
+    half = 0.5 * np.spacing(H.astype(np.float32)).astype(float)
+    assert marked.any()
+    assert np.all((np.abs(got - H) <= half + 3e-9 * H)[marked])
