@@ -162,6 +162,7 @@ int lmb_hologram_aberrated(const double *coords, long long npts,
  *                      or too few pixels to pay for the tables.
  * lmb_field_grid / lmb_hologram_grid: as lmb_field_aberrated /
  *                      lmb_hologram_aberrated (aberration 0: ideal optics);
+ *                      npts = nx * ny without points (else LMB_ERR_ARG),
  *                      nparticles = item_start[nitems], intervals from
  *                      lmb_radial_intervals, workspace of
  *                      lmb_radial_workspace_bytes(nparticles, intervals,
@@ -205,9 +206,12 @@ int lmb_hologram_grid(const lmb_grid *grid, const double *points,
  * in one plane; points nonzero: they are a list in that plane, not the grid.
  * coords: device, [3][npts].  field nonzero: lmb_field's output, else
  * lmb_hologram's.  The host arrays are read before the call returns.
+ * LMB_ERR_ARG: n, nitems or npts are not the plan's, or npts is not the
+ * grid's number of pixels where they are the grid's.
  */
 typedef struct lmb_render {
-  int nmax_cap, intervals;
+  int nmax_cap, intervals, n, nitems;
+  long long npts;
   size_t spheres, ab, nmax, tables, workspace_bytes;
 } lmb_render;
 int lmb_render_plan(const lmb_grid *grid, int points, long long npts,

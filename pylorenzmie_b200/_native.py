@@ -63,7 +63,8 @@ class Grid(ctypes.Structure):
 
 class Render(ctypes.Structure):
     _fields_ = [('nmax_cap', ctypes.c_int), ('intervals', ctypes.c_int),
-                ('spheres', ctypes.c_size_t), ('ab', ctypes.c_size_t),
+                ('n', ctypes.c_int), ('nitems', ctypes.c_int),
+                ('npts', ctypes.c_longlong), ('spheres', ctypes.c_size_t), ('ab', ctypes.c_size_t),
                 ('nmax', ctypes.c_size_t), ('tables', ctypes.c_size_t),
                 ('workspace_bytes', ctypes.c_size_t)]
 

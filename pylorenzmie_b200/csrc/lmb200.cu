@@ -635,7 +635,7 @@ int lmb_hologram_vjp_grid(const lmb_grid* grid, const double* points, long long 
   const int count =
       grad_plan(grid, npts, host_spheres, n, k, magnification, flags, &pl.spacing);
   if (!count) return LMB_ERR_UNSUPPORTED;
-  if (!points && npts != grid->nx * grid->ny) return LMB_ERR_ARG;
+  if (!points && !grid_holds(grid, npts)) return LMB_ERR_ARG;
   if (!workspace || workspace_bytes < lmb_vjp_grid_workspace_bytes(grid, npts, host_spheres, n,
                                                                    k, magnification, flags))
     return LMB_ERR_WORKSPACE;
@@ -682,6 +682,10 @@ int lmb_render_plan(const lmb_grid* grid, int points, long long npts,
                     double aberration, lmb_render* plan) {
   if (n < 0 || nitems < 0 || npts < 0 || !plan || (n > 0 && !host_spheres)) return LMB_ERR_ARG;
   if (!(wavelength > 0.) || !(n_m > 0.)) return LMB_ERR_ARG;
+  if (grid && !points && !grid_holds(grid, npts)) return LMB_ERR_ARG;
+  plan->n = n;
+  plan->nitems = nitems;
+  plan->npts = npts;
   int cap = 1;
   for (int i = 0; i < n; ++i) {
     const lmb_sphere& s = host_spheres[i];
@@ -771,8 +775,14 @@ int lmb_render_run(const lmb_render* plan, const lmb_grid* grid, int points,
                    double k, int flags, double aberration, int field, void* out,
                    void* workspace, size_t workspace_bytes, void* stream) {
   if (!plan || n < 0 || nitems < 0 || npts < 0 || bad_cap(plan->nmax_cap)) return LMB_ERR_ARG;
+  // the workspace is laid out for these
+  if (n != plan->n || nitems != plan->nitems || npts != plan->npts) return LMB_ERR_ARG;
   if (nitems == 0 || npts == 0) return LMB_OK;
   if ((n > 0 && !host_spheres) || !host_item_start || !out) return LMB_ERR_ARG;
+  for (int i = 0; i < nitems; ++i)
+    if (host_item_start[i] < 0 || host_item_start[i + 1] < host_item_start[i] ||
+        host_item_start[i + 1] > n)
+      return LMB_ERR_ARG;
   if (!workspace || workspace_bytes < plan->workspace_bytes) return LMB_ERR_WORKSPACE;
   cudaStream_t st = as_stream(stream);
   char* ws = static_cast<char*>(workspace);

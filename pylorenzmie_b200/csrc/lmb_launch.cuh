@@ -31,6 +31,12 @@ struct AttrEntry {
 inline std::vector<AttrEntry> g_smem_set;    // value: bytes set
 inline std::vector<AttrEntry> g_grid_sizes;  // value: grid
 
+// Whether npts is the grid's number of pixels.
+inline bool grid_holds(const lmb_grid* grid, long long npts) {
+  if (grid->nx < 1 || grid->ny < 1) return npts == 0;
+  return npts / grid->nx == grid->ny && npts % grid->nx == 0;
+}
+
 inline int current_device() {
   int dev = -1;
   return cudaGetDevice(&dev) == cudaSuccess ? dev : -1;

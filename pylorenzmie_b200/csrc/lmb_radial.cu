@@ -659,7 +659,9 @@ int grid_common(bool holo, const lmb_grid* grid, const lmb_sphere* spheres,
                 void* stream) {
   if (nitems < 0 || nparticles < 0 || nmax_cap < 1 || nmax_cap > LMB_NMAX_LIMIT)
     return LMB_ERR_ARG;
-  if (!grid || grid->nx < 0 || grid->ny < 0 || (points && npts < 0)) return LMB_ERR_ARG;
+  if (!grid || grid->nx < 0 || grid->ny < 0 || npts < 0) return LMB_ERR_ARG;
+  // the pixel kernels write nx * ny values an item, the output holds npts
+  if (!points && !grid_holds(grid, npts)) return LMB_ERR_ARG;
   if (nitems == 0 || grid->nx == 0 || grid->ny == 0 || (points && npts == 0))
     return LMB_OK;
   if (!spheres || !item_start || !ab || !nmax || !out || intervals < 1) return LMB_ERR_ARG;
