@@ -304,6 +304,13 @@ def on_grid(grid, coords, records, spheres, item_start, ab, nmax, cap,
 
 # radial tables larger than this are not built (the direct sums need none)
 RADIAL_WORKSPACE_LIMIT = 4 << 30
+# Pixel-orders (spheres x pixels x capacity) from which gradients take the
+# tables.  Below, the direct sums of the pixels take less time than reading
+# the pixels' layout back, the tables' extra launches and their chains of
+# orders.  Forward and backward measured both ways on a B200, 1-24 spheres of
+# 0.5-6 um on 101-901 px square: tables at 0.70-0.99 of the direct sums' speed
+# up to 3.9e7, at 1.05-1.2 from 4.2e7 on and 1.3-2.1 from 7.5e7 on.
+GRADIENT_TABLES = 4e7
 
 
 def jacobian(coords, spheres, ab, dab, nmax, cap, k, bohren=True,
@@ -397,17 +404,20 @@ def render(grid, coords, records, counts, instrument, cartesian, bohren,
 
 def vjp_on_grid(grid, coords, records, spheres, ab, dab, nmax, cap,
                 instrument, gout, bohren=True):
-    '''hologram_vjp for pixels of one plane (make_grid's result) from radial
-    tables (lmb_hologram_vjp_grid); None where they do not apply.'''
+    '''hologram_vjp for pixels of one plane (make_grid's result): from radial
+    tables (lmb_hologram_vjp_grid) where they apply and are the faster way.'''
     lib = _native.load()
     grid, full = grid
     n, npts = len(records), coords.shape[1]
     k, mag = float(instrument.wavenumber()), float(instrument.magnification)
     flags = _flags(True, bohren, False)
-    nbytes = lib.lmb_vjp_grid_workspace_bytes(
-        grid, npts, records.ctypes.data, n, k, mag, flags)
+    nbytes = 0
+    if n * npts * cap >= GRADIENT_TABLES:
+        nbytes = lib.lmb_vjp_grid_workspace_bytes(
+            grid, npts, records.ctypes.data, n, k, mag, flags)
     if not 0 < nbytes <= RADIAL_WORKSPACE_LIMIT:
-        return None
+        return hologram_vjp(coords, spheres, ab, dab, nmax, cap, k,
+                            gout.contiguous(), bohren)
     dev = coords.device
     ab, dab, nmax, spheres = _contiguous(ab, dab, nmax, spheres)
     gout = gout.to(torch.float32).contiguous()

@@ -4,8 +4,8 @@
 holograms of B single spheres, params (B, 6) = (x_p, y_p, z_p, a_p, n_p,
 k_p).  Its backward pass is a hand-written VJP kernel that reduces
 g * dH/dparam over the pixels, from radial tables of the hologram's
-derivatives where the pixels lie in a plane clear of the spheres
-(``lmb_hologram_vjp_grid``), else from recurrences run again pixel by pixel
+derivatives where the pixels lie in a plane clear of the spheres and are
+many enough (``lmb_hologram_vjp_grid``), else from recurrences run again pixel by pixel
 (``lmb_hologram_vjp``).  Nothing per order or per pixel is stored between
 forward and backward (only the O(n_max) Mie coefficients and their parameter
 derivatives).
@@ -22,20 +22,25 @@ from . import _kernels as K
 from .Instrument import Instrument
 
 
-def _prepare(params, instrument, host=None):
+def _read(params, instrument):
+    '''The parameters in FP64, on the device and the host, the instrument and
+    the capacity of orders.'''
     p = params.detach().to(torch.float64).contiguous()
     inst = instrument or Instrument()
-    if host is None:
-        host = p.cpu().numpy()
+    host = p.cpu().numpy()
     cap = K.nmax_cap_for(host[:, 3], host[:, 4], host[:, 5], inst.n_m,
                          inst.wavelength)
     # the capacity covers these spheres, so the coefficients can fail only on
     # invalid parameters: checked here, without reading the device again
     if not (np.isfinite(host).all() and (host[:, 3] > 0.).all()):
         raise ValueError('sphere parameters must be finite with a_p > 0')
-    ab, dab, nmax = K.sphere_ab(p, inst.n_m, inst.wavelength, cap, deriv=True,
-                                check=False)
-    return p, inst, cap, ab, dab, nmax
+    return p, host, inst, cap
+
+
+def _prepare(params, instrument):
+    p, _, inst, cap = _read(params, instrument)
+    return p, inst, cap, *K.sphere_ab(p, inst.n_m, inst.wavelength, cap,
+                                      deriv=True, check=False)
 
 
 def _coords(coordinates, device):
@@ -51,22 +56,24 @@ class HologramFunction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, params, coordinates, instrument, bohren):
-        # the parameters and the pixels' layout in one read-back
-        B, npts = params.shape[0], coordinates.shape[1]
-        grid, host = None, None
-        if B and npts:
-            both = torch.cat([
-                params.detach().to(torch.float64).reshape(-1),
-                coordinates[2, :1],
-                K.probe_grid(coordinates).view(torch.float64)]).cpu().numpy()
-            host = both[:6 * B].reshape(B, 6).copy()
-            grid = K.make_grid(both[6 * B], npts,
-                               both[6 * B + 1:].view(np.int64))
-        p, inst, cap, ab, dab, nmax = _prepare(params, instrument, host)
+        p, host, inst, cap = _read(params, instrument)
+        B, npts = p.shape[0], coordinates.shape[1]
+        # The pixels' layout is needed for tables only, and reading it back
+        # takes longer than the direct sums of small images.
+        tables = B * npts * cap >= K.GRADIENT_TABLES
+        if tables:
+            probed = torch.cat([coordinates[2, :1].view(torch.int64),
+                                K.probe_grid(coordinates)])
+        ab, dab, nmax = K.sphere_ab(p, inst.n_m, inst.wavelength, cap,
+                                    deriv=True, check=False)
+        grid = records = h = None
+        if tables:
+            probed = probed.cpu().numpy()
+            grid = K.make_grid(probed[:1].view(np.float64)[0], npts,
+                               probed[1:])
         item_start = torch.arange(B + 1, dtype=torch.int32, device=p.device)
-        h = None
-        records = None if grid is None else host.view(K.SPHERE_DTYPE).ravel()
         if grid is not None:
+            records = host.copy().view(K.SPHERE_DTYPE).ravel()
             h = K.on_grid(grid, coordinates, records, p, item_start, ab, nmax,
                           cap, inst, True, bohren, 0.)
         if h is None:
@@ -80,12 +87,11 @@ class HologramFunction(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gout):
         p, coordinates, ab, dab, nmax = ctx.saved_tensors
-        grad = None
         if ctx.grid is not None:
             grad = K.vjp_on_grid(ctx.grid, coordinates, ctx.records, p, ab,
                                  dab, nmax, ctx.cap, ctx.inst, gout,
                                  ctx.bohren)
-        if grad is None:
+        else:
             grad = K.hologram_vjp(coordinates, p, ab, dab, nmax, ctx.cap,
                                   ctx.inst.wavenumber(), gout.contiguous(),
                                   ctx.bohren)
