@@ -218,8 +218,9 @@ class LorenzMie(LMObject):
                             self.instrument, cartesian, bohren,
                             self._aberration(), field, self.double_precision)
         sp, item_start, ab, _, nmax, cap, rec = self._prepare(particle_lists)
-        if cartesian and self._grid is not None:
-            out = K.on_grid(self._grid, self._coords, rec, sp, item_start, ab,
+        grid = self._grid if cartesian else None
+        if grid is not None:
+            out = K.on_grid(grid, self._coords, rec, sp, item_start, ab,
                             nmax, cap, self.instrument, cartesian, bohren,
                             self._aberration(), field, self.double_precision)
             if out is not None:

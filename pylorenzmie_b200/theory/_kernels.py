@@ -266,17 +266,15 @@ def on_grid(grid, coords, records, spheres, item_start, ab, nmax, cap,
     fields, of pixels in one plane (make_grid's result) from radial tables
     (lmb_hologram_grid, lmb_field_grid), with ``fp64`` in 64 bits; None
     where they do not apply.  records: the spheres' host records.'''
+    n, npts = len(records), coords.shape[1]
     grid, full = grid
-    npts = coords.shape[1]
+    # particles are the table kernel's grid rows
+    least = IMAGE_TABLES / 2 if fp64 else IMAGE_TABLES
+    if n * npts * cap < least or n > 65535 or (fp64 and not full):
+        return None
     lib = _native.load()
     k = float(instrument.wavenumber())
     flags = _flags(cartesian, bohren, fp64)
-    n = len(records)
-    # Images of less than 200x200 pixels: their direct sums take as long as
-    # the tables (10 us) in one launch fewer.  Particles are the table
-    # kernel's grid rows.
-    if n > 65535 or (full and npts < 40000) or (fp64 and not full):
-        return None
     intervals = lib.lmb_radial_intervals(
         grid, npts, records.ctypes.data, n, k, float(instrument.magnification),
         flags, float(aberration))
@@ -304,12 +302,17 @@ def on_grid(grid, coords, records, spheres, item_start, ab, nmax, cap,
 
 # radial tables larger than this are not built (the direct sums need none)
 RADIAL_WORKSPACE_LIMIT = 4 << 30
-# Pixel-orders (spheres x pixels x capacity) from which gradients take the
-# tables.  Below, the direct sums of the pixels take less time than reading
-# the pixels' layout back, the tables' extra launches and their chains of
-# orders.  Forward and backward measured both ways on a B200, 1-24 spheres of
-# 0.5-6 um on 101-901 px square: tables at 0.70-0.99 of the direct sums' speed
-# up to 3.9e7, at 1.05-1.2 from 4.2e7 on and 1.3-2.1 from 7.5e7 on.
+# Pixel-orders (spheres x pixels x capacity) from which images of layered
+# spheres (FP64: from half as many) and gradients take the tables.  Below, the
+# direct sums of the pixels take less time than the tables' extra launches and
+# their chains of orders.  Calls measured both ways on a B200, 1-24 spheres of
+# 0.5-6 um on 101-1024 px square, tables against direct sums: FP32 images at
+# 0.94-1.16 of the speed up to 2e7, 1.0-1.3 from 2.5e7 and 1.3-1.7 from 8e7
+# on; FP64 images 0.91-1.0 up to 1e7, 1.0-1.2 from 1.2e7 and 1.2-1.5 from 4e7
+# on; gradients (forward and backward), which also read the pixels' layout
+# back for the tables, 0.70-0.99 up to 3.9e7, 1.05-1.2 from 4.2e7 and 1.3-2.1
+# from 7.5e7 on.
+IMAGE_TABLES = 2.5e7
 GRADIENT_TABLES = 4e7
 
 
