@@ -431,9 +431,10 @@ __device__ __noinline__ void fitr_direct(const FitCtx& c, int f, const lmb_featu
 
 // Persistent CTAs pull (feature, part) items: c.parts parts a feature, each
 // a run of its tiles.  A CTA builds the table of its part in shared memory
-// (FP64 nodes, then the polynomials) and evaluates its pixels
-// from it.  A tile's sums do not depend on how the tiles are dealt out.
-// cap: intervals that the table has room for.
+// (FP64 nodes, then the polynomials) and evaluates its pixels from it.  The
+// nodes' spacing follows from the whole feature, so a tile's sums do not
+// depend on how the tiles are dealt out, nor on the other features, while the
+// part's intervals find room.  cap: intervals that the table has room for.
 //
 // 256 features of 201x201 px, 25 orders: 0.13 ms, against 1.14-1.28 ms with
 // the orders summed at every pixel.  By clock64 stamps a CTA takes 9 k clocks
@@ -448,7 +449,7 @@ k_fit_eval_radial(FitCtx c, RadialMatrix A, int cap) {
   extern __shared__ __align__(16) char smem[];
   __shared__ float red[FITR_TPB / 32][32];
   __shared__ FitrPlan s_pl;
-  __shared__ float s_rho[2][FITR_TPB / 32];
+  __shared__ float s_rho[3][FITR_TPB / 32];
   __shared__ int s_item;
   constexpr int REC = fitr_rec(kKP), NF = fitr_funcs(kKP);
   const int nmaxp = c.nmax_cap + 1;
@@ -489,24 +490,31 @@ k_fit_eval_radial(FitCtx c, RadialMatrix A, int cap) {
     const int band = ft.nx > 0 ? fitr_band(ft.nx) : 0;
     const long long i0 = (long long)t0 * FITR_TILE;
     const long long i1 = min((long long)t1 * FITR_TILE, ft.npix);
-    // ---- the distances of the part's pixels
+    // ---- the distances of a list's pixels: the part's, and the farthest
     if (ft.nx == 0) {
-      float lo = 3e38f, hi = 0.f;
-      for (long long i = i0 + threadIdx.x; i < i1; i += FITR_TPB) {
+      float lo = 3e38f, hi = 0.f, far = 0.f;
+#pragma unroll 4
+      for (long long i = threadIdx.x; i < ft.npix; i += FITR_TPB) {
         const float2 xy = reinterpret_cast<const float2*>(c.coords)[ft.data_offset + i];
         const float dx = xy.x - float(ep.p[0]), dy = xy.y - float(ep.p[1]);
         const float r = sqrtf(dx * dx + dy * dy);
-        lo = fminf(lo, r);
-        hi = r <= hi ? hi : r;  // NaN passes on to hi
+        far = r <= far ? far : r;  // NaN passes on
+        if (i >= i0 && i < i1) {
+          lo = fminf(lo, r);
+          hi = r <= hi ? hi : r;
+        }
       }
       for (int o = 16; o > 0; o >>= 1) {
         lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
         const float h = __shfl_xor_sync(0xffffffffu, hi, o);
+        const float g = __shfl_xor_sync(0xffffffffu, far, o);
         hi = h <= hi ? hi : h;
+        far = g <= far ? far : g;
       }
       if (lane == 0) {
         s_rho[0][warp] = lo;
         s_rho[1][warp] = hi;
+        s_rho[2][warp] = far;
       }
       __syncthreads();
     }
@@ -527,8 +535,9 @@ k_fit_eval_radial(FitCtx c, RadialMatrix A, int cap) {
       const float zp = float(fabs(ep.p[2])), k = float(c.k);
       const double ox = (ft.nx > 0 ? ft.x0 : 0.) - ep.p[0];
       const double oy = (ft.nx > 0 ? ft.y0 : 0.) - ep.p[1];
-      // nearest and farthest distances; FP32, as the intervals have margins
-      float lo, hi;
+      // nearest and farthest distances, and the farthest of the feature's
+      // pixels; FP32, as the intervals have margins
+      float lo, hi, far;
       if (ft.nx > 0) {
         const float x0 = float(ox), x1 = x0 + float(ft.nx - 1);
         const float y0 = float(oy) + float(t0 * band);
@@ -537,19 +546,23 @@ k_fit_eval_radial(FitCtx c, RadialMatrix A, int cap) {
         const float nx = x0 > 0.f ? x0 : (x1 < 0.f ? -x1 : 0.f);
         const float ny = y0 > 0.f ? y0 : (y1 < 0.f ? -y1 : 0.f);
         const float fx = fmaxf(fabsf(x0), fabsf(x1)), fy = fmaxf(fabsf(y0), fabsf(y1));
+        const float gy = fmaxf(fabsf(float(oy)), fabsf(float(oy) + float(ft.ny - 1)));
         lo = sqrtf(nx * nx + ny * ny);
         hi = sqrtf(fx * fx + fy * fy);
+        far = sqrtf(fx * fx + gy * gy);
       } else {
         lo = s_rho[0][0];
         hi = s_rho[1][0];
+        far = s_rho[2][0];
         for (int w = 1; w < FITR_TPB / 32; ++w) {
           lo = fminf(lo, s_rho[0][w]);
           hi = s_rho[1][w] <= hi ? hi : s_rho[1][w];
+          far = s_rho[2][w] <= far ? far : s_rho[2][w];
         }
       }
       const double x = c.size_per_um * ep.p[3];  // size parameter
-      float rate = fitr_rate(k, float(x) / k, zp, hi);
-      bool ok = radial_clear(c.k, fabs(ep.p[2]), x / c.k, false) && hi < 8000.f &&
+      float rate = fitr_rate(k, float(x) / k, zp, far);
+      bool ok = radial_clear(c.k, fabs(ep.p[2]), x / c.k, false) && far < 8000.f &&
                 zp < 1e6f && isfinite(ep.p[0]) && isfinite(ep.p[1]);
       if (c.aberr != 0.) {  // the aberration's phase, as lmb_radial_intervals
         const float turn = 0.5f * fabsf(float(c.aberr)) / zp;
