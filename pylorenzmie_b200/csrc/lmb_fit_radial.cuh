@@ -20,7 +20,8 @@ namespace lmb {
 enum {
   FITR_TPB = 256,
   FITR_PAIRS = 4,     // (M, D) and its z_p, a_p, n_p derivatives
-  FITR_MAX_PARTS = 16
+  FITR_MAX_PARTS = 16,
+  FITR_SUM = 64  // patches of 64 pixels in one sum of a tile
 };
 
 // float4 per interval: 3 per pair; an odd number keeps neighbouring
@@ -326,15 +327,18 @@ __device__ inline void fitr_polynomials(const RadialMatrix& A, const double* val
 // grid of nx columns; (ax, rx, ay, ry): the grid's first pixel minus the
 // particle, split as radial_distance wants it.  A warp takes 8x8 pixels, two
 // per lane (rows y and y + 4): eight lanes on 4x2 pixels read intervals in
-// different banks.
+// different banks.  With [w0, w1) only these of the fitr_patches.
+__device__ inline int fitr_patches(int nx, int rows) {
+  return ((nx + 7) / 8) * ((rows + 7) / 8);
+}
 template <typename F>
 __device__ inline void fitr_rows(int nx, int row0, int rows, float ax, float rx, float ay,
-                                 float ry, F f) {
+                                 float ry, int w0, int w1, F f) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int pc = (nx + 7) / 8, np = pc * ((rows + 7) / 8);
+  const int pc = (nx + 7) / 8;
   const int lx = 4 * ((lane >> 3) & 1) + (lane & 3);
   const int ly = 2 * (lane >> 4) + ((lane >> 2) & 1);
-  for (int w = warp; w < np; w += FITR_TPB / 32) {
+  for (int w = w0 + warp; w < w1; w += FITR_TPB / 32) {
     const int pr = w / pc, col = 8 * (w - pr * pc) + lx, row = row0 + 8 * pr + ly;
     if (col >= nx || row >= row0 + rows) continue;
     const float X = ax + float(col);
@@ -361,10 +365,12 @@ __device__ inline RadialDistance fitr_list_distance(double dx, double dy, float*
   return radial_distance(pk(px.x, px.x), pk(lx.x, lx.x), pk(px.y, px.y), pk(lx.y, lx.y));
 }
 
-// Sum of acc over the block into out[0..FIT_NSUM) (doubles), fixed order.
+// Sum of acc over the block into (add: onto) out[0..FIT_NSUM) (doubles), fixed
+// order, FP32 within a warp.
 // Each warp halves the values it holds at every step of the butterfly, so
 // that 28 sums take 31 shuffles instead of 140.
-__device__ inline void fitr_reduce(float* acc, float (*red)[32], double* out) {
+__device__ inline void fitr_reduce(float* acc, float (*red)[32], double* out,
+                                   bool add = false) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float v[32];
 #pragma unroll
@@ -383,8 +389,8 @@ __device__ inline void fitr_reduce(float* acc, float (*red)[32], double* out) {
   red[warp][lane] = v[0];
   __syncthreads();
   if (threadIdx.x < FIT_NSUM) {
-    float s = 0.f;
-    for (int w = 0; w < FITR_TPB / 32; ++w) s += red[w][threadIdx.x];
+    double s = add ? out[threadIdx.x] : 0.;
+    for (int w = 0; w < FITR_TPB / 32; ++w) s += double(red[w][threadIdx.x]);
     out[threadIdx.x] = s;
   }
   __syncthreads();
@@ -407,25 +413,29 @@ __device__ __noinline__ void fitr_direct(const FitCtx& c, int f, const lmb_featu
       b = a + (long long)band * ft.nx;
     }
     if (b > ft.npix) b = ft.npix;
-    float acc[FIT_NSUM];
+    double* out = c.partial + (size_t)(c.tile_begin[f] + t) * FIT_NSUM;
+    constexpr int kSum = 64 * FITR_SUM;  // pixels in one sum, as the tables'
+    for (long long a0 = a; a0 < b; a0 += kSum) {
+      float acc[FIT_NSUM];
 #pragma unroll
-    for (int j = 0; j < FIT_NSUM; ++j) acc[j] = 0.f;
-    for (long long i = a + threadIdx.x; i < b; i += FITR_TPB) {
-      double x, y;
-      fit_pixel_xy(ft, c.coords, i, &x, &y);
-      const double dx = x - p[0], dy = y - p[1];
-      const Geometry<float> g =
-          geometry<float>(c.k, dx, dy, -p[2], 0., p[2], c.flags & LMB_BOHREN);
-      float H, dH[6];
-      if (c.aberr != 0.)
-        holo_jac_pixel<true>(g, coef, nm, float(c.k), &H, dH, c.aberr, dx, dy, p[2]);
-      else
-        holo_jac_pixel<false>(g, coef, nm, float(c.k), &H, dH);
-      const float r = (H - c.data[ft.data_offset + i]) * inv_noise;
-      for (int j = 0; j < 6; ++j) dH[j] *= inv_noise;
-      fitr_add<true>(r, dH, acc);
+      for (int j = 0; j < FIT_NSUM; ++j) acc[j] = 0.f;
+      for (long long i = a0 + threadIdx.x; i < min(b, a0 + kSum); i += FITR_TPB) {
+        double x, y;
+        fit_pixel_xy(ft, c.coords, i, &x, &y);
+        const double dx = x - p[0], dy = y - p[1];
+        const Geometry<float> g =
+            geometry<float>(c.k, dx, dy, -p[2], 0., p[2], c.flags & LMB_BOHREN);
+        float H, dH[6];
+        if (c.aberr != 0.)
+          holo_jac_pixel<true>(g, coef, nm, float(c.k), &H, dH, c.aberr, dx, dy, p[2]);
+        else
+          holo_jac_pixel<false>(g, coef, nm, float(c.k), &H, dH);
+        const float r = (H - c.data[ft.data_offset + i]) * inv_noise;
+        for (int j = 0; j < 6; ++j) dH[j] *= inv_noise;
+        fitr_add<true>(r, dH, acc);
+      }
+      fitr_reduce(acc, red, out, a0 > a);
     }
-    fitr_reduce(acc, red, c.partial + (size_t)(c.tile_begin[f] + t) * FIT_NSUM);
   }
 }
 
@@ -615,33 +625,40 @@ k_fit_eval_radial(FitCtx c, RadialMatrix A, int cap) {
     const float spacing = float(pl.spacing), inv_spacing = float(1. / pl.spacing);
     const float inv_half = float(2. / pl.spacing);
     for (int t = t0; t < t1; ++t) {
-      float acc[FIT_NSUM];
+      double* out = c.partial + (size_t)(c.tile_begin[f] + t) * FIT_NSUM;
+      const int rows = min(band, ft.ny - t * band);
+      const int np = ft.nx > 0 ? fitr_patches(ft.nx, rows) : 1;
+      // at most 16 pixels a thread in a row of FP32 additions: tiles of crops
+      // wider than 512 px take several sums
+      for (int w0 = 0; w0 < np; w0 += FITR_SUM) {
+        float acc[FIT_NSUM];
 #pragma unroll
-      for (int j = 0; j < FIT_NSUM; ++j) acc[j] = 0.f;
-      if (ft.nx > 0) {
-        const int row0 = t * band;
-        const float* data = c.data + ft.data_offset;
-        fitr_rows(ft.nx, row0, min(band, ft.ny - row0), pl.ax, pl.rx, pl.ay, pl.ry,
-                  [&](float x, f2 y, const RadialDistance& d, long long i, bool two) {
-                    const float d0 = data[i], d1 = two ? data[i + 4LL * ft.nx] : 0.f;
-                    fitr_pixel<kKP>(tab, d.r0.x, d.corr.x, d.y.x, x, y.x, inv_spacing, spacing,
-                                    inv_half, pl.lo, pl.n, d0, inv_noise, acc);
-                    if (two)
-                      fitr_pixel<kKP>(tab, d.r0.y, d.corr.y, d.y.y, x, y.y, inv_spacing,
-                                      spacing, inv_half, pl.lo, pl.n, d1, inv_noise, acc);
-                  });
-      } else {
-        const long long a = (long long)t * FITR_TILE, b = min(a + FITR_TILE, ft.npix);
-        for (long long i = a + threadIdx.x; i < b; i += FITR_TPB) {
-          const float2 xy = reinterpret_cast<const float2*>(c.coords)[ft.data_offset + i];
-          float x, y;
-          const RadialDistance d = fitr_list_distance(double(xy.x) - ep.p[0],
-                                                      double(xy.y) - ep.p[1], &x, &y);
-          fitr_pixel<kKP>(tab, d.r0.x, d.corr.x, d.y.x, x, y, inv_spacing, spacing, inv_half,
-                          pl.lo, pl.n, c.data[ft.data_offset + i], inv_noise, acc);
+        for (int j = 0; j < FIT_NSUM; ++j) acc[j] = 0.f;
+        if (ft.nx > 0) {
+          const float* data = c.data + ft.data_offset;
+          fitr_rows(ft.nx, t * band, rows, pl.ax, pl.rx, pl.ay, pl.ry, w0,
+                    min(np, w0 + FITR_SUM),
+                    [&](float x, f2 y, const RadialDistance& d, long long i, bool two) {
+                      const float d0 = data[i], d1 = two ? data[i + 4LL * ft.nx] : 0.f;
+                      fitr_pixel<kKP>(tab, d.r0.x, d.corr.x, d.y.x, x, y.x, inv_spacing,
+                                      spacing, inv_half, pl.lo, pl.n, d0, inv_noise, acc);
+                      if (two)
+                        fitr_pixel<kKP>(tab, d.r0.y, d.corr.y, d.y.y, x, y.y, inv_spacing,
+                                        spacing, inv_half, pl.lo, pl.n, d1, inv_noise, acc);
+                    });
+        } else {
+          const long long a = (long long)t * FITR_TILE, b = min(a + FITR_TILE, ft.npix);
+          for (long long i = a + threadIdx.x; i < b; i += FITR_TPB) {
+            const float2 xy = reinterpret_cast<const float2*>(c.coords)[ft.data_offset + i];
+            float x, y;
+            const RadialDistance d = fitr_list_distance(double(xy.x) - ep.p[0],
+                                                        double(xy.y) - ep.p[1], &x, &y);
+            fitr_pixel<kKP>(tab, d.r0.x, d.corr.x, d.y.x, x, y, inv_spacing, spacing,
+                            inv_half, pl.lo, pl.n, c.data[ft.data_offset + i], inv_noise, acc);
+          }
         }
+        fitr_reduce(acc, red, out, w0 > 0);
       }
-      fitr_reduce(acc, red, c.partial + (size_t)(c.tile_begin[f] + t) * FIT_NSUM);
     }
   }
 }
@@ -793,7 +810,8 @@ k_vjp_radial(GradPlan pl, RadialMatrix A, int cap, const lmb_sphere* __restrict_
           add(d.r0.x, d.corr.x, d.y.x, x, y, i);
         }
       } else {
-        fitr_rows(int(pl.nx), row0, rows, fax, frx, fay, fry,
+        fitr_rows(int(pl.nx), row0, rows, fax, frx, fay, fry, 0,
+                  fitr_patches(int(pl.nx), rows),
                   [&](float x, f2 y, const RadialDistance& d, long long i, bool two) {
                     add(d.r0.x, d.corr.x, d.y.x, x, y.x, i);
                     if (two) add(d.r0.y, d.corr.y, d.y.y, x, y.y, i + 4 * pl.nx);
