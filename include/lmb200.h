@@ -418,9 +418,8 @@ typedef struct lmb_fit_settings {
   int max_iterations; /* hard cap on evaluations per call, >= 1 */
   int tile_config;    /* launch shape of the evaluation kernel, 0 = default;
                          see lmb_fit_tile_config; or LMB_FIT_RADIAL */
-  int reach;          /* with LMB_FIT_RADIAL, >= 0: an upper estimate of a
-                         pixel's distance from its sphere (px), which sets
-                         the room for the tables; 0: unknown */
+  int reach;          /* with LMB_FIT_RADIAL, >= 0: the room for the tables,
+                         from lmb_fit_radial_reach; 0: as much as there is */
 } lmb_fit_settings;
 
 /*
@@ -431,6 +430,15 @@ typedef struct lmb_fit_settings {
  * by pixel).  The launch shapes of lmb_fit_tile_config sum at every pixel.
  */
 #define LMB_FIT_RADIAL 100
+/*
+ * Host only: lmb_fit_settings.reach of a batch with these start values
+ * (host), or 0 where a launch shape is the better evaluation: a quarter or
+ * more of the spheres too near the plane for tables, or no room for them.
+ * far: an upper estimate of a pixel's distance from its sphere (px) during
+ * the fit; aberration as in lmb_fit_batch_aberrated.
+ */
+int lmb_fit_radial_reach(const lmb_sphere *starts, int n, double far,
+                         double k, double magnification, double aberration);
 
 /*
  * Launch shapes of the fit's evaluation kernel (threads per CTA, pixels per

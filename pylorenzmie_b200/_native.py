@@ -129,6 +129,7 @@ _SIGNATURES = {
     'lmb_hologram_vjp_grid': (_i, [ctypes.POINTER(Grid), _vp, _ll, _vp, _vp,
                                    _i, _vp, _vp, _vp, _i, _d, _d, _i, _vp,
                                    _vp, _vp, _sz, _vp]),
+    'lmb_fit_radial_reach': (_i, [_vp, _i, _d, _d, _d, _d]),
     'lmb_fit_workspace_bytes': (_sz, [_i, _ll, _i]),
     'lmb_chi2_workspace_bytes': (_sz, [_ll, _i]),
     'lmb_chi2_batch': (_i, [_vp, _ll, _vp, _d, _vp, _vp, _i, _vp, _vp, _i,

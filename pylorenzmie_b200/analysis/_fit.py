@@ -320,7 +320,7 @@ def fit_device(d_feat, d_data, d_coords, d_params, nfeatures, total_pixels,
     aberrated model (lmb_fit_batch_aberrated, or lmb_fit_batch_streamed
     with the coefficient).  ``tile_config``: a launch shape
     (lmb_fit_tile_config), or LMB_FIT_RADIAL with ``reach``
-    (PackedFeatures.reach).'''
+    (lmb_fit_radial_reach).'''
     dev = d_data.device
     lib = _native.load()
     settings = dict(DEFAULT_SETTINGS if settings is None else settings)
@@ -419,17 +419,15 @@ def default_shape(nfeatures):
     return SMALL_SHAPE if nfeatures < SMALL_BATCH else 0
 
 
-# Reach (k times px) of the features that the evaluation from radial tables
-# takes: the table's room in shared memory, ~650 intervals of 0.65 radian
-# (crops of 500 px at the default magnification).  Measured on a B200 against
-# launch shape 0: an evaluation of 256 features of 201x201 px 1.14 -> 0.13 ms.
-# A table costs ~15 us of serial FP64 work, whatever the pixels, so batches
-# of fewer than SMALL_BATCH features of at most RADIAL_PIXELS pixels (a
-# frame's features on their random subsets) keep SMALL_SHAPE: 32 features of
-# 1460 px 22 against 16 us.  Multilayer spheres keep the sums at every pixel:
-# their uncertainties in a_p and z_p can follow the rounding of the Jacobian
-# (a batch of 24 moved by up to 9e-5 of itself, towards the 64-bit values).
-RADIAL_REACH = 400.
+# The evaluation from radial tables is taken where lmb_fit_radial_reach finds
+# room.  Measured on a B200 against launch shape 0: an evaluation of 256
+# features of 201x201 px 1.14 -> 0.13 ms.  A table costs ~15 us of serial FP64
+# work, whatever the pixels, so batches of fewer than SMALL_BATCH features of
+# at most RADIAL_PIXELS pixels (a frame's features on their random subsets)
+# keep SMALL_SHAPE: 32 features of 1460 px 22 against 16 us.  Multilayer
+# spheres keep the sums at every pixel: their uncertainties in a_p and z_p can
+# follow the rounding of the Jacobian (a batch of 24 moved by up to 9e-5 of
+# itself, towards the 64-bit values).
 RADIAL_PIXELS = 4096
 LARGE = 'large'
 
@@ -450,16 +448,17 @@ def evaluation(packed, starts, instrument, variables, nmax_cap, layers, dev,
     npix = packed.features['npix']
     if layers is None and (B >= SMALL_BATCH or (
             npix[0] if B == 1 else npix.max()) > RADIAL_PIXELS):
-        reach = packed.reach(starts)
-        if reach * float(instrument.wavenumber()) > RADIAL_REACH:
-            reach = 0
+        reach = _native.load().lmb_fit_radial_reach(
+            starts.ctypes.data, B, packed.reach(starts),
+            float(instrument.wavenumber()), float(instrument.magnification),
+            float(aberration))
     shape = default_shape(B)
     if autotune and not aberration and not (reach and autotune is LARGE):
         from .. import autotune as _tuner     # the aberrated fit has one shape
         shape = _tuner.tune(packed, starts, instrument, variables, nmax_cap,
                             layers, dev)
     if reach:
-        return _native.LMB_FIT_RADIAL, int(np.ceil(reach))
+        return _native.LMB_FIT_RADIAL, reach
     return shape, 0
 
 

@@ -33,6 +33,10 @@ __host__ __device__ constexpr int fitr_funcs(bool kp) { return 2 * (FITR_PAIRS +
 // pixel, fitr_rate): the degree-5 polynomials of half a spacing to either
 // side are then off by 2 (0.65 / 4)^6 / 6! = 5e-8 of its amplitude.
 #define FITR_SPACING 0.65
+// The largest reach (k times px, times the rate where that is above 1) that
+// lmb_fit_radial_reach gives: the room of ~620 intervals in shared memory,
+// crops of 500 px at a magnification of 0.048 um.
+#define FITR_REACH 400.
 
 // The fastest oscillation of H along rho, in units of k: the carrier of the
 // interference term turns by k sin(theta), theta the steepest ray from the
