@@ -334,13 +334,14 @@ def b200_arm(args):
     if args.tile_config is None:
         tile_config = _fit.evaluation(b0['packed'], b0['start'], inst,
                                       variables, b0['cap'], None, dev,
-                                      _fit.LARGE, 0.)[0]
+                                      None, 0.)[0]
     else:
         tile_config = int(args.tile_config)
     radial = tile_config == _native.LMB_FIT_RADIAL
     for b in batches:
-        b['reach'] = (int(np.ceil(b['packed'].reach(b['start'])))
-                      if radial else 0)
+        b['reach'] = _fit.evaluation(
+            b['packed'], b['start'], inst, variables, b['cap'], None, dev,
+            False, 0.)[1] if radial else 0
 
     peak = ctypes.c_double()
     _native.check(lib.lmb_measure_fp32_peak(ctypes.byref(peak),

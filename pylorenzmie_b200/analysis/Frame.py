@@ -186,7 +186,7 @@ class Frame(Hologram):
             params, res, _ = _fit.fit_items(
                 items, starts, members[0].model.instrument, opt0.variables,
                 opt0.settings, device=members[0].model.device, layers=layers,
-                autotune=_fit.default_autotune(len(members)),
+                autotune=None,
                 aberration=opt0._aberration())
             for j, f in enumerate(members):
                 f.optimizer._data = np.asarray(items[j][0])

@@ -293,10 +293,11 @@ class Optimizer(LMObject):
                     is kept, their outer radius and index are fitted
         starts    : array (B, 6) of x_p, y_p, z_p, a_p, n_p, k_p (overrides
                     the particles' start values)
-        autotune  : time the evaluation kernel's launch shapes once per
-                    problem class and use the fastest where the radial
-                    tables do not apply (default: timed only there, for
-                    batches of 64 features or more)
+        autotune  : time the ways to evaluate the features, the radial
+                    tables where they apply and the launch shapes of the
+                    sums at every pixel, once per problem class and use the
+                    fastest (default: only where the tables do not apply,
+                    for batches of 64 features or more)
         chunks    : pipeline depth: the batch is fitted in this many parts,
                     each on its own stream, so that converting and copying
                     one part overlaps the fit of the previous one (default:
@@ -317,8 +318,6 @@ class Optimizer(LMObject):
                 getattr(p, 'r_0', (0., 0., 0.)), float)), p.a_p, p.n_p,
                 getattr(p, 'k_p', 0.)] for p in particles], dtype=float)
         items = [self._pixels(h) for h in holograms]
-        if autotune is None:
-            autotune = _fit.default_autotune(len(holograms))
         params, res, npix = _fit.fit_items(
             items, starts, self.model.instrument, self.variables,
             self.settings, device=self.model.device, layers=layers,
@@ -334,8 +333,9 @@ class Optimizer(LMObject):
         batches : iterable of (holograms, starts) or (holograms,
                   particles) pairs; starts an array (B, 6), particles a
                   list of Sphere or LayeredSphere start values
-        autotune: time the evaluation kernel's launch shapes (default: as
-                  optimize_batch, by the first batch's size)
+        autotune: as optimize_batch, timed on the first batch before the
+                  pipeline starts; a launch shape found there serves the
+                  later batches
         depth   : fits running at once; the next batch is converted and
                   copied while they run.  Default 2, which keeps the GPU
                   busy; 4 when the first batch holds LayeredSphere
@@ -346,7 +346,6 @@ class Optimizer(LMObject):
                 set(self.variables) <= set(PARAM_KEYS)):
             raise ValueError('optimize_stream fits sphere parameters only')
         variables = list(self.variables)
-        first = [True]
 
         def items():
             for holograms, second in batches:
@@ -361,15 +360,10 @@ class Optimizer(LMObject):
                                               float)), p.a_p, p.n_p,
                                         getattr(p, 'k_p', 0.)]
                                        for p in second], dtype=float)
-                if first[0]:
-                    first[0] = False
-                    self._stream_tune = (
-                        autotune if autotune is not None
-                        else _fit.default_autotune(len(holograms)))
                 yield [self._pixels(h) for h in holograms], starts, layers
 
         gen = items()
-        # the first batch decides autotuning before the pipeline starts
+        # the first batch decides the depth
         try:
             head = next(gen)
         except StopIteration:
@@ -382,7 +376,7 @@ class Optimizer(LMObject):
             depth = 2 if head[2] is None else 4
         for params, res, npix in _fit.fit_stream(
                 chain(), self.model.instrument, variables, self.settings,
-                device=self.model.device, autotune=self._stream_tune,
+                device=self.model.device, autotune=autotune,
                 depth=depth, aberration=self._aberration()):
             yield batch_frame(params, res, npix, variables)
 

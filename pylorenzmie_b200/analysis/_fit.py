@@ -429,20 +429,14 @@ def default_shape(nfeatures):
 # follow the rounding of the Jacobian (a batch of 24 moved by up to 9e-5 of
 # itself, towards the 64-bit values).
 RADIAL_PIXELS = 4096
-LARGE = 'large'
-
-
-def default_autotune(nfeatures):
-    '''autotune of a batch whose caller does not say: LARGE (where the
-    radial tables do not apply) for 64 features or more.'''
-    return LARGE if nfeatures >= SMALL_BATCH else False
 
 
 def evaluation(packed, starts, instrument, variables, nmax_cap, layers, dev,
                autotune, aberration):
     '''(tile_config, reach) of a batch's evaluation kernel: radial tables
-    where they apply, else a launch shape that sums at every pixel, timed
-    with ``autotune`` (LARGE: only if it is needed).'''
+    where they apply, else a launch shape that sums at every pixel.  With
+    ``autotune`` the fastest of these, timed; None: timed where the tables do
+    not apply, for SMALL_BATCH features or more.'''
     B = starts.shape[0]
     reach = 0
     npix = packed.features['npix']
@@ -452,14 +446,14 @@ def evaluation(packed, starts, instrument, variables, nmax_cap, layers, dev,
             starts.ctypes.data, B, packed.reach(starts),
             float(instrument.wavenumber()), float(instrument.magnification),
             float(aberration))
-    shape = default_shape(B)
-    if autotune and not aberration and not (reach and autotune is LARGE):
-        from .. import autotune as _tuner     # the aberrated fit has one shape
-        shape = _tuner.tune(packed, starts, instrument, variables, nmax_cap,
-                            layers, dev)
-    if reach:
-        return _native.LMB_FIT_RADIAL, reach
-    return shape, 0
+    if autotune is None:
+        autotune = B >= SMALL_BATCH and not reach
+    config = _native.LMB_FIT_RADIAL if reach else default_shape(B)
+    if autotune and not aberration:       # the aberrated fit has one shape
+        from .. import autotune as _tuner
+        config = _tuner.tune(packed, starts, instrument, variables, nmax_cap,
+                             layers, dev, reach=reach)
+    return config, reach if config == _native.LMB_FIT_RADIAL else 0
 
 
 def fit_packed(packed, starts, instrument, variables, settings=None,
@@ -749,7 +743,8 @@ def fit_stream(batches, instrument, variables, settings=None, device=None,
     rounds holds one slot while later batches pass through the others;
     finished batches wait, up to 8 x depth of them, to be yielded in order.
     A pinned buffer is rewritten only after its previous copy has
-    completed.'''
+    completed.  ``autotune``: as evaluation, on the first batch; a launch
+    shape that it finds serves the later ones.'''
     dev = get_device(device)
     _, s_copy = _fit_streams(dev)
     nstage = depth + 1
@@ -757,6 +752,7 @@ def fit_stream(batches, instrument, variables, settings=None, device=None,
         _stream_staging.append(_Staging())
     slots = _Slots(depth)
     done_events = [None] * nstage
+    first, shape = True, None       # a launch shape that the tuner chose
     k = 0
 
     def launch(fit_slot, ev, views, B, total, nmax_cap, starts, layers,
@@ -784,9 +780,17 @@ def fit_stream(batches, instrument, variables, settings=None, device=None,
                 continue
             nmax_cap = fit_capacity(starts, float(instrument.n_m),
                                     float(instrument.wavelength), layers)
+            # timed on the first batch only, before other fits run
             tile_config, reach = evaluation(packed, starts, instrument,
                                             variables, nmax_cap, layers, dev,
-                                            autotune, aberration)
+                                            autotune if first else False,
+                                            aberration)
+            if first and not reach and not aberration and (
+                    autotune or (autotune is None and B >= SMALL_BATCH)):
+                shape = tile_config
+            elif shape is not None and (autotune or not reach):
+                tile_config, reach = shape, 0
+            first = False
             slot = k % nstage
             if done_events[slot] is not None:
                 done_events[slot].synchronize()  # its last copy has landed

@@ -2,11 +2,12 @@
 
 The evaluation kernel exists in several launch shapes (threads per CTA,
 pixels per thread, register cap, CTA- or warp-granular tiles; see
-``lmb_fit_tile_config``).  For a problem class -- partial-wave capacity
-bucket and mean crop size bucket, on one GPU model -- the tuner times every
-shape on a probe batch cut from the caller's own features (device time of
-the evaluation launches, measured by the library with CUDA events) and
-keeps the fastest.  Results are cached in memory and in a JSON file
+``lmb_fit_tile_config``), beside the one that reads radial tables.  For a
+problem class -- partial-wave capacity bucket and mean crop size bucket, on
+one GPU model -- the tuner times every shape, and the tables where they
+apply, on a probe batch cut from the caller's own features (device time of
+the evaluation launches, measured by the library with CUDA events) and keeps
+the fastest.  Results are cached in memory and in a JSON file
 (``$LMB200_AUTOTUNE_CACHE`` or ``~/.cache/pylorenzmie_b200/autotune.json``).
 '''
 import ctypes
@@ -59,11 +60,12 @@ def _bucket(value, edges):
 
 
 def problem_key(gpu_name, nmax_cap, mean_pixels, layered=False,
-                batch=PROBE_FEATURES):
+                batch=PROBE_FEATURES, tables=False):
     return (f'{gpu_name}|nmax<={_bucket(nmax_cap, NMAX_BUCKETS)}|'
             f'px<={_bucket(mean_pixels, PIXEL_BUCKETS)}|'
             f'b<={_bucket(batch, BATCH_BUCKETS)}|'
-            f'{"layered" if layered else "sphere"}')
+            f'{"layered" if layered else "sphere"}'
+            f'{"|tables" if tables else ""}')
 
 
 def _load_file():
@@ -98,15 +100,17 @@ def lookup(key):
 
 
 def tune(packed, starts, instrument, variables, nmax_cap, layers=None,
-         device=None, repeats=2):
-    '''Best shape index for this batch's problem class (timed if unknown).'''
+         device=None, repeats=2, reach=0):
+    '''Best tile_config for this batch's problem class (timed if unknown): a
+    launch shape or, with a ``reach`` (lmb_fit_radial_reach), the tables.'''
     import torch
     from .analysis import _fit
     dev = device if device is not None else torch.device('cuda')
     name = torch.cuda.get_device_name(dev)
     B = packed.features.shape[0]
     mean_px = float(packed.features['npix'].mean()) if B else 0.
-    key = problem_key(name, nmax_cap, mean_px, layers is not None, B)
+    key = problem_key(name, nmax_cap, mean_px, layers is not None, B,
+                      reach > 0)
     hit = lookup(key)
     if hit is not None:
         return int(hit['config'])
@@ -128,14 +132,18 @@ def tune(packed, starts, instrument, variables, nmax_cap, layers=None,
     d_feat, d_data, d_coords, d_params = _fit.upload(probe, starts[:n], dev)
     p0 = d_params.clone()
     timings = {}
-    for (i, _, _, _) in shapes():
+    configs = [i for i, _, _, _ in shapes()]
+    if reach:
+        configs.append(_native.LMB_FIT_RADIAL)
+    for i in configs:
         best = None
         for _ in range(repeats):
             d_params.copy_(p0)
             _, fs = _fit.fit_device(d_feat, d_data, d_coords, d_params, n,
                                     probe.total, instrument, variables, None,
                                     nmax_cap, starts[:n], stats=True,
-                                    tile_config=i, layers=sub_layers)
+                                    tile_config=i, layers=sub_layers,
+                                    reach=reach)
             per = fs.eval_ms / max(fs.eval_launches, 1)
             best = per if best is None else min(best, per)
         timings[i] = best
