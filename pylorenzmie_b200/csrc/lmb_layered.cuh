@@ -262,7 +262,8 @@ LMB_HD void layered_shell_up(const LayeredScalars& s, int ii, const dz* d1a,
 }
 
 // a_n, b_n and their (a_p, n_p) derivatives from the outer Ha, Hb and the
-// medium's psi, zeta (with d/dx); same output layout as mie_coefficient.
+// medium's psi, zeta (with d/dx): out = {a_n, b_n}, dout = {da/da_p, db/da_p,
+// da/dn_p, db/dn_p}.
 LMB_HD void layered_coefficient(const LayeredScalars& s, int n, const dz& ha,
                                 const dz& hb, const double* psi,
                                 const double* psix, const zd* zeta,

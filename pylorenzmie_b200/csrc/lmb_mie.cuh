@@ -309,15 +309,4 @@ LMB_HD zd mie_coefficient_one(const MieScalars& s, int n, int which,
   return v;
 }
 
-// Both a_n, b_n (out[0], out[1]) and, if dout != 0, their derivatives
-// dout = {da/da_p, db/da_p, da/dn_p, db/dn_p}, for 1 <= n <= nmax.
-LMB_HD void mie_coefficient(const MieScalars& s, int n, const zd* d1in,
-                            const zd* d1inz, const double* psi,
-                            const double* psix, const zd* zeta,
-                            const zd* zetax, zd* out, zd* dout) {
-  for (int j = 0; j < 2; ++j)
-    out[j] = mie_coefficient_one(s, n, j, d1in, d1inz, psi, psix, zeta, zetax,
-                                 dout ? dout + j : (zd*)0);
-}
-
 }  // namespace lmb

@@ -8,6 +8,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <cmath>
 #include <vector>
 
 #include "lmb_layered.cuh"
@@ -21,43 +22,67 @@ using namespace lmb;
 
 #define API extern "C"
 
-// ab: [cap+1][2] complex (4 doubles per n), dab: [cap+1][4] complex.
-API int h_sphere_ab(double a_p, double n_p, double k_p, double n_m, double lam,
-                int cap, double* ab, double* dab, int* nmax) {
+// ab: [cap+1][2] complex (4 doubles per n), dab: [cap+1][4] complex.  The
+// phases of block_sphere_ab, in its order; its fallback is taken where the
+// waves inside overflow, or with quotients != 0.
+static int sphere_ab_impl(double a_p, double n_p, double k_p, double n_m, double lam, int cap,
+                          double* ab, double* dab, int* nmax, bool quotients) {
   MieScalars s = mie_setup(a_p, n_p, k_p, n_m, lam);
   *nmax = s.nmax;
   if (s.nmax > cap) return 3;
-  std::vector<zd> d1in(s.nmax + 1), d1inz(s.nmax + 1), zeta(s.nmax + 1),
-      zetax(s.nmax + 1);
-  std::vector<double> d1m(s.nmax + 1), d1mx(s.nmax + 1), psi(s.nmax + 1),
-      psix(s.nmax + 1);
-  std::vector<zd> nz(s.nmax + 1), nz2(s.nmax + 1);
-  std::vector<double> nx(s.nmax + 1), nx2(s.nmax + 1);
-  for (int n = 1; n <= s.nmax; ++n) {  // as the kernel's two warps
-    mie_orders_inside(s, n, nz.data(), nz2.data());
-    mie_orders_medium(s, n, nx.data(), nx2.data());
+  const int nm = s.nmax;
+  std::vector<zd> q(nm + 1), rr(nm + 1), d1in(nm + 1), d1inz(nm + 1), zeta(nm + 1),
+      zetax(nm + 1);
+  std::vector<double> d1m(nm + 1), d1mx(nm + 1), psi(nm + 1), psix(nm + 1), nx(nm + 1),
+      nx2(nm + 1);
+  const zd iz = recip(s.x * s.m);
+  mie_inside_waves(nm, iz, q.data());
+  if (!quotients && std::isfinite(q[0].re) && std::isfinite(q[0].im)) {
+    for (int n = 1; n <= nm; ++n)
+      mie_inside_order(n, iz, q.data(), d1in.data(), dab ? rr.data() : (zd*)0, d1inz.data());
+    d1in[nm] = mk(0., 0.);
+    if (dab) mie_inside_tangent(nm, rr.data(), d1inz.data());
+  } else {
+    for (int n = 1; n <= nm; ++n) mie_orders_inside(s, n, q.data(), rr.data());
+    mie_d1_inside(s, q.data(), rr.data(), d1in.data(), d1inz.data());
   }
-  mie_d1_inside(s, nz.data(), nz2.data(), d1in.data(), d1inz.data());
+  for (int n = 1; n <= nm; ++n) mie_orders_medium(s, n, nx.data(), nx2.data());
   mie_d1_medium(s, nx.data(), nx2.data(), d1m.data(), d1mx.data());
-  mie_upward(s, nx.data(), nx2.data(), d1m.data(), d1mx.data(), psi.data(),
-             psix.data(), zeta.data(), zetax.data());
+  const double sx = sin(s.x), cx = cos(s.x);
+  for (int n = 1; n <= nm; ++n) mie_psi_order(n, d1m.data(), d1mx.data(), nx.data(), nx2.data());
+  mie_psi(nm, sx, cx, nx.data(), nx2.data(), psi.data(), psix.data());
+  for (int n = 1; n < nm; ++n)
+    mie_psi_inverse(n, psi.data(), psix.data(), d1m.data(), d1mx.data());
+  for (int part = 0; part < 2; ++part)
+    mie_zeta(nm, part, s.x, sx, cx, nx.data(), nx2.data(), d1m.data(), d1mx.data(),
+             reinterpret_cast<double*>(zeta.data()) + part,
+             reinterpret_cast<double*>(zetax.data()) + part);
   memset(ab, 0, sizeof(double) * 4 * (cap + 1));
   if (dab) memset(dab, 0, sizeof(double) * 8 * (cap + 1));
-  for (int n = 1; n <= s.nmax; ++n) {
-    zd out[2], dout[4];
-    mie_coefficient(s, n, d1in.data(), d1inz.data(), psi.data(), psix.data(),
-                    zeta.data(), zetax.data(), out, dab ? dout : 0);
-    ab[4 * n + 0] = out[0].re;
-    ab[4 * n + 1] = out[0].im;
-    ab[4 * n + 2] = out[1].re;
-    ab[4 * n + 3] = out[1].im;
-    if (dab)
-      for (int j = 0; j < 4; ++j) {
-        dab[8 * n + 2 * j] = dout[j].re;
-        dab[8 * n + 2 * j + 1] = dout[j].im;
-      }
-  }
+  for (int n = 1; n <= nm; ++n)
+    for (int j = 0; j < 2; ++j) {
+      zd d[3];
+      const zd v = mie_coefficient_one(s, n, j, d1in.data(), d1inz.data(), psi.data(),
+                                       psix.data(), zeta.data(), zetax.data(), dab ? d : (zd*)0);
+      ab[4 * n + 2 * j] = v.re;
+      ab[4 * n + 2 * j + 1] = v.im;
+      if (dab)
+        for (int i = 0; i < 2; ++i) {
+          dab[8 * n + 4 * i + 2 * j] = d[2 * i].re;
+          dab[8 * n + 4 * i + 2 * j + 1] = d[2 * i].im;
+        }
+    }
   return 0;
+}
+
+API int h_sphere_ab(double a_p, double n_p, double k_p, double n_m, double lam,
+                    int cap, double* ab, double* dab, int* nmax) {
+  return sphere_ab_impl(a_p, n_p, k_p, n_m, lam, cap, ab, dab, nmax, false);
+}
+
+API int h_sphere_ab_quotients(double a_p, double n_p, double k_p, double n_m, double lam,
+                              int cap, double* ab, double* dab, int* nmax) {
+  return sphere_ab_impl(a_p, n_p, k_p, n_m, lam, cap, ab, dab, nmax, true);
 }
 
 // Multilayer coefficients: radii [L], idx [L][2]; outputs as h_sphere_ab.

@@ -37,6 +37,7 @@ def load():
         tmp.replace(LIB)
     lib = ctypes.CDLL(str(LIB))
     lib.h_sphere_ab.argtypes = [ctypes.c_double] * 5 + [ctypes.c_int, _dp, _dp, _ip]
+    lib.h_sphere_ab_quotients.argtypes = lib.h_sphere_ab.argtypes
     lib.h_layered_ab.argtypes = [_dp, _dp, ctypes.c_int, ctypes.c_double,
                                  ctypes.c_double, ctypes.c_int, _dp, _dp, _ip]
     lib.h_layered_ab_split.argtypes = lib.h_layered_ab.argtypes
@@ -85,13 +86,15 @@ class Harness:
     def __init__(self):
         self.lib = load()
 
-    def sphere_ab(self, a_p, n_p, k_p, n_m, wavelength, cap=1024, deriv=False):
+    def sphere_ab(self, a_p, n_p, k_p, n_m, wavelength, cap=1024, deriv=False,
+                  quotients=False):
         ab = np.zeros((cap + 1, 2, 2))
         dab = np.zeros((cap + 1, 4, 2)) if deriv else None
         nmax = ctypes.c_int()
-        st = self.lib.h_sphere_ab(a_p, n_p, k_p, n_m, wavelength, cap, ptr(ab),
-                                  ptr(dab) if deriv else None,
-                                  ctypes.byref(nmax))
+        fn = self.lib.h_sphere_ab_quotients if quotients else \
+            self.lib.h_sphere_ab
+        st = fn(a_p, n_p, k_p, n_m, wavelength, cap, ptr(ab),
+                ptr(dab) if deriv else None, ctypes.byref(nmax))
         if st != 0:
             raise ValueError(f'nmax {nmax.value} above cap')
         n = nmax.value
