@@ -151,6 +151,7 @@ int lmb_hologram_aberrated(const double *coords, long long npts,
  *                      length divides npts); the pixels that are not finite
  *                      or not in the first one's plane; then, as doubles,
  *                      the bounds min x, min y, max x, max y.
+ * lmb_plane_probe      the same and an eighth value, the first pixel's z.
  * lmb_radial_intervals host only: the table intervals a particle that
  *                      these n spheres (host records, a_p the outer radius)
  *                      need for npts pixels, or 0 where the tables do not
@@ -175,6 +176,8 @@ typedef struct lmb_grid {
 } lmb_grid;
 int lmb_grid_probe(const double *coords, long long npts,
                    unsigned long long *out, void *stream);
+int lmb_plane_probe(const double *coords, long long npts,
+                    unsigned long long *out, void *stream);
 /* The same of coordinates in host memory, out in host memory too. */
 int lmb_grid_probe_host(const double *coords, long long npts, long long *out);
 int lmb_radial_intervals(const lmb_grid *grid, long long npts,

@@ -98,6 +98,7 @@ _SIGNATURES = {
     'lmb_hologram_aberrated': (_i, [_vp, _ll, _vp, _vp, _i, _vp, _vp, _i,
                                     _d, _i, _d, _vp, _vp]),
     'lmb_grid_probe': (_i, [_vp, _ll, _vp, _vp]),
+    'lmb_plane_probe': (_i, [_vp, _ll, _vp, _vp]),
     'lmb_grid_probe_host': (_i, [_vp, _ll, _vp]),
     'lmb_radial_intervals': (_i, [ctypes.POINTER(Grid), _ll, _vp, _i, _d, _d,
                                   _i, _d]),

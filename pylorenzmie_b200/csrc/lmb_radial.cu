@@ -19,7 +19,7 @@ namespace {
 // Is a coordinate list a unit-step pixel grid, or at least in one plane?
 
 enum { PROBE_ROW, PROBE_OFF_GRID, PROBE_OFF_PLANE, PROBE_LO_X, PROBE_LO_Y, PROBE_HI_X,
-       PROBE_HI_Y };
+       PROBE_HI_Y, PROBE_Z };
 
 // Doubles as unsigned integers in the same order, and back.
 __device__ inline unsigned long long ordered(double v) {
@@ -87,9 +87,10 @@ __global__ void k_probe_check(const double* __restrict__ coords, long long npts,
       else atomicMax(out + PROBE_LO_X + j, b[j]);
 }
 
-__global__ void k_probe_bounds(unsigned long long* out) {
+__global__ void k_probe_bounds(unsigned long long* out, const double* z) {
   for (int j = PROBE_LO_X; j <= PROBE_HI_Y; ++j)
     out[j] = (unsigned long long)__double_as_longlong(unordered(out[j]));
+  if (z) out[PROBE_Z] = (unsigned long long)__double_as_longlong(*z);
 }
 
 // ---------------------------------------------------------------------------
@@ -744,21 +745,31 @@ int grid_common(bool holo, const lmb_grid* grid, const lmb_sphere* spheres,
   return LMB_OK;
 }
 
-}  // namespace
-
-extern "C" {
-
-int lmb_grid_probe(const double* coords, long long npts, unsigned long long* out,
-                   void* stream) {
+int probe(const double* coords, long long npts, unsigned long long* out, bool z,
+          void* stream) {
   if (npts < 1 || !coords || !out) return LMB_ERR_ARG;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const unsigned blocks = unsigned(std::min<long long>((npts + 255) / 256, 1184));
   k_probe_init<<<1, 1, 0, st>>>(npts, out);
   k_probe_row<<<blocks, 256, 0, st>>>(coords, npts, out);
   k_probe_check<<<blocks, 256, 0, st>>>(coords, npts, out);
-  k_probe_bounds<<<1, 1, 0, st>>>(out);
+  k_probe_bounds<<<1, 1, 0, st>>>(out, z ? coords + 2 * npts : nullptr);
   LMB_CK(cudaGetLastError());
   return LMB_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int lmb_grid_probe(const double* coords, long long npts, unsigned long long* out,
+                   void* stream) {
+  return probe(coords, npts, out, false, stream);
+}
+
+int lmb_plane_probe(const double* coords, long long npts, unsigned long long* out,
+                    void* stream) {
+  return probe(coords, npts, out, true, stream);
 }
 
 int lmb_radial_intervals(const lmb_grid* grid, long long npts, const lmb_sphere* spheres,

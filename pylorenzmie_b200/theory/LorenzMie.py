@@ -143,17 +143,20 @@ class LorenzMie(LMObject):
     @property
     def _grid(self):
         '''The coordinates as pixels of one plane (K.make_grid), or None;
-        found once for each device copy of the coordinates.'''
+        found once for each device copy of the coordinates, from that copy
+        or, for few pixels, from what it is made of.'''
         if self._grid_dev is None:
-            host = self._coordinates
-            npts = host.shape[1]
+            npts = self._coordinates.shape[1]
             found = None
-            if 0 < npts <= 16384:      # less than the launches would take
-                found = K.probe_host(np.ascontiguousarray(host))
+            if self._coords_dev is None and 0 < npts <= 16384:
+                # less than the launches would take
+                host = np.ascontiguousarray(self._coordinates)
+                found = K.probe_host(host)
+                self._coords_dev = torch.from_numpy(host).to(self.device)
             elif npts:
                 found = K.probe_grid(self._coords).cpu().numpy()
             self._grid_dev = (None if found is None else
-                              K.make_grid(host[2, 0], npts, found),)
+                              K.probed_grid(npts, found),)
         return self._grid_dev[0]
 
     # ------------------------------------------------------------------
@@ -212,8 +215,8 @@ class LorenzMie(LMObject):
     def _items(self, particle_lists, cartesian, bohren, field):
         flat = [p for plist in particle_lists for p in plist]
         if not any(type(p) is not Sphere and K.is_layered(p) for p in flat):
-            coords = self._coords
-            return K.render(self._grid, coords, _records(flat),
+            grid = self._grid
+            return K.render(grid, self._coords, _records(flat),
                             [len(pl) for pl in particle_lists],
                             self.instrument, cartesian, bohren,
                             self._aberration(), field, self.double_precision)

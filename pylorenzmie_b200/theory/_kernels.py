@@ -228,21 +228,28 @@ def field(coords, spheres, item_start, ab, nmax, cap, k, cartesian=True,
 
 def probe_grid(coords):
     '''Queue the check whether coords (3, npts) is a unit-step pixel grid,
-    or at least in one plane: a device tensor for make_grid.'''
-    out = torch.empty(7, dtype=torch.int64, device=coords.device)
-    _native.check(_native.load().lmb_grid_probe(
+    or at least in one plane: a device tensor for make_grid, the first
+    pixel's z its last value.'''
+    out = torch.empty(8, dtype=torch.int64, device=coords.device)
+    _native.check(_native.load().lmb_plane_probe(
         ptr(coords), coords.shape[1], ptr(out), stream_handle(coords.device)),
-        'lmb_grid_probe')
+        'lmb_plane_probe')
     return out
 
 
 def probe_host(coords):
     '''probe_grid of a host array (3, npts): its values at once.'''
-    out = np.empty(7, dtype=np.int64)
+    out = np.empty(8, dtype=np.int64)
     _native.check(_native.load().lmb_grid_probe_host(
         coords.ctypes.data, coords.shape[1], out.ctypes.data),
         'lmb_grid_probe_host')
+    out[7:].view(np.float64)[0] = coords[2, 0]
     return out
+
+
+def probed_grid(npts, probed):
+    '''make_grid in the probed plane.'''
+    return make_grid(probed[7:].view(np.float64)[0], npts, probed)
 
 
 def make_grid(z, npts, probed):
@@ -250,7 +257,7 @@ def make_grid(z, npts, probed):
     list in the plane z (a numpy int64 array), the grid being a box around
     the pixels otherwise; None if they are not in one plane.'''
     nx, off_grid, off_plane = (int(v) for v in probed[:3])
-    x0, y0, x1, y1 = (float(v) for v in probed[3:].view(np.float64))
+    x0, y0, x1, y1 = (float(v) for v in probed[3:7].view(np.float64))
     if off_plane or max(x1 - x0, y1 - y0) > 1e9:
         return None
     if off_grid == 0 and npts % nx == 0:

@@ -62,15 +62,12 @@ class HologramFunction(torch.autograd.Function):
         # takes longer than the direct sums of small images.
         tables = B * npts * cap >= K.GRADIENT_TABLES
         if tables:
-            probed = torch.cat([coordinates[2, :1].view(torch.int64),
-                                K.probe_grid(coordinates)])
+            probed = K.probe_grid(coordinates)
         ab, dab, nmax = K.sphere_ab(p, inst.n_m, inst.wavelength, cap,
                                     deriv=True, check=False)
         grid = records = h = None
         if tables:
-            probed = probed.cpu().numpy()
-            grid = K.make_grid(probed[:1].view(np.float64)[0], npts,
-                               probed[1:])
+            grid = K.probed_grid(npts, probed.cpu().numpy())
         item_start = torch.arange(B + 1, dtype=torch.int32, device=p.device)
         if grid is not None:
             records = host.copy().view(K.SPHERE_DTYPE).ravel()
