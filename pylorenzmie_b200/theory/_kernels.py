@@ -288,9 +288,10 @@ def on_grid(grid, coords, records, spheres, item_start, ab, nmax, cap,
     if not intervals:
         return None
     nbytes = lib.lmb_radial_workspace_bytes(n, intervals, flags)
-    if nbytes > RADIAL_WORKSPACE_LIMIT:
-        return None
     dev = spheres.device
+    ws = _tables_workspace(nbytes, dev)
+    if ws is None:
+        return None
     nitems = item_start.shape[0] - 1
     if field:
         out = torch.empty((nitems, 3, npts), device=dev,
@@ -298,7 +299,6 @@ def on_grid(grid, coords, records, spheres, item_start, ab, nmax, cap,
     else:
         out = torch.empty((nitems, npts), device=dev,
                           dtype=torch.float64 if fp64 else torch.float32)
-    ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
     name = 'lmb_field_grid' if field else 'lmb_hologram_grid'
     _native.check(getattr(lib, name)(
         grid, None if full else ptr(coords), npts, ptr(spheres),
@@ -309,6 +309,19 @@ def on_grid(grid, coords, records, spheres, item_start, ab, nmax, cap,
 
 # radial tables larger than this are not built (the direct sums need none)
 RADIAL_WORKSPACE_LIMIT = 4 << 30
+
+
+def _tables_workspace(nbytes, dev):
+    '''Scratch with radial tables in it, or None where there is no room for
+    it: the direct sums, which need next to none, then take the call.'''
+    if nbytes > RADIAL_WORKSPACE_LIMIT:
+        return None
+    try:
+        return torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    except torch.OutOfMemoryError:
+        return None
+
+
 # Pixel-orders (spheres x pixels x capacity) from which images of layered
 # spheres (FP64: from half as many) and gradients take the tables.  Below, the
 # direct sums of the pixels take less time than the tables' extra launches and
@@ -403,7 +416,13 @@ def render(grid, coords, records, counts, instrument, cartesian, bohren,
     else:
         out = torch.empty((nitems, npts), device=dev,
                           dtype=torch.float64 if fp64 else torch.float32)
-    ws = torch.empty(plan.workspace_bytes, dtype=torch.uint8, device=dev)
+    ws = None
+    if plan.intervals:
+        ws = _tables_workspace(plan.workspace_bytes, dev)
+        if ws is None:                      # direct sums: what precedes them
+            plan.intervals, plan.workspace_bytes = 0, plan.tables
+    if ws is None:
+        ws = torch.empty(plan.workspace_bytes, dtype=torch.uint8, device=dev)
     _native.check(lib.lmb_render_run(
         plan, box, not full, coords.data_ptr(), npts, host, n,
         start.ctypes.data, nitems, n_m, lam, k, flags, aberration, field,
@@ -421,18 +440,19 @@ def vjp_on_grid(grid, coords, records, spheres, ab, dab, nmax, cap,
     n, npts = len(records), coords.shape[1]
     k, mag = float(instrument.wavenumber()), float(instrument.magnification)
     flags = _flags(True, bohren, False)
-    nbytes = 0
+    nbytes, ws = 0, None
     if n * npts * cap >= GRADIENT_TABLES:
         nbytes = lib.lmb_vjp_grid_workspace_bytes(
             grid, npts, records.ctypes.data, n, k, mag, flags)
-    if not 0 < nbytes <= RADIAL_WORKSPACE_LIMIT:
+    if nbytes:
+        ws = _tables_workspace(nbytes, coords.device)
+    if ws is None:
         return hologram_vjp(coords, spheres, ab, dab, nmax, cap, k,
                             gout.contiguous(), bohren)
     dev = coords.device
     ab, dab, nmax, spheres = _contiguous(ab, dab, nmax, spheres)
     gout = gout.to(torch.float32).contiguous()
     grad = torch.empty((n, 6), dtype=torch.float64, device=dev)
-    ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
     _native.check(lib.lmb_hologram_vjp_grid(
         grid, None if full else ptr(coords), npts, records.ctypes.data,
         ptr(spheres), n, ptr(ab), ptr(dab), ptr(nmax), cap, k, mag, flags,
