@@ -249,14 +249,13 @@ LMB_HD f2 radial_eval(const f4* r, float t) {
 // rule and c and s are rounded to FP32, and U may cancel against c V (behind
 // a large sphere of high index, near its axis, both are up to a hundred times
 // E).  The hologram is off by at most 2 sqrt(H) times the sum over the
-// particles.  On the CPU build, over 2.4 million pixels of single spheres of
-// 0.3-24 um, indices to 2.6, from 1.8 / k above the sphere on, the field is
-// off by at most 2.4e-7 of that.  Over 60 frames of 16 spheres the largest
-// error is 8.9e-6 (with 4e-7 1.45e-5, and 9.3e-6 with the direct sums and
-// their own bound); it costs 2 of 160 us a frame.  1.8 |U|, what |E| comes to
-// where U does not cancel, lowers the mean error of ordinary images: 7.6e-8
-// for 8.3e-8 of the hologram over a batch of 128 images.
-#define RADIAL_FIELD_REL 5e-7f
+// particles.  On the CPU build, over 2.4 million pixels of spheres of 0.3-24
+// um, indices to 2.6, from 1.8 / k above the sphere on: the field is off by
+// at most 2.4e-7 of that, an unmarked pixel's hologram by at most 7.2e-6.
+// 1.8 |U|, what |E| comes to where U does not cancel, keeps the error of
+// ordinary images lower still: 7.6e-8 for 8.3e-8 of the hologram over a batch
+// of 128 images.
+#define RADIAL_FIELD_REL 4e-7f
 
 LMB_HD float radial_bound(f2 u, f2 v, f2 w, float c, float s, float x) {
   const float mu = fmaxf(fabsf(u.x), fabsf(u.y));

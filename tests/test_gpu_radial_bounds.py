@@ -49,22 +49,3 @@ def test_small_spheres_near_the_plane(a, n, z, double):
     got = LorenzMie(coordinates=c, particle=s, double_precision=double).field()
     err = np.abs(got - E).max() / np.abs(E).max()
     assert err <= (1e-12 if double else 1e-6)
-
-
-@pytest.mark.parametrize('seed', [3, 11, 16, 24])
-def test_largest_error_of_frames(seed):
-    '''1e-5: an unmarked pixel's bound is 2e-5, with 5e-7 of the field's size;
-    the field is off by at most 2.4e-7 of that.  (The direct sums leave up to
-    9.3e-6 on such frames.)'''
-    from pylorenzmie_b200 import LorenzMie, workloads
-    rng = np.random.default_rng(seed)
-    c = LorenzMie.meshgrid((1024, 1280))
-    p = np.zeros((16, 6))
-    p[:, 0], p[:, 1] = rng.uniform(0., 1280., 16), rng.uniform(0., 1024., 16)
-    p[:, 3], p[:, 4] = rng.uniform(0.4, 3., 16), rng.uniform(1.38, 1.7, 16)
-    p[:, 2] = np.maximum(rng.uniform(50., 600., 16), p[:, 3] / 0.048 + 10.)
-    spheres = workloads.spheres(p)
-    h32, h64 = (LorenzMie(coordinates=c, particle=spheres,
-                          double_precision=d).hologram()
-                for d in (False, True))
-    assert np.abs(h32 - h64).max() <= 1e-5
