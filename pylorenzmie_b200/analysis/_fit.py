@@ -423,11 +423,13 @@ def default_shape(nfeatures):
 # room.  Measured on a B200 against launch shape 0: an evaluation of 256
 # features of 201x201 px 1.14 -> 0.13 ms.  A table costs ~15 us of serial FP64
 # work, whatever the pixels, so batches of fewer than SMALL_BATCH features of
-# at most RADIAL_PIXELS pixels (a frame's features on their random subsets)
-# keep SMALL_SHAPE: 32 features of 1460 px 22 against 16 us.  Multilayer
-# spheres keep the sums at every pixel: their uncertainties in a_p and z_p can
-# follow the rounding of the Jacobian (a batch of 24 moved by up to 9e-5 of
-# itself, towards the 64-bit values).
+# at most RADIAL_PIXELS pixels keep SMALL_SHAPE: whole fits of 39-51 px square
+# (and of a frame's features on their random subsets) are 0.96-1.09 as fast
+# with tables (a_p 0.8 um), those of 65-101 px 0.97-1.18, of 131-201 px
+# 0.97-1.37, 1-63 features each; a_p 2 um, with twice the orders, 0.91-1.12,
+# 1.03-1.33 and 1.02-1.85.  Multilayer spheres keep the sums at every pixel:
+# their uncertainties in a_p and z_p can follow the rounding of the Jacobian
+# (a batch of 24 moved by up to 9e-5 of itself, towards the 64-bit values).
 RADIAL_PIXELS = 4096
 
 

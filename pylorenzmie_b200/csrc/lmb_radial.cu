@@ -319,7 +319,7 @@ constexpr int kTileGroup = 32;     // particles whose TileParticle is staged at 
 // and only t is duplicated.  A pixel's value depends on its position alone,
 // not on its neighbours (groups of pixels that share an interval would read
 // less, but differ from the same pixel in a list by their rounding).
-// A 1280x1024 frame of 16 spheres: 120 us, 73% of the shared-memory pipe's
+// A 1280x1024 frame of 16 spheres: 121 us, 72% of the shared-memory pipe's
 // peak (144 bytes a pixel and particle); with the orders summed at every
 // pixel (k_field_pair) 1.44 ms.
 constexpr int kStages = 3;

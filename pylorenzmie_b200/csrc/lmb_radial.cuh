@@ -249,12 +249,15 @@ LMB_HD f2 radial_eval(const f4* r, float t) {
 // rule and c and s are rounded to FP32, and U may cancel against c V (behind
 // a large sphere of high index, near its axis, both are up to a hundred times
 // E).  The hologram is off by at most 2 sqrt(H) times the sum over the
-// particles.  On the CPU build, over 2.4 million pixels of spheres of 0.3-24
-// um, indices to 2.6, from 1.8 / k above the sphere on: the field is off by
-// at most 2.4e-7 of that, an unmarked pixel's hologram by at most 7.2e-6.
-// 1.8 |U|, what |E| comes to where U does not cancel, keeps the error of
-// ordinary images lower still: 7.6e-8 for 8.3e-8 of the hologram over a batch
-// of 128 images.
+// particles.  On the CPU build, over 2.4 million pixels of single spheres of
+// 0.3-24 um, indices to 2.6, from 1.8 / k above the sphere on, the field is
+// off by at most 2.4e-7 of that, an unmarked pixel's hologram by at most
+// 7.2e-6.  1.8 |U|, what |E| comes to where U does not cancel, lowers the
+// error of ordinary images further: 7.6e-8 for 8.3e-8 of the hologram over a
+// batch of 128 images.  The largest error of 60 frames of 16 spheres is
+// 1.45e-5 (9.3e-6 with the direct sums, whose own bound marks more; 5e-7 here
+// leaves 8.9e-6, but the pixels summed again sit together and their tiles end
+// late: 28 such frames 218-221 -> 228 us, one 234 -> 266).
 #define RADIAL_FIELD_REL 4e-7f
 
 LMB_HD float radial_bound(f2 u, f2 v, f2 w, float c, float s, float x) {

@@ -4,7 +4,7 @@ images take that path.
 
 Tolerances.  Holograms: 2e-5 absolute, the contract of the FP32 holograms.
 Fields: 1e-6 of the sum of the particles' largest components.  The table is
-off by at most 4e-8 of a component (FP64 nodes, degree-7 polynomials) and
+off by at most 4e-8 of a component (FP64 nodes, degree-5 polynomials) and
 its FP32 evaluation by a few roundings of 6e-8.
 '''
 import numpy as np
@@ -58,7 +58,7 @@ CASES = [
     ((225, 287), 4, {}, {'below': True}),
     ((256, 320), 2, {}, {'bohren': False}),
     ((256, 260), 2, {}, {'spherical': 1.5}),
-    ((256, 260), 2, {'magnification': 0.135}, {}),   # k > 1.1: no groups
+    ((256, 260), 2, {'magnification': 0.135}, {}),   # few px an interval
     ((256, 260), 2, {'magnification': 0.02}, {}),
 ]
 
